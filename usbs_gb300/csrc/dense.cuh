@@ -154,47 +154,69 @@ __device__ inline bool warp_syev(double* A, int lda, int n, double* w, double* Z
 }
 
 // Rotation (c, s) that zeroes the (p, q) entry of the symmetric 2 x 2 block
-// [[app, apq], [apq, aqq]] (Rutishauser's formulas).
+// [[app, apq], [apq, aqq]] (Rutishauser's formulas).  Where |theta| >= 2^64 its
+// square overflows and the formulas give t = 0 with theta's sign, c = 1: those
+// lanes divide ones instead, because quotients with such operands leave the
+// fast path of the division for the whole warp (late in a sweep most warps
+// have such a pair).
 __device__ __forceinline__ void jacobi_rot(float app, float aqq, float apq, float& c, float& sn) {
   c = 1.0f;
   sn = 0.0f;
   if (apq != 0.0f) {
-    const float theta = (aqq - app) / (2.0f * apq);
-    const float t = copysignf(1.0f, theta) / (fabsf(theta) + sqrtf(theta * theta + 1.0f));
+    float d = aqq - app, e = 2.0f * apq;
+    const bool big = fabsf(d) >= 0x1p64f * fabsf(e);
+    const float sgn = copysignf(1.0f, e) * d;      // theta's sign
+    if (big) { d = 1.0f; e = 1.0f; }
+    const float theta = d / e;
+    float t = 1.0f / (fabsf(theta) + sqrtf(theta * theta + 1.0f));
+    t = copysignf(big ? 0.0f : t, big ? sgn : theta);
     c = rsqrtf(t * t + 1.0f);
     sn = t * c;
   }
 }
 
-// Pair i (0 <= i < M/2) of round r (0 <= r < M-1) of the round-robin
-// ("chess tournament") order, p < q: index 0 stays, 1..M-1 rotate.
-template <int M>
-__device__ __forceinline__ void jacobi_pair(int r, int i, int& p, int& q) {
-  if (i == 0) {
-    p = 0;
-    q = 1 + r;
-  } else {
-    p = r + i;
-    p = (p >= M - 1) ? p - (M - 1) : p;
-    p += 1;
-    q = r - i + M - 1;
-    q = (q >= M - 1) ? q - (M - 1) : q;
-    q += 1;
-  }
-  if (p > q) { const int t = p; p = q; q = t; }
+// a x - b y and a x + b y with the second product rounded (the choice is spelt
+// out so that the result does not depend on the code around it).
+__device__ __forceinline__ float rot_sub(float a, float x, float b, float y) {
+  return __fmaf_rn(a, x, -__fmul_rn(b, y));
+}
+__device__ __forceinline__ float rot_add(float a, float x, float b, float y) {
+  return __fmaf_rn(a, x, __fmul_rn(b, y));
 }
 
+// Pair i (0 <= i < M/2) of rounds r = 0, 1, ... of the round-robin ("chess
+// tournament") order, p < q: index 0 stays, 1..M-1 rotate.  Pair 0 of round r
+// is (0, 1 + r), pair i > 0 is {1 + (r + i) mod (M-1), 1 + (r - i) mod (M-1)}.
+template <int M>
+struct JacobiPair {
+  int a, b;
+  bool first;
+  __device__ __forceinline__ explicit JacobiPair(int i)
+      : a(1 + i), b(1 + (M - 1 - i) % (M - 1)), first(i == 0) {}
+  __device__ __forceinline__ int p() const { return first ? 0 : min(a, b); }
+  __device__ __forceinline__ int q() const { return max(a, b); }
+  __device__ __forceinline__ void next() {
+    a = (a == M - 1) ? 1 : a + 1;
+    b = (b == M - 1) ? 1 : b + 1;
+  }
+};
+
 // Cyclic parallel Jacobi eigensolver (float) for a symmetric n x n matrix, run
-// by a whole CTA (blockDim a multiple of 32) at order M (32 or 16; indices >= n
+// by a CTA of 8 warps at order M (32 or 16; indices >= n
 // are padding that couples to nothing): M/2 disjoint rotations per round in
 // round-robin order, sweeps until the off-diagonal Frobenius norm is below
 // 4 eps ||A||_F.
 // One CTA barrier per round: A is double-buffered (a round reads one buffer
 // and writes the other), and every warp forms the round's M/2 rotations itself
-// (lane l: pair l mod M/2) and hands them to its threads by shuffle.  Thread
+// (lane l: pair l mod M/2, which is also the column pair of its block).  Thread
 // (I, J) maps the 2 x 2 block of pairs (I, J) through the row rotation of I
 // and the column rotation of J (the pairs are disjoint, so the block depends
-// only on itself), and rotates rows J and J + M/2 of Z by pair I.
+// only on itself).  The eigenvectors are kept transposed (row p of Z is vector
+// p): a warp rotates those of its own row pairs, conflict-free.  A round is
+// bound by the rotation's chain of two divisions and two roots (about 310
+// cycles) and by instruction issue: everything that does not depend on the
+// rotation is loaded before it, and the indices and rotations of the row pairs
+// come by shuffle from the lanes that hold them.
 // A and A2 (row-major, lda >= M, each with room for 2 lda + n M floats) are
 // destroyed; w receives the eigenvalues ascending, Z (row-major, ldz >= M) the
 // eigenvectors as columns.  Returns false (uniformly) if 20 sweeps do not
@@ -217,11 +239,15 @@ __device__ inline bool cta_jacobi_f32(float* A, float* A2, int lda, int n, float
     fro = warp_sum(fro);
     if (lane == 0) red[0] = fro * (4.0f * 1.2e-7f) * (4.0f * 1.2e-7f);
   }
-  __syncthreads();
-  const float tol2 = red[0];
   float* cur = A;
   float* nxt = A2;
   bool ok = false;
+  const int I = ((32 / H) * wid + lane / H) % H;
+  const int z0 = ((32 / H) * wid + lane / M) % H, z1 = (z0 + 32 / M) % H, zr = lane % M;
+  const bool own = tid < H * H;          // whole warps
+  JacobiPair<M> pj(lane % H);
+  __syncthreads();
+  const float tol2 = red[0];
   for (int sweep = 0; sweep < 20; ++sweep) {
     if (wid == 0) {
       float off = 0.0f;
@@ -235,36 +261,47 @@ __device__ inline bool cta_jacobi_f32(float* A, float* A2, int lda, int n, float
     __syncthreads();
     if (red[1] <= tol2) { ok = true; break; }
     for (int r = 0; r < M - 1; ++r) {
-      int pl, ql;
-      jacobi_pair<M>(r, lane % H, pl, ql);
-      float cl, sl;
-      jacobi_rot(cur[pl * lda + pl], cur[ql * lda + ql], cur[pl * lda + ql], cl, sl);
-      for (int base = 0; base < H * H; base += nt) {      // trip count uniform over the CTA
-        const int e = base + tid;
-        const int I = (e / H) % H, J = e % H;
-        const float c = __shfl_sync(0xffffffffu, cl, I), sn = __shfl_sync(0xffffffffu, sl, I);
-        const float c2 = __shfl_sync(0xffffffffu, cl, J), s2 = __shfl_sync(0xffffffffu, sl, J);
-        if (e < H * H) {
-          int p, q, p2, q2;
-          jacobi_pair<M>(r, I, p, q);
-          jacobi_pair<M>(r, J, p2, q2);
-          const float app = cur[p * lda + p2], apq = cur[p * lda + q2];
-          const float aqp = cur[q * lda + p2], aqq = cur[q * lda + q2];
-          // rows
-          const float bpp = c * app - sn * aqp, bpq = c * apq - sn * aqq;
-          const float bqp = sn * app + c * aqp, bqq = sn * apq + c * aqq;
-          // columns
-          nxt[p * lda + p2] = c2 * bpp - s2 * bpq;
-          nxt[p * lda + q2] = s2 * bpp + c2 * bpq;
-          nxt[q * lda + p2] = c2 * bqp - s2 * bqq;
-          nxt[q * lda + q2] = s2 * bqp + c2 * bqq;
-#pragma unroll
-          for (int j = J; j < M; j += H) {
-            const float zp = Z[j * ldz + p], zq = Z[j * ldz + q];
-            Z[j * ldz + p] = c * zp - sn * zq;
-            Z[j * ldz + q] = sn * zp + c * zq;
-          }
+      if (own) {
+        const int p2 = pj.p(), q2 = pj.q(), pq = p2 | (q2 << 16);
+        const float* dp = cur + p2 * lda;
+        const float dpp = dp[p2], dpq = dp[q2], dqq = cur[q2 * lda + q2];
+        const int w0 = __shfl_sync(0xffffffffu, pq, z0), w1 = __shfl_sync(0xffffffffu, pq, z1);
+        int wi;
+        if constexpr (M == 32) wi = (lane < 16) ? w0 : w1;
+        else wi = __shfl_sync(0xffffffffu, pq, I);
+        const int p = (wi & 0xffff) * lda, q = (wi >> 16) * lda;
+        const float app = cur[p + p2], apq = cur[p + q2];
+        const float aqp = cur[q + p2], aqq = cur[q + q2];
+        float* zp0 = Z + (w0 & 0xffff) * ldz + zr;
+        float* zq0 = Z + (w0 >> 16) * ldz + zr;
+        float* zp1 = Z + (w1 & 0xffff) * ldz + zr;
+        float* zq1 = Z + (w1 >> 16) * ldz + zr;
+        const float vp0 = *zp0, vq0 = *zq0, vp1 = *zp1, vq1 = *zq1;
+        float c2, s2;
+        jacobi_rot(dpp, dqq, dpq, c2, s2);
+        const float c0 = __shfl_sync(0xffffffffu, c2, z0), s0 = __shfl_sync(0xffffffffu, s2, z0);
+        const float c1 = __shfl_sync(0xffffffffu, c2, z1), s1 = __shfl_sync(0xffffffffu, s2, z1);
+        float c, sn;
+        if constexpr (M == 32) {
+          c = (lane < 16) ? c0 : c1;
+          sn = (lane < 16) ? s0 : s1;
+        } else {
+          c = __shfl_sync(0xffffffffu, c2, I);
+          sn = __shfl_sync(0xffffffffu, s2, I);
         }
+        // rows
+        const float bpp = rot_sub(c, app, sn, aqp), bpq = rot_sub(c, apq, sn, aqq);
+        const float bqp = rot_add(sn, app, c, aqp), bqq = rot_add(sn, apq, c, aqq);
+        // columns
+        nxt[p + p2] = rot_sub(c2, bpp, s2, bpq);
+        nxt[p + q2] = rot_add(s2, bpp, c2, bpq);
+        nxt[q + p2] = rot_sub(c2, bqp, s2, bqq);
+        nxt[q + q2] = rot_add(s2, bqp, c2, bqq);
+        *zp0 = rot_sub(c0, vp0, s0, vq0);
+        *zq0 = rot_add(s0, vp0, c0, vq0);
+        *zp1 = rot_sub(c1, vp1, s1, vq1);
+        *zq1 = rot_add(s1, vp1, c1, vq1);
+        pj.next();
       }
       __syncthreads();
       float* t = cur;
@@ -290,16 +327,16 @@ __device__ inline bool cta_jacobi_f32(float* A, float* A2, int lda, int n, float
     w[r] = v;
   }
   __syncthreads();
-  // permute Z's columns: Z[:, rank[c]] = Z_old[:, c]
+  // the vectors in their order, as columns: Z[:, rank[c]] = vector c
   float* zs = nxt + 2 * lda;   // n x n, stride M
   for (int e = tid; e < n * n; e += nt) {
-    const int i = e / n, c = e - (e / n) * n;
-    zs[i * M + c] = Z[i * ldz + c];
+    const int c = e / n, i = e - (e / n) * n;
+    zs[c * M + i] = Z[c * ldz + i];
   }
   __syncthreads();
   for (int e = tid; e < n * n; e += nt) {
     const int i = e / n, c = e - (e / n) * n;
-    Z[i * ldz + rk[c]] = zs[i * M + c];
+    Z[i * ldz + rk[c]] = zs[c * M + i];
   }
   __syncthreads();
   return ok;

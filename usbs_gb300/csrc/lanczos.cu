@@ -85,7 +85,6 @@ struct LzShared {
       double ys[LZ_BLOCK];
       double wred[LZ_NW][MP1];
     } st;
-    VT cys[LZ_BLOCK];            // cluster kernel: row results of the SpMV, in the vector type
     struct {                     // restart on CTA 0 (T, X, R, S, W row-major, ld MP1)
       double T[MAXM * MP1];
       double X[MAXM * MP1];
@@ -97,8 +96,8 @@ struct LzShared {
     double red4[4][MP1];         // cluster reduction: the four level-two sums
   } u;
   double h[MP1];
-  VT hv[MP1];                    // h in the vector type, converted once per reduction
   double bnorm;                  // cluster kernel: sqrt(h[0]) of a norm reduction ...
+  VT hv[MP1];                    // h in the vector type, converted once per reduction (16-byte aligned)
   VT binv;                       // ... and 1 / bnorm in the vector type
   double alpha[MAXM];
   double beta[MAXM];
@@ -352,15 +351,168 @@ __device__ void phase_update_norm(const TeamDesc<VT>& P, SH& sh, int t0, int t1,
   block_reduce_cols(one, 1, sh, part_out, P.nctas);
 }
 
+__device__ __forceinline__ unsigned cl_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cl_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
+               "barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cl_map(const void* p, unsigned rank) {
+  uint32_t a = (uint32_t)__cvta_generic_to_shared(p), r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+// Reads of a peer's (or the own) shared memory written before the last cluster
+// barrier.  volatile keeps them after that barrier and in order among
+// themselves; without a memory clobber plain loads may be issued around them.
+__device__ __forceinline__ float cl_ld(uint32_t a, float) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ double cl_ld(uint32_t a, double) {
+  double v;
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void cl_st(uint32_t a, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+
+// M[i][j] = v in every CTA's copy of M (the CTAs' shared memory is laid out alike)
+__device__ __forceinline__ void cl_share(double* p, int C, double v) {
+  for (int r = 0; r < C; ++r) cl_st(cl_map(p, r), v);
+}
+
+// cta_refine_eig (dense.cuh) with its four n x n products and the quotients E
+// dealt out over the C CTAs of the cluster, which all hold the same A, X and
+// lam: each CTA forms n^2 / C entries, as cta_refine_eig forms them, and writes
+// them to every CTA.  The products are 4 n^3 FP64 FMAs at 2 per clock and SM:
+// done by every CTA redundantly they took 170k cycles per step (n = 32).
+__device__ inline void cl_refine_eig(const double* A, double* X, double* R, double* S, double* W,
+                                     double* lam, double* red, int n, int ld, int rank, int C) {
+  const int tid = threadIdx.x, nt = blockDim.x, nn = n * n;
+  const int e0 = nn * rank / C, e1 = nn * (rank + 1) / C;
+  // W = A X
+  for (int e = e0 + tid; e < e1; e += nt) {
+    const int i = e / n, j = e - i * n;
+    double v = 0.0;
+    for (int l = 0; l < n; ++l) {
+      const double a = A[i * ld + l];
+      if (a != 0.0) v += a * X[l * ld + j];
+    }
+    cl_share(W + i * ld + j, C, v);
+  }
+  cl_sync();
+  // R = I - X^T X and S = X^T W, one of the two per thread
+  for (int e = 2 * e0 + tid; e < 2 * e1; e += nt) {
+    const bool second = e >= e0 + e1;
+    const int f = second ? e - e1 : e - e0;
+    const int i = f / n, j = f - i * n;
+    const double* B = second ? W : X;
+    double r = 0.0;
+    for (int l = 0; l < n; ++l) r += X[l * ld + i] * B[l * ld + j];
+    if (second) cl_share(S + i * ld + j, C, r);
+    else cl_share(R + i * ld + j, C, ((i == j) ? 1.0 : 0.0) - r);
+  }
+  cl_sync();
+  if (tid < n) lam[tid] = S[tid * ld + tid] / (1.0 - R[tid * ld + tid]);
+  __syncthreads();
+  // delta = 2 (||S - diag(lam)||_F + ||A||_F ||R||_F)
+  double sa = 0.0, aa = 0.0, rr = 0.0;
+  for (int e = tid; e < nn; e += nt) {
+    const int i = e / n, j = e - i * n;
+    const double d = S[i * ld + j] - ((i == j) ? lam[i] : 0.0);
+    sa += d * d;
+    aa += A[i * ld + j] * A[i * ld + j];
+    rr += R[i * ld + j] * R[i * ld + j];
+  }
+  sa = block_sum(sa, red);
+  __syncthreads();
+  aa = block_sum(aa, red);
+  __syncthreads();
+  rr = block_sum(rr, red);
+  const double delta = 2.0 * (sqrt(sa) + sqrt(aa) * sqrt(rr));
+  // E into W (every CTA is past its last read of the old W)
+  for (int e = e0 + tid; e < e1; e += nt) {
+    const int i = e / n, j = e - i * n;
+    const double dl = lam[j] - lam[i];
+    cl_share(W + i * ld + j, C,
+             (fabs(dl) > delta) ? (S[i * ld + j] + lam[j] * R[i * ld + j]) / dl
+                                : 0.5 * R[i * ld + j]);
+  }
+  cl_sync();
+  // X <- X + X E   (result into S, then copied back)
+  for (int e = e0 + tid; e < e1; e += nt) {
+    const int i = e / n, j = e - i * n;
+    double v = 0.0;
+    for (int l = 0; l < n; ++l) v += X[i * ld + l] * W[l * ld + j];
+    cl_share(S + i * ld + j, C, X[i * ld + j] + v);
+  }
+  cl_sync();
+  for (int e = tid; e < nn; e += nt) {
+    const int i = e / n, j = e - i * n;
+    X[i * ld + j] = S[i * ld + j];
+  }
+  __syncthreads();
+}
+
+// Key whose unsigned order is the order of finite or infinite doubles (-0 = +0).
+__device__ __forceinline__ unsigned long long order_key(double x) {
+  const long long b = __double_as_longlong(x == 0.0 ? 0.0 : x);
+  return (unsigned long long)b ^ (b < 0 ? ~0ull : 0x8000000000000000ull);
+}
+
+// order[] = the positions a selection sort of v[0..m-1] (ascending, the first of
+// equal values at each step, by swaps) ends with.  Warp 0, lane p at position p,
+// integer keys: the comparisons stay off the FP64 pipe, where one thread's
+// loop of them took tens of thousands of cycles.  NaNs take the plain loop.
+__device__ __forceinline__ void select_order(const double* v, int m, int* order) {
+  const int lane = threadIdx.x;
+  if (lane >= 32) return;
+  const bool in = lane < m;
+  if (__any_sync(0xffffffffu, in && isnan(v[in ? lane : 0]))) {
+    if (lane == 0) {
+      for (int i = 0; i < m; ++i) order[i] = i;
+      for (int i = 0; i < m - 1; ++i) {
+        int kmin = i;
+        for (int j = i + 1; j < m; ++j)
+          if (v[order[j]] < v[order[kmin]]) kmin = j;
+        const int t = order[i]; order[i] = order[kmin]; order[kmin] = t;
+      }
+    }
+    return;
+  }
+  const unsigned long long key = in ? order_key(v[lane]) : ~0ull;
+  unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
+  int idx = lane;
+  for (int i = 0; i < m - 1; ++i) {
+    const bool c = in && lane >= i;
+    const unsigned mhi = __reduce_min_sync(0xffffffffu, c ? hi : 0xffffffffu);
+    const bool th = c && hi == mhi;
+    const unsigned mlo = __reduce_min_sync(0xffffffffu, th ? lo : 0xffffffffu);
+    const int k = __ffs(__ballot_sync(0xffffffffu, th && lo == mlo)) - 1;
+    const int src = (lane == i) ? k : (lane == k) ? i : lane;
+    hi = __shfl_sync(0xffffffffu, hi, src);
+    lo = __shfl_sync(0xffffffffu, lo, src);
+    idx = __shfl_sync(0xffffffffu, idx, src);
+  }
+  if (in) order[lane] = idx;
+}
+
 // CTA 0 of a team: projected eigenproblem and thick-restart selection
 // (solver/lanczos.py:128-168, 202-221).  k = number of saved vectors of the
 // finished cycle, beta_last = beta[m-1].
-// LOCAL_YS: every CTA of a cluster runs this redundantly (identical inputs give
-// identical results) and keeps the saved Ritz vectors in sh.u.Ys; only the CTA
+// LOCAL_YS: every CTA of a cluster (rank of C) runs this on identical inputs to
+// identical results (the FP64 refinement's products shared out) and keeps the saved Ritz vectors in sh.u.Ys; only the CTA
 // with write_out set stores alpha/beta/ctl.  Otherwise (team kernel) the Ritz
 // vectors go through P.Ybuf.
 template <bool LOCAL_YS, typename VT, typename D>
-__device__ void restart_select(const D& P, LzShared<VT>& sh, int k, bool write_out = true) {
+__device__ void restart_select(const D& P, LzShared<VT>& sh, int k, bool write_out = true,
+                               int rank = 0, int C = 1) {
   const int m = P.m, tid = threadIdx.x;
   double* T = sh.u.rs.T;
   double* X = sh.u.rs.X;
@@ -393,17 +545,15 @@ __device__ void restart_select(const D& P, LzShared<VT>& sh, int k, bool write_o
   __syncthreads();
   if (sizeof(VT) == 8) {
     // ... refined to FP64 accuracy by two Ogita-Aishima steps, then re-sorted
-    cta_refine_eig(T, X, sh.u.rs.R, sh.u.rs.S, sh.u.rs.W, sh.ritz, sh.red, m, MP1);
-    cta_refine_eig(T, X, sh.u.rs.R, sh.u.rs.S, sh.u.rs.W, sh.ritz, sh.red, m, MP1);
-    if (tid == 0) {
-      for (int i = 0; i < m; ++i) sh.order[i] = i;
-      for (int i = 0; i < m - 1; ++i) {
-        int kmin = i;
-        for (int j = i + 1; j < m; ++j)
-          if (sh.ritz[sh.order[j]] < sh.ritz[sh.order[kmin]]) kmin = j;
-        const int t = sh.order[i]; sh.order[i] = sh.order[kmin]; sh.order[kmin] = t;
-      }
+    // (a peer may still run its Jacobi sweeps in the buffers the refinement shares)
+    if constexpr (LOCAL_YS) cl_sync();
+    for (int it = 0; it < 2; ++it) {
+      if constexpr (LOCAL_YS)
+        cl_refine_eig(T, X, sh.u.rs.R, sh.u.rs.S, sh.u.rs.W, sh.ritz, sh.red, m, MP1, rank, C);
+      else
+        cta_refine_eig(T, X, sh.u.rs.R, sh.u.rs.S, sh.u.rs.W, sh.ritz, sh.red, m, MP1);
     }
+    select_order(sh.ritz, m, sh.order);
     __syncthreads();
     double* Sx = sh.u.rs.S;
     for (int e = tid; e < m * m; e += LZ_BLOCK) {
@@ -420,38 +570,47 @@ __device__ void restart_select(const D& P, LzShared<VT>& sh, int k, bool write_o
     __syncthreads();
   }
   const double* Z = X;
-  if (tid == 0) {
+  if (tid < 32) {
+    // lane c: Ritz pair c.  The residual tests, the gap ratios (one FP64
+    // division each) and the finiteness test run side by side; as one thread's
+    // loop they took about 25k cycles per restart.
+    const int lane = tid;
+    const bool in = lane < m;
     // a NaN / Inf in the projected matrix (e.g. from a non-finite operator)
     // ends the call after this restart with ST_NONFINITE
-    bool fin = true;
-    for (int c = 0; c < m; ++c) fin = fin && isfinite(sh.alpha[c]) && isfinite(sh.beta[c]);
-    if (!fin) atomicOr(P.status, ST_NONFINITE);
+    const bool fin = !in || (isfinite(sh.alpha[lane]) && isfinite(sh.beta[lane]));
     const double bl = sh.beta[m - 1];
-    int nconv = m;
-    for (int c = 0; c < m; ++c) {
-      if (!(bl * fabs(Z[(m - 1) * MP1 + c]) < P.tol)) { nconv = c; break; }
-    }
+    const bool open = in && !(bl * fabs(Z[(m - 1) * MP1 + lane]) < P.tol);
+    const unsigned ob = __ballot_sync(0xffffffffu, open);
+    const int nconv = ob ? __ffs(ob) - 1 : m;
     const int delta = min(m - P.num_desired, 2 * (m - nconv) / 5);
     const double lt = sh.ritz[min(nconv, m - 1)];
-    int kl = 0;
-    double bv = 0.0;
-    for (int c = 0; c < m; ++c) {
-      const int kr = c + delta;
-      double g = 0.0;
-      if (kr <= m) g = (sh.ritz[c] - lt) / (sh.ritz[min(kr, m - 1)] - lt);
-      if (c == 0) { bv = g; kl = 0; if (isnan(g)) break; continue; }
-      if (isnan(g)) { kl = c; break; }
-      if (g > bv) { bv = g; kl = c; }
+    double g = 0.0;
+    if (in) {
+      const int kr = lane + delta;
+      if (kr <= m) g = (sh.ritz[lane] - lt) / (sh.ritz[min(kr, m - 1)] - lt);
     }
+    // first NaN, else the first largest ratio
+    const unsigned nb = __ballot_sync(0xffffffffu, in && isnan(g));
+    const unsigned long long key = order_key(g);
+    const unsigned hi = in ? (unsigned)(key >> 32) : 0u, lo = (unsigned)key;
+    const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
+    const bool th = in && hi == mhi;
+    const unsigned mlo = __reduce_max_sync(0xffffffffu, th ? lo : 0u);
+    const unsigned tb = __ballot_sync(0xffffffffu, th && lo == mlo);
+    const int kl = nb ? __ffs(nb) - 1 : __ffs(tb) - 1;
     const int kright = kl + delta;
-    int kn = 0;
-    for (int c = 0; c < m; ++c)
-      if (kl >= c || kright < c) sh.order[kn++] = c;
-    int pos = kn;
-    for (int c = 0; c < m; ++c)
-      if (!(kl >= c || kright < c)) sh.order[pos++] = c;
-    sh.k_next = kn;
-    sh.nconv = nconv;
+    const bool keep = in && (kl >= lane || kright < lane);
+    const unsigned kb = __ballot_sync(0xffffffffu, keep);
+    const unsigned below = (1u << lane) - 1u;
+    const int kn = __popc(kb);
+    if (in) sh.order[keep ? __popc(kb & below) : kn + lane - __popc(kb & below)] = lane;
+    const bool bad = !__all_sync(0xffffffffu, fin);
+    if (lane == 0) {
+      if (bad) atomicOr(P.status, ST_NONFINITE);
+      sh.k_next = kn;
+      sh.nconv = nconv;
+    }
   }
   __syncthreads();
   const int kn = sh.k_next;
@@ -1320,16 +1479,23 @@ __global__ void __launch_bounds__(LZ_BLOCK) st_rotate_kernel(const __grid_consta
 // A problem of at most CL_MAX_CTAS x rc rows runs as one thread-block cluster.
 // CTA r of the cluster owns rows [r rc, (r+1) rc) and keeps, for the whole
 // eigsh call, its rows of the basis Q (column-major, stride rc), the two work
-// vectors and, when it fits, its slice of the operator (CSR with the column
-// pre-split into owner CTA and local row) in shared memory.  The SpMV gathers
-// x straight from the owner CTAs' shared memory (distributed shared memory,
-// mapa + ld.shared::cluster); each phase's per-CTA partial sums are written to
+// vectors and, when it fits, its slice of the operator in shared memory.  The
+// SpMV gathers x from the owner CTAs' shared memory (distributed shared memory,
+// mapa + ld.shared::cluster; the address of each entry's row is formed once) or
+// from a copy of all of x that each CTA makes per step (see the rule in the
+// kernel); each phase's per-CTA partial sums are written to
 // the CTA's own shared memory and, after a hardware cluster barrier, summed by
 // every CTA over the cluster in the same fixed order, so all CTAs hold
 // bit-identical coefficients and take identical branches.  The restart's
 // projected eigenproblem is solved redundantly by every CTA (identical inputs,
-// identical results), which needs no broadcast.  A cluster is co-scheduled by
-// the hardware, so there is no software barrier and no spin-wait.
+// identical results), which needs no broadcast; its FP64 refinement is shared
+// out.  A cluster is co-scheduled by the hardware, so there is no software
+// barrier and no spin-wait.
+// Bound by latency: FP32 torus n = 10^4 runs 20k cycles per step (SpMV and dots
+// 5.9k, second projection 5.6k, norm pass 2.6k, reductions 4.5k, barriers 1.7k)
+// and 160k per restart, 2.22 ms per call of 131 steps (3.53 ms with one
+// gather, one column and one shuffle level at a time); FP64 ER n = 800 of
+// degree 48 3.06 ms (8.25 ms).
 constexpr int CL_MAX_CTAS = 16;
 
 template <typename VT>
@@ -1352,31 +1518,6 @@ struct ClusterBatch {
   int count, csize;
   ClusterDesc<VT> t[MAX_TEAMS];
 };
-
-__device__ __forceinline__ unsigned cl_rank() {
-  unsigned r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cl_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
-               "barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t cl_map(const void* p, unsigned rank) {
-  uint32_t a = (uint32_t)__cvta_generic_to_shared(p), r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ float cl_ld(uint32_t a, float) {
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ double cl_ld(uint32_t a, double) {
-  double v;
-  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
-  return v;
-}
 
 // per-CTA shared-memory layout of the cluster kernel (byte offsets)
 struct ClLayout {
@@ -1436,200 +1577,437 @@ __device__ __forceinline__ void cl_reduce(const double* part, int C, int nv, LzS
   __syncthreads();
 }
 
+// The cluster kernel's dynamic shared memory as words of VT from its start (the
+// basis comes first); every vector below is an offset from there, so that the
+// accesses are shared-memory instructions with 32-bit addresses.
+template <typename VT>
+__device__ __forceinline__ VT* cl_dyn_words() {
+  extern __shared__ __align__(16) unsigned char cl_dyn[];
+  return (VT*)cl_dyn;
+}
+
 template <typename VT>
 struct ClCtx {
-  const ClusterDesc<VT>* P;
-  int rank, C, r0, rows;
+  int rank, C, n, m, rc, r0, rows;
+  int lanes, lp;        // accumulators per row of the SpMV, threads per row (lp <= lanes)
   bool staged;          // CSR slice in shared memory
-  int p0;               // first entry of the slice
-  VT* Qs;               // (m+1) x rc
-  VT* vb;               // 2 x rc
-  double* part;         // 3 x MP1
-  int* rp;              // rows+1, relative to p0
-  int* cg;              // (owner << 24) | local row
-  VT* vs;
+  int rp, cg, vs;       // its row bounds (rows+1 ints, from the slice's start), columns, values
+  int xs;               // the whole x, copied at the start of each SpMV (or -1)
+  const int* g_rowptr;  // the operator in global memory (slices that do not fit)
+  const int* g_col;
+  const VT* g_val;
 };
 
-// Phase A: y = Op (x * xscale) for own rows -> vout, partial Q[:, c] . y (c <= i).
-// x is column `xcol` of the cluster's vectors: xq selects Qs (else vb); the
-// gathers read the owner CTA's copy.  If wq, Qs[:, i] = x * xscale (own rows).
-template <typename VT, int L>
-__device__ void cl_phase_spmv(const ClCtx<VT>& X, LzShared<VT>& sh, int i, const VT* xbase,
-                              VT xscale, bool wq, VT* vout, double* part_out) {
+// Row sums of the SpMV.  A row's entries are dealt round-robin to `lanes`
+// accumulators that are then added pairwise (distance lanes/2, ..., 1).  A row
+// takes lp <= lanes threads, each with NL = lanes / lp of the accumulators in
+// registers (thread t: t, t + lp, ...), so the first log2(NL) levels of the tree
+// need no shuffle; the sums do not depend on lp.  lp is chosen so that one pass
+// of the CTA covers its rows: with one row per warp (lanes = 32, 62 FP64 rows of
+// 49 entries per CTA) the shuffle tree's FP64 adds took 50k cycles per step,
+// because an FP64 warp instruction holds its pipe for 64 cycles however few
+// lanes carry a row.
+// XS: x is read from the CTA's copy and cg holds byte offsets in it; else cg
+// holds the shared::cluster address of the entry's row in its owner's Q[:, 0].
+template <typename VT, int NL, bool XS>
+__device__ __forceinline__ VT cl_row_sum(const ClCtx<VT>& X, int lr, int lig, int xo) {
   typedef typename Acc<VT>::type AT;
-  const ClusterDesc<VT>& P = *X.P;
-  const int tid = threadIdx.x, rc = P.rc;
-  constexpr int GPP = LZ_BLOCK / L;
-  const int g = tid / L, lig = tid - (tid / L) * L;
-  AT acc[MP1];
+  const int L = X.lanes, lp = X.lp;
+  AT s[NL];
 #pragma unroll
-  for (int c = 0; c < MP1; ++c) acc[c] = (AT)0;
-  for (int base = 0; base < X.rows; base += LZ_BLOCK) {
-    // SpMV of rows base..base+255 (L lanes per row) into sh.u.st.ys; groups of
-    // up to 4 passes load their row bounds and first entries before any gather
-    constexpr int CH = L < 4 ? L : 4;
-#pragma unroll 1
-    for (int q0 = 0; q0 < L; q0 += CH) {
-      int pb[CH], pe[CH];
+  for (int u = 0; u < NL; ++u) s[u] = (AT)0;
+  if (lr < X.rows) {
+    constexpr int B = NL < 8 ? NL : 8;           // entries in flight per round trip ...
+    constexpr int U = NL < 8 ? 8 / NL : 1;       // ... over U trips round the accumulators
+    if (X.staged) {
+      const VT* D = cl_dyn_words<VT>();
+      const int* rp = cl_dyn_words<int>() + X.rp;
+      const uint32_t* cg = cl_dyn_words<uint32_t>() + X.cg;
+      const int e = rp[lr + 1];
+      for (int p0 = rp[lr] + lig; p0 < e; p0 += U * L) {
 #pragma unroll
-      for (int q = 0; q < CH; ++q) {
-        const int lr = base + (q0 + q) * GPP + g;
-        pb[q] = 0; pe[q] = 0;
-        if (lr < X.rows) {
-          if (X.staged) { pb[q] = X.rp[lr] + lig; pe[q] = X.rp[lr + 1]; }
-          else { pb[q] = P.rowptr[X.r0 + lr] + lig; pe[q] = P.rowptr[X.r0 + lr + 1]; }
-        }
-      }
-      // the first entry of each of the CH rows: all gathers in flight at once
-      VT av[CH], xv[CH];
+        for (int b0 = 0; b0 < NL; b0 += B) {
+          VT av[U * B], xv[U * B];
+          uint32_t ad[U * B];
 #pragma unroll
-      for (int q = 0; q < CH; ++q) {
-        av[q] = (VT)0;
-        xv[q] = (VT)0;
-        if (pb[q] < pe[q]) {
-          if (X.staged) {
-            const int w = X.cg[pb[q]];
-            av[q] = X.vs[pb[q]];
-            xv[q] = cl_ld(cl_map(xbase + (w & 0xffffff), (unsigned)w >> 24), (VT)0);
-          } else {
-            const int gc = P.col[pb[q]];
-            const int o = gc / rc;
-            av[q] = P.val[pb[q]];
-            xv[q] = cl_ld(cl_map(xbase + (gc - o * rc), (unsigned)o), (VT)0);
+          for (int v = 0; v < U * B; ++v) {
+            const int p = p0 + (v / B) * L + (b0 + v % B) * lp;
+            ad[v] = (p < e) ? cg[p] : 0u;
+            av[v] = (p < e) ? D[X.vs + p] : (VT)0;
+          }
+#pragma unroll
+          for (int v = 0; v < U * B; ++v) {
+            const int p = p0 + (v / B) * L + (b0 + v % B) * lp;
+            if constexpr (XS) {
+              xv[v] = *(const VT*)((const char*)(D + X.xs) + ad[v]);
+            } else {
+              xv[v] = (VT)0;
+              if (p < e) xv[v] = cl_ld(ad[v] + xo * (int)sizeof(VT), (VT)0);
+            }
+          }
+#pragma unroll
+          for (int v = 0; v < U * B; ++v) {
+            const int p = p0 + (v / B) * L + (b0 + v % B) * lp;
+            if (p < e) s[b0 + v % B] += (AT)av[v] * (AT)xv[v];
           }
         }
       }
-      AT sacc[CH];
+    } else {
+      const int e = X.g_rowptr[X.r0 + lr + 1];
+      for (int p0 = X.g_rowptr[X.r0 + lr] + lig; p0 < e; p0 += U * L) {
 #pragma unroll
-      for (int q = 0; q < CH; ++q) {
-        sacc[q] = (AT)0;
-        if (pb[q] < pe[q]) sacc[q] += (AT)av[q] * (AT)xv[q];
-        if (X.staged) {
-          for (int p = pb[q] + L; p < pe[q]; p += L) {
-            const int w = X.cg[p];
-            sacc[q] += (AT)X.vs[p] * (AT)cl_ld(cl_map(xbase + (w & 0xffffff), (unsigned)w >> 24), (VT)0);
+        for (int b0 = 0; b0 < NL; b0 += B) {
+          VT av[U * B], xv[U * B];
+          int gc[U * B];
+#pragma unroll
+          for (int v = 0; v < U * B; ++v) {
+            const int p = p0 + (v / B) * L + (b0 + v % B) * lp;
+            gc[v] = (p < e) ? X.g_col[p] : -1;
+            av[v] = (p < e) ? X.g_val[p] : (VT)0;
           }
-        } else {
-          for (int p = pb[q] + L; p < pe[q]; p += L) {
-            const int gc = P.col[p];
-            const int o = gc / rc;
-            sacc[q] += (AT)P.val[p] * (AT)cl_ld(cl_map(xbase + (gc - o * rc), (unsigned)o), (VT)0);
+#pragma unroll
+          for (int v = 0; v < U * B; ++v) {
+            xv[v] = (VT)0;
+            if (gc[v] >= 0) {
+              if constexpr (XS) {
+                xv[v] = cl_dyn_words<VT>()[X.xs + gc[v]];
+              } else {
+                const int o = gc[v] / X.rc;
+                xv[v] = cl_ld(cl_map(cl_dyn_words<VT>() + xo + (gc[v] - o * X.rc), (unsigned)o), (VT)0);
+              }
+            }
           }
-        }
-      }
 #pragma unroll
-      for (int q = 0; q < CH; ++q) {
-#pragma unroll
-        for (int o = L >> 1; o > 0; o >>= 1) sacc[q] += __shfl_xor_sync(0xffffffffu, sacc[q], o);
-        if (lig == 0) sh.u.cys[(q0 + q) * GPP + g] = (VT)sacc[q];
-      }
-    }
-    __syncthreads();
-    const int lr = base + tid;
-    if (lr < X.rows) {
-      const VT y = sh.u.cys[tid] * xscale;
-      vout[lr] = y;
-      VT xn = (VT)0;
-      if (wq) {
-        xn = xbase[lr] * xscale;
-        X.Qs[(size_t)i * rc + lr] = xn;
-      }
-#pragma unroll
-      for (int c = 0; c < MP1; ++c) {
-        if (c <= i) {
-          const VT qc = (wq && c == i) ? xn : X.Qs[(size_t)c * rc + lr];
-          acc[c] += (AT)qc * (AT)y;
+          for (int v = 0; v < U * B; ++v)
+            if (gc[v] >= 0) s[b0 + v % B] += (AT)av[v] * (AT)xv[v];
         }
       }
     }
-    __syncthreads();
   }
-  block_reduce_cols(acc, i + 1, sh, part_out, 1);
+#pragma unroll
+  for (int o = NL / 2; o > 0; o >>= 1) {
+#pragma unroll
+    for (int u = 0; u < o; ++u) s[u] += s[u + o];
+  }
+  AT r = s[0];
+  for (int o = lp >> 1; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+  return (VT)r;
+}
+
+// vout = Op x * xscale for own rows; x and vout are offsets, the gathers read the
+// owner CTA's copy of x (or this CTA's copy of all of it)
+template <typename VT, int NL, bool XS>
+__device__ __forceinline__ void cl_spmv_rows(const ClCtx<VT>& X, int xo, VT xscale, int vout) {
+  const int lp = X.lp, gpp = LZ_BLOCK / lp;
+  const int g = threadIdx.x / lp, lig = threadIdx.x & (lp - 1);
+  for (int base = 0; base < X.rows; base += gpp) {
+    const VT s = cl_row_sum<VT, NL, XS>(X, base + g, lig, xo);
+    if (lig == 0 && base + g < X.rows) cl_dyn_words<VT>()[vout + base + g] = s * xscale;
+  }
+}
+template <typename VT, bool XS>
+__device__ __forceinline__ void cl_spmv(const ClCtx<VT>& X, int xo, VT xscale, int vout) {
+  switch (X.lanes / X.lp) {
+    case 1: cl_spmv_rows<VT, 1, XS>(X, xo, xscale, vout); break;
+    case 2: cl_spmv_rows<VT, 2, XS>(X, xo, xscale, vout); break;
+    case 4: cl_spmv_rows<VT, 4, XS>(X, xo, xscale, vout); break;
+    case 8: cl_spmv_rows<VT, 8, XS>(X, xo, xscale, vout); break;
+    case 16: cl_spmv_rows<VT, 16, XS>(X, xo, xscale, vout); break;
+    default: cl_spmv_rows<VT, 32, XS>(X, xo, xscale, vout); break;
+  }
+}
+
+// xs = x: warps take blocks of 256 rows of one owner CTA (starting with the next
+// CTA, so that the cluster's CTAs read from different peers), eight consecutive
+// 32-word rows of loads in flight per warp
+template <typename VT>
+__device__ __forceinline__ void cl_stage_x(const ClCtx<VT>& X, int xo) {
+  VT* D = cl_dyn_words<VT>();
+  const int lane = threadIdx.x & 31, parts = (X.rc + 255) / 256;
+  for (int id = threadIdx.x >> 5; id < X.C * parts; id += LZ_NW) {
+    const int part = id / X.C;
+    int o = X.rank + 1 + id - part * X.C;
+    if (o >= X.C) o -= X.C;
+    const int j0 = part * 256 + lane, rows = min(X.rc, X.n - o * X.rc);
+    const uint32_t src = cl_map(D + xo + j0, (unsigned)o);
+    VT v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      v[u] = (VT)0;
+      if (j0 + 32 * u < rows) v[u] = cl_ld(src + 32 * u * (int)sizeof(VT), (VT)0);
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (j0 + 32 * u < rows) D[X.xs + o * X.rc + j0 + 32 * u] = v[u];
+  }
+}
+
+// Columns c0 .. c0 + CW - 1 of the partial dots of one row-warp: acc[c] over its
+// rows, then summed across the warp by a butterfly whose payload halves while
+// more than one column is left (distance 16, 8, 4, 2, 1: the association of a
+// plain warp sum), to sh.u.st.wred[rw][c].
+template <int CW, typename VT>
+__device__ __forceinline__ void cl_warp_cols(typename Acc<VT>::type* acc, LzShared<VT>& sh,
+                                             int rw, int c0) {
+  typedef typename Acc<VT>::type AT;
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int h = 16, w = CW; h >= 1; h >>= 1) {
+    if (w > 1) {
+      w >>= 1;
+      const bool up = (lane & h) != 0;
+#pragma unroll
+      for (int j = 0; j < CW / 2; ++j) {
+        if (j < w) {
+          const AT send = up ? acc[j] : acc[j + w];
+          const AT keep = up ? acc[j + w] : acc[j];
+          acc[j] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+        }
+      }
+    } else {
+      acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], h);
+    }
+  }
+  constexpr int LPC = 32 / CW;                   // lanes that hold one column
+  if (lane % LPC == 0) sh.u.st.wred[rw][c0 + lane / LPC] = (double)acc[0];
+}
+
+// out[c] = sum over the nrw row-warps, in their order, of wred[.][c], c < nv
+template <typename VT>
+__device__ __forceinline__ void cl_block_cols(LzShared<VT>& sh, int nrw, int nv, double* out) {
+  __syncthreads();
+  for (int c = threadIdx.x; c < nv; c += LZ_BLOCK) {
+    double s = 0.0;
+#pragma unroll
+    for (int w = 0; w < LZ_NW; ++w)
+      if (w < nrw) s += sh.u.st.wred[w][c];
+    out[c] = s;
+  }
+}
+
+// A thread's rows are taken RT at a time (lr, lr + 256, ...).  In FP32 the loads
+// and FMA chains of three rows overlap (CTAs of at most 256 rows: one); in FP64 one row's chain already
+// keeps its pipe busy (64 cycles per instruction).
+template <typename VT> constexpr int cl_rt() { return sizeof(VT) == 4 ? 3 : 1; }
+
+// G columns c0 .. of a thread's RT rows; with PART, those at or past nv as 0.
+// Rows past the CTA's last are read too (whatever follows them in the layout;
+// their results are not used): the row offsets stay immediates.
+template <int RT, int G, bool PART, typename VT>
+__device__ __forceinline__ void cl_ld_cols(const ClCtx<VT>& X, int lr, int c0, int nv,
+                                           VT (&q)[RT][G]) {
+  const VT* D = cl_dyn_words<VT>() + c0 * X.rc + lr;
+#pragma unroll
+  for (int c = 0; c < G; ++c) {
+#pragma unroll
+    for (int r = 0; r < RT; ++r)
+      q[r][c] = (!PART || c0 + c < nv) ? D[c * X.rc + r * LZ_BLOCK] : (VT)0;
+  }
+}
+template <typename VT>
+__device__ __forceinline__ void cl_hv8(const LzShared<VT>& sh, int c0, VT (&h)[8]) {
+  if constexpr (sizeof(VT) == 4) {
+    const float4 a = *(const float4*)(sh.hv + c0), b = *(const float4*)(sh.hv + c0 + 4);
+    h[0] = a.x; h[1] = a.y; h[2] = a.z; h[3] = a.w;
+    h[4] = b.x; h[5] = b.y; h[6] = b.z; h[7] = b.w;
+  } else {
+#pragma unroll
+    for (int c = 0; c < 8; c += 2) {
+      const double2 a = *(const double2*)(sh.hv + c0 + c);
+      h[c] = a.x; h[c + 1] = a.y;
+    }
+  }
+}
+
+// acc[c] += Q[lr, c] y over a thread's RT rows lr, lr + 256, ..., c < nv
+template <int RT, bool PART, typename VT>
+__device__ __forceinline__ void cl_dot8(const ClCtx<VT>& X, int lr, int g, int nv,
+                                        const VT (&y)[RT], typename Acc<VT>::type* acc) {
+  typedef typename Acc<VT>::type AT;
+  VT q[RT][8];
+  cl_ld_cols<RT, 8, PART>(X, lr, g, nv, q);
+#pragma unroll
+  for (int r = 0; r < RT; ++r)
+    if (lr + r * LZ_BLOCK < X.rows) {
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+        if (!PART || g + c < nv) acc[c] += (AT)q[r][c] * (AT)y[r];
+    }
+}
+template <int RT, typename VT>
+__device__ __forceinline__ void cl_dot_rows(const ClCtx<VT>& X, int lr, int nv, int vec,
+                                            typename Acc<VT>::type* acc) {
+  VT y[RT];
+#pragma unroll
+  for (int r = 0; r < RT; ++r) y[r] = cl_dyn_words<VT>()[vec + lr + r * LZ_BLOCK];
+#pragma unroll
+  for (int g = 0; g < 32; g += 8) {
+    if (RT == 1 && g + 8 <= nv) cl_dot8<RT, false>(X, lr, g, nv, y, acc + g);
+    else if (g < nv) cl_dot8<RT, true>(X, lr, g, nv, y, acc + g);
+  }
+}
+
+// Partial dots Q[:, c] . vec, c < nv <= 32, over the CTA's rows.  Lane l of
+// row-warp w accumulates rows 32 w + l, 32 w + l + 256, ...; CTAs with at most
+// 128, 64 or 32 rows have 4, 2 or 1 row-warps and give each 2, 4 or 8 warps,
+// which split the columns, so that all four SM sub-partitions (and their FP64
+// pipes) work.  vec may just have been written by other threads.
+template <int CW, typename VT>
+__device__ __forceinline__ void cl_dots_w(const ClCtx<VT>& X, LzShared<VT>& sh, int nv, int vec,
+                                          double* part_out) {
+  typedef typename Acc<VT>::type AT;
+  constexpr int NRW = CW / 4;                    // row-warps: 8 CW / 32
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int rw = wid % NRW, c0 = (wid / NRW) * CW;
+  AT acc[CW];
+#pragma unroll
+  for (int c = 0; c < CW; ++c) acc[c] = (AT)0;
+  if (c0 < nv) {
+    if constexpr (CW == 32) {
+      constexpr int RT = cl_rt<VT>();
+      for (int lr = threadIdx.x; lr - lane < X.rows; lr += RT * LZ_BLOCK) {
+        if (RT > 1 && X.rows > LZ_BLOCK) cl_dot_rows<RT>(X, lr, nv, vec, acc);
+        else cl_dot_rows<1>(X, lr, nv, vec, acc);
+      }
+    } else {
+      const int lr = 32 * rw + lane;             // at most one row per lane
+      if (lr < X.rows) {
+        const VT y = cl_dyn_words<VT>()[vec + lr];
+        VT q[1][CW];
+        cl_ld_cols<1, CW, true>(X, lr, c0, nv, q);
+#pragma unroll
+        for (int c = 0; c < CW; ++c)
+          if (c0 + c < nv) acc[c] += (AT)q[0][c] * (AT)y;
+      }
+    }
+    cl_warp_cols<CW>(acc, sh, rw, c0);
+  }
+  cl_block_cols(sh, NRW, nv, part_out);
+}
+template <typename VT>
+__device__ __forceinline__ void cl_dots(const ClCtx<VT>& X, LzShared<VT>& sh, int nv, int vec,
+                                        double* part_out) {
+  if (X.rows > 128) cl_dots_w<32>(X, sh, nv, vec, part_out);
+  else if (X.rows > 64) cl_dots_w<16>(X, sh, nv, vec, part_out);
+  else if (X.rows > 32) cl_dots_w<8>(X, sh, nv, vec, part_out);
+  else cl_dots_w<4>(X, sh, nv, vec, part_out);
+}
+
+// Phase A: vout = Op (x * xscale) for own rows, partial Q[:, c] . vout (c <= i);
+// if wq, Q[:, i] = x * xscale (own rows)
+template <typename VT>
+__device__ __forceinline__ void cl_phase_spmv(const ClCtx<VT>& X, LzShared<VT>& sh, int i, int xo,
+                                              VT xscale, bool wq, int vout, double* part_out) {
+  VT* D = cl_dyn_words<VT>();
+  if (wq)
+    for (int lr = threadIdx.x; lr < X.rows; lr += LZ_BLOCK) D[i * X.rc + lr] = D[xo + lr] * xscale;
+  if (X.xs >= 0) {
+    cl_stage_x(X, xo);
+    __syncthreads();
+    cl_spmv<VT, true>(X, xo, xscale, vout);
+  } else {
+    cl_spmv<VT, false>(X, xo, xscale, vout);
+  }
+  __syncthreads();
+  cl_dots(X, sh, i + 1, vout, part_out);
 }
 
 template <typename VT>
 __device__ void cl_phase_random(const ClCtx<VT>& X, LzShared<VT>& sh, int nv, uint64_t key,
-                                VT* buf, double* part_out) {
-  typedef typename Acc<VT>::type AT;
-  const int rc = X.P->rc;
-  AT acc[MP1];
-#pragma unroll
-  for (int c = 0; c < MP1; ++c) acc[c] = (AT)0;
-  for (int lr = threadIdx.x; lr < X.rows; lr += LZ_BLOCK) {
-    const VT r = (VT)hash_normal(key, (uint64_t)(X.r0 + lr));
-    buf[lr] = r;
-#pragma unroll
-    for (int c = 0; c < MP1; ++c)
-      if (c < nv) acc[c] += (AT)X.Qs[(size_t)c * rc + lr] * (AT)r;
-  }
-  block_reduce_cols(acc, nv, sh, part_out, 1);
+                                int buf, double* part_out) {
+  for (int lr = threadIdx.x; lr < X.rows; lr += LZ_BLOCK)
+    cl_dyn_words<VT>()[buf + lr] = (VT)hash_normal(key, (uint64_t)(X.r0 + lr));
+  __syncthreads();
+  cl_dots(X, sh, nv, buf, part_out);
 }
 
-template <typename VT>
-__device__ void cl_phase_update_dot(const ClCtx<VT>& X, LzShared<VT>& sh, int nv, VT* buf,
-                                    double* part_out) {
-  typedef typename Acc<VT>::type AT;
-  const int rc = X.P->rc;
-  AT acc[MP1];
+// x[r] = buf[.] - sum_{c < nv} Q[., c] hv[c] in column order for a thread's RT
+// rows (lr, lr + 256, ...), written back to buf
+template <int RT, bool PART, typename VT>
+__device__ __forceinline__ void cl_combine8(const ClCtx<VT>& X, const LzShared<VT>& sh, int lr,
+                                            int g, int nv, VT (&s)[RT]) {
+  VT q[RT][8], h[8];
+  cl_ld_cols<RT, 8, PART>(X, lr, g, nv, q);
+  cl_hv8(sh, g, h);
 #pragma unroll
-  for (int c = 0; c < MP1; ++c) acc[c] = (AT)0;
-  for (int lr = threadIdx.x; lr < X.rows; lr += LZ_BLOCK) {
-    VT qr[MP1];
-    VT s = (VT)0;
+  for (int c = 0; c < 8; ++c)
+    if (!PART || g + c < nv) {
 #pragma unroll
-    for (int c = 0; c < MP1; ++c) {
-      if (c < nv) {
-        qr[c] = X.Qs[(size_t)c * rc + lr];
-        s += qr[c] * sh.hv[c];
-      }
+      for (int r = 0; r < RT; ++r) s[r] += q[r][c] * h[c];
     }
-    const VT q1 = buf[lr] - s;
-    buf[lr] = q1;
-#pragma unroll
-    for (int c = 0; c < MP1; ++c)
-      if (c < nv) acc[c] += (AT)qr[c] * (AT)q1;
-  }
-  block_reduce_cols(acc, nv, sh, part_out, 1);
 }
-
+template <int RT, typename VT>
+__device__ __forceinline__ void cl_combine(const ClCtx<VT>& X, const LzShared<VT>& sh, int nv,
+                                           int lr, int buf, VT* x) {
+  VT* D = cl_dyn_words<VT>() + buf + lr;
+  VT s[RT];
+#pragma unroll
+  for (int r = 0; r < RT; ++r) {
+    s[r] = (VT)0;
+    x[r] = D[r * LZ_BLOCK];
+  }
+  // one row: straight-line code for the groups of eight; three rows: a loop (a
+  // third of the code, and the rows overlap as it is)
+  if constexpr (RT == 1) {
+#pragma unroll
+    for (int g = 0; g < 32; g += 8) {
+      if (g + 8 <= nv) cl_combine8<RT, false>(X, sh, lr, g, nv, s);
+      else if (g < nv) cl_combine8<RT, true>(X, sh, lr, g, nv, s);
+    }
+  } else {
+#pragma unroll 1
+    for (int g = 0; g < nv; g += 8) cl_combine8<RT, true>(X, sh, lr, g, nv, s);
+  }
+#pragma unroll
+  for (int r = 0; r < RT; ++r) {
+    x[r] -= s[r];
+    if (lr + r * LZ_BLOCK < X.rows) D[r * LZ_BLOCK] = x[r];
+  }
+}
+// cl_combine of the rows that are left from lr on (at most RT), the squares of
+// the results added to nrm
 template <typename VT>
-__device__ void cl_phase_update_norm(const ClCtx<VT>& X, LzShared<VT>& sh, int nv, VT* buf,
-                                     double* part_out) {
+__device__ __forceinline__ void cl_update_rows(const ClCtx<VT>& X, const LzShared<VT>& sh, int nv,
+                                               int lr, int buf, typename Acc<VT>::type& nrm) {
   typedef typename Acc<VT>::type AT;
-  const int rc = X.P->rc;
-  AT nrm = (AT)0;
-  for (int lr = threadIdx.x; lr < X.rows; lr += LZ_BLOCK) {
-    VT s = (VT)0;
+  constexpr int RT = cl_rt<VT>();
+  VT x[RT];
+  if (RT > 1 && X.rows > LZ_BLOCK) cl_combine<RT>(X, sh, nv, lr, buf, x);
+  else cl_combine<1>(X, sh, nv, lr, buf, x);
 #pragma unroll
-    for (int c = 0; c < MP1; ++c)
-      if (c < nv) s += X.Qs[(size_t)c * rc + lr] * sh.hv[c];
-    const VT q2 = buf[lr] - s;
-    buf[lr] = q2;
-    nrm += (AT)q2 * (AT)q2;
-  }
-  AT one[MP1];
-  one[0] = nrm;
-  block_reduce_cols(one, 1, sh, part_out, 1);
+  for (int r = 0; r < RT; ++r)
+    if (lr + r * LZ_BLOCK < X.rows) nrm += (AT)x[r] * (AT)x[r];
 }
 
+// Phase B: buf -= Q h (c < nv); partial Q[:, c] . buf
 template <typename VT>
-__device__ void cl_spmv_dispatch(const ClCtx<VT>& X, LzShared<VT>& sh, int i, const VT* xbase,
-                                 VT xscale, bool wq, VT* vout, double* part_out) {
-  switch (X.P->lanes) {
-    case 1: cl_phase_spmv<VT, 1>(X, sh, i, xbase, xscale, wq, vout, part_out); break;
-    case 2: cl_phase_spmv<VT, 2>(X, sh, i, xbase, xscale, wq, vout, part_out); break;
-    case 4: cl_phase_spmv<VT, 4>(X, sh, i, xbase, xscale, wq, vout, part_out); break;
-    case 8: cl_phase_spmv<VT, 8>(X, sh, i, xbase, xscale, wq, vout, part_out); break;
-    case 16: cl_phase_spmv<VT, 16>(X, sh, i, xbase, xscale, wq, vout, part_out); break;
-    default: cl_phase_spmv<VT, 32>(X, sh, i, xbase, xscale, wq, vout, part_out); break;
-  }
+__device__ __forceinline__ void cl_phase_update_dot(const ClCtx<VT>& X, LzShared<VT>& sh, int nv,
+                                                    int buf, double* part_out) {
+  const int lane = threadIdx.x & 31;
+  typename Acc<VT>::type unused = 0;
+  for (int lr = threadIdx.x; lr - lane < X.rows; lr += cl_rt<VT>() * LZ_BLOCK)
+    cl_update_rows(X, sh, nv, lr, buf, unused);
+  __syncthreads();
+  cl_dots(X, sh, nv, buf, part_out);
+}
+
+// Phase C: buf -= Q h (c < nv); part_out[0] = sum buf^2 over own rows
+template <typename VT>
+__device__ __forceinline__ void cl_phase_update_norm(const ClCtx<VT>& X, LzShared<VT>& sh, int nv,
+                                                     int buf, double* part_out) {
+  const int lane = threadIdx.x & 31;
+  typename Acc<VT>::type nrm = 0;
+  for (int lr = threadIdx.x; lr - lane < X.rows; lr += cl_rt<VT>() * LZ_BLOCK)
+    cl_update_rows(X, sh, nv, lr, buf, nrm);
+  nrm = warp_sum(nrm);
+  if (lane == 0) sh.u.st.wred[threadIdx.x >> 5][0] = (double)nrm;
+  cl_block_cols(sh, min(LZ_NW, (X.rows + 31) / 32), 1, part_out);
 }
 
 template <typename VT>
 __global__ void __launch_bounds__(LZ_BLOCK, 1)
 lanczos_cluster_kernel(const __grid_constant__ ClusterBatch<VT> batch) {
-  __shared__ LzShared<VT> sh;
-  extern __shared__ __align__(16) unsigned char cl_dyn[];
+  __shared__ __align__(16) LzShared<VT> sh;
   const int C = batch.csize;
   const ClusterDesc<VT>& P = batch.t[blockIdx.x / C];
   const int rank = (int)cl_rank();
@@ -1637,34 +2015,62 @@ lanczos_cluster_kernel(const __grid_constant__ ClusterBatch<VT> batch) {
   const int n = P.n, m = P.m, rc = P.rc;
   const size_t ld = (size_t)P.ld;
   const ClLayout Lo = cl_layout<VT>(m, rc, P.csr_cap);
+  VT* D = cl_dyn_words<VT>();
   ClCtx<VT> X;
-  X.P = &P;
   X.rank = rank;
   X.C = C;
+  X.n = n;
+  X.m = m;
+  X.rc = rc;
   X.r0 = rank * rc;
   X.rows = max(0, min(rc, n - X.r0));
-  X.Qs = (VT*)(cl_dyn + Lo.q);
-  X.vb = (VT*)(cl_dyn + Lo.vb);
-  X.part = (double*)(cl_dyn + Lo.part);
-  X.rp = (int*)(cl_dyn + Lo.rp);
-  X.cg = (int*)(cl_dyn + Lo.cg);
-  X.vs = (VT*)(cl_dyn + Lo.val);
-  double* part0 = X.part;
-  double* part1 = X.part + MP1;
-  double* part2 = X.part + 2 * MP1;
+  X.lanes = P.lanes;
+  X.rp = (int)(Lo.rp / sizeof(int));
+  X.cg = (int)(Lo.cg / sizeof(int));
+  X.vs = (int)(Lo.val / sizeof(VT));
+  X.g_rowptr = P.rowptr;
+  X.g_col = P.col;
+  X.g_val = P.val;
+  const int vb = (int)(Lo.vb / sizeof(VT));        // the two work vectors
+  double* part0 = cl_dyn_words<double>() + Lo.part / sizeof(double);
+  double* part1 = part0 + MP1;
+  double* part2 = part0 + 2 * MP1;
   // stage Q[:, 0] (the start vector) and, if it fits, the operator slice
-  for (int lr = tid; lr < X.rows; lr += LZ_BLOCK) X.Qs[lr] = P.Q[X.r0 + lr];
-  X.p0 = (X.rows > 0) ? P.rowptr[X.r0] : 0;
+  for (int lr = tid; lr < X.rows; lr += LZ_BLOCK) D[lr] = P.Q[X.r0 + lr];
+  const int p0 = (X.rows > 0) ? P.rowptr[X.r0] : 0;
   const int p1 = (X.rows > 0) ? P.rowptr[X.r0 + X.rows] : 0;
-  X.staged = (p1 - X.p0) <= P.csr_cap;
+  X.staged = (p1 - p0) <= P.csr_cap;
+  X.lp = 1;
+  // (a slice read from global memory keeps one thread per accumulator: its
+  // consecutive entries are then consecutive lanes')
+  while (2 * X.lp <= X.lanes && (!X.staged || 2 * X.lp * X.rows <= LZ_BLOCK)) X.lp *= 2;
+  X.xs = -1;
   if (X.staged) {
-    for (int lr = tid; lr <= X.rows; lr += LZ_BLOCK) X.rp[lr] = P.rowptr[X.r0 + lr] - X.p0;
-    for (int p = X.p0 + tid; p < p1; p += LZ_BLOCK) {
+    int* rp = cl_dyn_words<int>() + X.rp;
+    uint32_t* cg = cl_dyn_words<uint32_t>() + X.cg;
+    int remote = 0;
+    for (int p = p0 + tid; p < p1; p += LZ_BLOCK) {
       const int gc = P.col[p];
-      const int o = gc / rc;
-      X.cg[p - X.p0] = (o << 24) | (gc - o * rc);
-      X.vs[p - X.p0] = P.val[p];
+      remote += (gc < X.r0 || gc >= X.r0 + X.rows) ? 1 : 0;
+      cg[p - p0] = (uint32_t)gc;
+      D[X.vs + p - p0] = P.val[p];
     }
+    for (int lr = tid; lr <= X.rows; lr += LZ_BLOCK) rp[lr] = P.rowptr[X.r0 + lr] - p0;
+    remote = (int)block_sum((double)remote, sh.red);
+    // A copy of all of x where there is room for it and the rows' entries in
+    // other CTAs number at least a quarter of it: the copy reads consecutive
+    // words of its peers, the gather scattered ones.  Phase A in kilocycles per
+    // step, copied / gathered (16 CTAs): ER n = 5000 degree 30 FP32 11.6 / 32,
+    // degree 8 8.7 / 12.4, n = 9000 degree 6 11.2 / 15, n = 800 degree 48 FP64
+    // 9.1 / 13; below the line, torus n = 2500 FP32 5.2 / 3.7 (few peers).
+    const int used = (p1 - p0 + 3) & ~3;
+    if (P.csr_cap - used >= n && 4 * remote >= n) X.xs = X.vs + used;
+    for (int p = tid; p < p1 - p0; p += LZ_BLOCK) {
+      const int gc = (int)cg[p], o = gc / rc;
+      cg[p] = X.xs >= 0 ? (uint32_t)(gc * (int)sizeof(VT)) : cl_map(D + (gc - o * rc), (unsigned)o);
+    }
+  } else if ((size_t)P.csr_cap * (sizeof(int) + sizeof(VT)) >= (size_t)n * sizeof(VT)) {
+    X.xs = (int)(Lo.cg / sizeof(VT));     // the operator stays in global memory: the room is x's
   }
   int k = 0, nconv = 0, restart = 0, breakdowns = 0, steps = 0, sum_nv = 0, sum_kn = 0;
   long long clk_start = clock64(), clk_restart = 0;
@@ -1679,10 +2085,10 @@ lanczos_cluster_kernel(const __grid_constant__ ClusterBatch<VT> batch) {
   while (nconv < P.num_desired && restart < P.max_restarts) {
     int cur = 0;
     for (int i = k; i < m; ++i) {
-      const VT* xbase;
+      int xbase;
       bool wq;
       if (i == k) {
-        xbase = X.Qs + (size_t)k * rc;
+        xbase = k * rc;
         invb = (VT)1;
         wq = false;
       } else {
@@ -1693,7 +2099,7 @@ lanczos_cluster_kernel(const __grid_constant__ ClusterBatch<VT> batch) {
           // Krylov space exhausted: random vector orthogonalised twice
           // against Q[:, :i] (solver/lanczos.py:107-117)
           ++breakdowns;
-          VT* buf = X.vb + (size_t)prev * rc;
+          const int buf = vb + prev * rc;
           cl_phase_random(X, sh, i, (uint64_t)i, buf, part0);
           cl_sync();
           cl_reduce(part0, C, i, sh);
@@ -1707,12 +2113,12 @@ lanczos_cluster_kernel(const __grid_constant__ ClusterBatch<VT> batch) {
         } else {
           invb = sh.binv;
         }
-        xbase = X.vb + (size_t)prev * rc;
+        xbase = vb + prev * rc;
         wq = true;
       }
-      VT* vout = X.vb + (size_t)cur * rc;
+      const int vout = vb + cur * rc;
       if (timing) { const long long c = clock64(); tp[1] += c - tmark; tmark = c; }
-      cl_spmv_dispatch(X, sh, i, xbase, invb, wq, vout, part0);
+      cl_phase_spmv(X, sh, i, xbase, invb, wq, vout, part0);
       if (timing) { const long long c = clock64(); tp[2] += c - tmark; tmark = c; }
       cl_sync();
       if (timing) { const long long c = clock64(); tp[0] += c - tmark; tmark = c; }
@@ -1743,7 +2149,7 @@ lanczos_cluster_kernel(const __grid_constant__ ClusterBatch<VT> batch) {
       if (tid == 0) sh.beta[m - 1] = b;
       if (b < 1e-15) {
         ++breakdowns;
-        VT* buf = X.vb + (size_t)prev * rc;
+        const int buf = vb + prev * rc;
         cl_phase_random(X, sh, m, (uint64_t)m, buf, part0);
         cl_sync();
         cl_reduce(part0, C, m, sh);
@@ -1760,30 +2166,45 @@ lanczos_cluster_kernel(const __grid_constant__ ClusterBatch<VT> batch) {
     }
     __syncthreads();
     const long long c0 = clock64();
-    restart_select<true>(P, sh, k, /*write_out=*/rank == 0);
+    restart_select<true>(P, sh, k, /*write_out=*/rank == 0, rank, C);
     if (timing) clk_restart += clock64() - c0;
     // every CTA of the cluster found the same projected matrix, so all of
     // them see their own ST_NONFINITE here and leave together
     if (*(volatile int*)P.status & ST_NONFINITE) { ++restart; break; }
     const int kn = sh.k_next;
     nconv = sh.nconv;
-    const VT* last = stepped ? (X.vb + (size_t)prev * rc) : (X.Qs + (size_t)m * rc);
+    const VT* last = D + (stepped ? vb + prev * rc : m * rc);
     const VT lscale = stepped ? invb : (VT)1;
     for (int lr = tid; lr < X.rows; lr += LZ_BLOCK) {
       VT qr[MAXM];
 #pragma unroll
-      for (int j = 0; j < MAXM; ++j) qr[j] = (j < m) ? X.Qs[(size_t)j * rc + lr] : (VT)0;
+      for (int j = 0; j < MAXM; ++j) qr[j] = (j < m) ? D[j * rc + lr] : (VT)0;
       const VT xl = last[lr] * lscale;
-      for (int c = 0; c < kn; ++c) {
-        if (c >= m) break;
-        VT s = (VT)0;
+      // four output columns per pass, their Y entries read together (Y is zero
+      // past column kn, so the last pass may overrun kn)
+      for (int c0 = 0; c0 < kn; c0 += 4) {
+        VT s[4] = {(VT)0, (VT)0, (VT)0, (VT)0};
 #pragma unroll
         for (int j = 0; j < MAXM; ++j)
-          if (j < m) s += qr[j] * sh.u.Ys[j * MAXM + c];
-        X.Qs[(size_t)c * rc + lr] = s;
+          if (j < m) {
+            VT y4[4];
+            if constexpr (sizeof(VT) == 4) {
+              const float4 a = *(const float4*)&sh.u.Ys[j * MAXM + c0];
+              y4[0] = a.x; y4[1] = a.y; y4[2] = a.z; y4[3] = a.w;
+            } else {
+              const double2 a = *(const double2*)&sh.u.Ys[j * MAXM + c0];
+              const double2 b = *(const double2*)&sh.u.Ys[j * MAXM + c0 + 2];
+              y4[0] = a.x; y4[1] = a.y; y4[2] = b.x; y4[3] = b.y;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) s[u] += qr[j] * y4[u];
+          }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (c0 + u < kn) D[(c0 + u) * rc + lr] = s[u];
       }
-      X.Qs[(size_t)kn * rc + lr] = xl;
-      if (kn != m) X.Qs[(size_t)m * rc + lr] = xl;
+      D[kn * rc + lr] = xl;
+      if (kn != m) D[m * rc + lr] = xl;
     }
     k = kn;
     sum_kn += kn;
@@ -1796,7 +2217,7 @@ lanczos_cluster_kernel(const __grid_constant__ ClusterBatch<VT> batch) {
   if (restart > 0) {
     for (int c = 0; c <= m; ++c)
       for (int lr = tid; lr < X.rows; lr += LZ_BLOCK)
-        P.Q[(size_t)c * ld + X.r0 + lr] = X.Qs[(size_t)c * rc + lr];
+        P.Q[(size_t)c * ld + X.r0 + lr] = D[c * rc + lr];
   }
   if (rank == 0 && tid == 0) {
     P.ctl[2] = restart;
