@@ -443,6 +443,10 @@ int usbs_qap_round(int l, int s, const double* Omega, const double* P, int ld, c
 int usbs_selftest_wait_limits(int which, int nctas, long long limit_ns, unsigned int* counters,
                               int* status, void* stream);
 
+/* y[i] = 1 / x[i] by the interior-point kernels' integer reciprocal (n values,
+ * device pointers), for comparison with the IEEE division. */
+int usbs_selftest_recip(long long n, const double* x, double* y, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -7,13 +7,13 @@
 //    coordinates: Newton system (s x s) assembled from the symmetric Kronecker
 //    product T (x) S^-1 and solved by LU; line search over the step grid
 //    0.9^j, j < ipm_max_iters, keeping the largest step at which S + a dS and
-//    T + a dT stay positive definite (tested by Cholesky, one grid point per
-//    thread), exactly the reference's "smallest eigenvalue > 0" rule.
+//    T + a dT stay positive definite (32 LDL^T tests at a time), exactly the reference's "smallest eigenvalue > 0" rule.
 //  * eigS_kernel  eigh(S) of the bundle matrix and everything the outer
 //    iteration derives from it (solver/usbs.py:409-412, 568-585, 627-644).
 //  * cholqr_kernel  R^-1 of one (shifted) Cholesky-QR pass for the new bundle
 //    basis (replaces the Householder QR of solver/usbs.py:641-642).
 #include "common.cuh"
+#include "recip.cuh"
 #include "dense.cuh"
 #include "internal.h"
 #include "solver.h"
@@ -32,10 +32,7 @@ struct IpmShared {
   double q12[IPM_MAXS], h1[IPM_MAXS], sI[IPM_MAXS], sS[IPM_MAXS], sT[IPM_MAXS];
   double F1[IPM_MAXS], ord[IPM_MAXS], dsT[IPM_MAXS], sSi[IPM_MAXS];
   double S[IPM_MAXK * IPM_MAXK], T[IPM_MAXK * IPM_MAXK], Si[IPM_MAXK * IPM_MAXK];
-  double dS[IPM_MAXK * IPM_MAXK], dT[IPM_MAXK * IPM_MAXK], wk[IPM_MAXK * IPM_MAXK];
-  double redv[IPM_BLOCK / 32];
-  int redi[IPM_BLOCK / 32];
-  double lcol[IPM_MAXS];
+  double dS[IPM_MAXK * IPM_MAXK], dT[IPM_MAXK * IPM_MAXK];
   double dinv[IPM_MAXS];
   double u2[IPM_MAXS], w2[IPM_MAXS];   // per-column terms of the rank-2 correction
   int cord[IPM_MAXS];                  // svec indices, off-diagonal ones first
@@ -80,29 +77,72 @@ __device__ __forceinline__ double symkron_sum(const double* T, const double* X, 
   return (((b == c) == (b2 == c2)) ? 0.5 : RSQ2) * S;
 }
 
-// Positive-definiteness test of A + s dA (k x k, lower triangle) by LDL^T
-// without pivoting: PD iff every pivot is positive (equivalent to Cholesky
+// 32 positive-definiteness tests of M + step dM (k x k, lower triangle) by LDL^T
+// without pivoting, whole CTA, eight lanes each: test t < 16 is of (S, dS), the
+// others of (T, dT).  PD iff every pivot is positive (equivalent to Cholesky
 // succeeding, i.e. to the smallest eigenvalue being > 0, up to round-off at the
-// boundary).  One reciprocal per column, no square roots.
-// L holds the unit lower factor l_ip and U the unscaled l_ip d_p (packed lower
-// triangles), so each update term l_ip (l_jp d_p) is one FMA.
-__device__ __forceinline__ bool pd_test(const double* A, const double* dA, double s, int k) {
-  double L[IPM_MAXS], U[IPM_MAXS];
-  for (int j = 0; j < k; ++j) {
-    const int rj = j * (j + 1) / 2;
-    double d = A[j * k + j] + s * dA[j * k + j];
-    for (int p = 0; p < j; ++p) d -= L[rj + p] * U[rj + p];
-    if (!(d > 0.0)) return false;
-    const double inv = 1.0 / d;
-    for (int i = j + 1; i < k; ++i) {
-      const int ri = i * (i + 1) / 2;
-      double v = A[i * k + j] + s * dA[i * k + j];
-      for (int p = 0; p < j; ++p) v -= L[ri + p] * U[rj + p];
-      U[ri + j] = v;
-      L[ri + j] = v * inv;
+// boundary).  One reciprocal per column (on the integer pipes), no square roots.
+// Right-looking, the trailing triangle's entries dealt to the eight lanes: an
+// entry sees a_ij + s da_ij, then - l_ip u_jp for p = 0, 1, ..., u_jp = l_jp d_p,
+// one FMA each.  The FP64 unit takes a warp instruction every 19 cycles SM-wide
+// but one warp only every 60: with one lane per test on one warp a round of 32
+// tests took 26k cycles (k = 11).
+// ws: 32 (s + IPM_MAXK) doubles.  Returns the mask of the tests that passed.
+__device__ unsigned pd_tests(const double* S, const double* dS, const double* T, const double* dT,
+                             int k, int s, const int* bi, const int* ci, bool active, double step,
+                             double* ws, unsigned* mask) {
+  constexpr int G = 8, EU = (IPM_MAXS + G - 1) / G;
+  const int tid = threadIdx.x, lane = tid & 31, g = lane & (G - 1);
+  const int test = tid / G;
+  double* M = ws + test * (s + IPM_MAXK);
+  double* L = M + s;
+  const double* A = (test < 16) ? S : T;
+  const double* dA = (test < 16) ? dS : dT;
+  if (tid == 0) *mask = 0u;
+  int bc[EU];                          // packed coordinates of this lane's triangle entries
+#pragma unroll
+  for (int u = 0; u < EU; ++u) {
+    const int t = g + G * u;
+    bc[u] = (t < s) ? (bi[t] << 8) | ci[t] : 0;
+  }
+  bool pd = active;
+  if (active) {
+#pragma unroll
+    for (int u = 0; u < EU; ++u) {
+      const int t = g + G * u;
+      if (t < s) {
+        const int e = (bc[u] >> 8) * k + (bc[u] & 255);
+        M[t] = A[e] + step * dA[e];
+      }
     }
   }
-  return true;
+  __syncthreads();
+  for (int p = 0; p < k; ++p) {
+    const double d = pd ? M[p * (p + 1) / 2 + p] : 1.0;
+    if (!(d > 0.0)) pd = false;
+    if (__any_sync(0xffffffffu, pd)) {
+      const double inv = recip_exact(d);
+      for (int i = p + 1 + g; i < k; i += G)
+        if (pd) L[i] = M[i * (i + 1) / 2 + p] * inv;
+      __syncwarp();
+      const int m = (k - 1 - p) * (k - p) / 2;
+#pragma unroll
+      for (int u = 0; u < EU; ++u) {
+        if (G * u < m) {
+          const int t = g + G * u;
+          if (t < m && pd) {
+            const int i = p + 1 + (bc[u] >> 8), j = p + 1 + (bc[u] & 255);
+            double* v = M + i * (i + 1) / 2 + j;
+            *v -= L[i] * M[j * (j + 1) / 2 + p];
+          }
+        }
+      }
+    }
+    __syncwarp();
+  }
+  if (pd && g == 0) atomicOr(mask, 1u << test);
+  __syncthreads();
+  return *mask;
 }
 
 struct IpmScal {
@@ -125,69 +165,49 @@ __device__ __forceinline__ unsigned long long abs_key(double x) {
 }
 
 // Inverse of an n x n matrix (n <= IPM_MAXK, row-major, lda = n) by Gauss-Jordan
-// elimination with partial pivoting on [A | I], whole CTA: per pivot, warp 0
-// picks the row (largest |a|, ties to the smaller index), every thread then
-// updates one or two entries of the 2n-wide augmented rows.  Per element the
-// arithmetic is that of the row-by-row algorithm (pivot row scaled by 1/a_jj,
-// a_ic - a_ij * row_c).  A is destroyed.  Returns false if a pivot is zero.
-__device__ bool cta_inverse(double* A, int n, double* Ainv, double* fcol, int* piv_s,
-                            double* inv_s) {
-  const int tid = threadIdx.x, lane = tid & 31, nt = blockDim.x;
-  for (int e = tid; e < n * n; e += nt) Ainv[e] = ((e / n) == (e % n)) ? 1.0 : 0.0;
+// elimination with partial pivoting on [A | I], whole CTA.  ws holds two n x 2n
+// augmented matrices: a pivot step reads one and writes the other, so it takes
+// one barrier, and each thread forms one entry of the new matrix, the pivot row's
+// scaled entry included.  Every warp picks the pivot itself (largest |a| by
+// integer keys, ties to the smaller row) and forms its reciprocal on the integer
+// pipes.  Per element the arithmetic is that of the row-by-row algorithm (rows
+// j and piv exchanged, pivot row scaled by 1/a_jj, a_ic - a_ij * row_c).  Returns
+// false if a pivot is zero.  (With the exchange, the column copy, the scaling
+// and the update as four steps between barriers it took 28k cycles at n = 11.)
+__device__ bool cta_inverse(const double* A, int n, double* Ainv, double* ws) {
+  const int tid = threadIdx.x, lane = tid & 31, ld = 2 * n;
+  double* cur = ws;
+  double* nxt = ws + n * ld;
+  for (int e = tid; e < n * ld; e += IPM_BLOCK) {
+    const int i = e / ld, c = e - i * ld;
+    cur[e] = (c < n) ? A[i * n + c] : ((c - n == i) ? 1.0 : 0.0);
+  }
   bool ok = true;
   __syncthreads();
   for (int j = 0; j < n; ++j) {
-    if (tid < 32) {
-      // largest |a| key among rows j.., ties to the smaller row: warp reduction
-      // instructions on the high word, then the low word among the lanes
-      // holding the top high word, then the smallest row among ties
-      const bool valid = lane >= j && lane < n;
-      const unsigned long long key = valid ? abs_key(A[lane * n + j]) : 0ull;
-      const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
-      const unsigned mhi = __reduce_max_sync(0xffffffffu, valid ? hi : 0u);
-      const bool th = valid && hi == mhi;
-      const unsigned mlo = __reduce_max_sync(0xffffffffu, th ? lo : 0u);
-      const bool tl = th && lo == mlo;
-      const unsigned mrow = __reduce_min_sync(0xffffffffu, tl ? (unsigned)lane : 0xffffffffu);
-      int bi = (mrow == 0xffffffffu) ? 0x7fffffff : (int)mrow;
-      if (lane == 0) {
-        if (bi == 0x7fffffff) bi = j;
-        *piv_s = bi;
-        const double pv = A[bi * n + j];
-        *inv_s = (pv == 0.0) ? 0.0 : 1.0 / pv;
-      }
+    const bool valid = lane >= j && lane < n;
+    const double a = valid ? cur[lane * ld + j] : 0.0;
+    const unsigned long long key = abs_key(a);
+    const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
+    const unsigned mhi = __reduce_max_sync(0xffffffffu, valid ? hi : 0u);
+    const bool th = valid && hi == mhi;
+    const unsigned mlo = __reduce_max_sync(0xffffffffu, th ? lo : 0u);
+    const int piv = (int)__reduce_min_sync(0xffffffffu, (th && lo == mlo) ? (unsigned)lane : (unsigned)j + 32u) & 31;
+    const double pv = __shfl_sync(0xffffffffu, a, piv);
+    const bool zero = abs_key(pv) == 0ull;
+    const double inv = zero ? 0.0 : recip_exact(pv);
+    if (zero) ok = false;
+    for (int e = tid; e < n * ld; e += IPM_BLOCK) {
+      const int i = e / ld, c = e - i * ld;
+      const int src = (i == j) ? piv : (i == piv) ? j : i;
+      const double rowc = cur[piv * ld + c] * inv;
+      nxt[e] = (i == j) ? rowc : cur[src * ld + c] - cur[src * ld + j] * rowc;
     }
     __syncthreads();
-    const int piv = *piv_s;
-    const double inv = *inv_s;
-    if (inv == 0.0) ok = false;
-    if (piv != j) {
-      for (int c = tid; c < 2 * n; c += nt) {
-        double* M = (c < n) ? A : Ainv;
-        const int cc = (c < n) ? c : c - n;
-        const double t = M[j * n + cc];
-        M[j * n + cc] = M[piv * n + cc];
-        M[piv * n + cc] = t;
-      }
-      __syncthreads();
-    }
-    for (int i = tid; i < n; i += nt) fcol[i] = A[i * n + j];
-    __syncthreads();
-    for (int c = tid; c < 2 * n; c += nt) {
-      double* M = (c < n) ? A : Ainv;
-      const int cc = (c < n) ? c : c - n;
-      M[j * n + cc] *= inv;
-    }
-    __syncthreads();
-    for (int e = tid; e < n * 2 * n; e += nt) {
-      const int i = e / (2 * n), c = e - i * 2 * n;
-      if (i == j) continue;
-      double* M = (c < n) ? A : Ainv;
-      const int cc = (c < n) ? c : c - n;
-      M[i * n + cc] -= fcol[i] * M[j * n + cc];
-    }
-    __syncthreads();
+    double* t = cur; cur = nxt; nxt = t;
   }
+  for (int e = tid; e < n * n; e += IPM_BLOCK) Ainv[e] = cur[(e / n) * ld + n + e % n];
+  __syncthreads();
   return ok;
 }
 
@@ -209,177 +229,200 @@ __device__ void cta_matvec3(const double* M, const double* x, int s, double* par
 
 // LU with partial pivoting and solve, whole CTA (G&VL Alg. 3.4.1, right-looking
 // with a one-column look-ahead).  A is stored column-major (A[c * lda + i] is
-// row i, column c), so every column access of the pivot chain is contiguous.
-// On GB300 an FP64 warp instruction holds its SM sub-partition's FP64 pipe for
-// 64 cycles, so the pivot chain of each column is kept off the critical path:
-// while warps 1..7 eliminate b and apply the rank-1 update of column j to
-// columns j+2.., warp 0 updates column j+1 (lane q holds rows j+1+q, j+33+q,
-// j+65+q in registers, and only the blocks that still hold rows take part),
-// picks the next pivot from those registers (largest |a|, ties to the smaller
-// row index as in LAPACK; warp reduction instructions on the integer keys of
-// |a|), forms its reciprocal and the next multipliers.  Rows are swapped
-// physically at the start of each column.  L is not stored: b is eliminated
-// alongside.  Every element sees the arithmetic of the textbook algorithm
+// row i, column c).  Every element sees the arithmetic of the textbook algorithm
 // (a_ic - l_i a_jc, l_i = a_ij * (1/a_jj)).  Partial pivoting is needed: in
 // the bundle subproblems' Newton systems about two thirds of the
 // factorisations exchange rows somewhere.
-constexpr int LU_RPL = (IPM_MAXS + 31) / 32;   // rows per lane of warp 0
-__device__ void ipm_lu_solve(double* A, int lda, double* b, int n, double* dinv, double* lcol,
-                             int* ok_out) {
-  const int tid = threadIdx.x, lane = tid & 31;
-  __shared__ double lnext[IPM_MAXS];
-  __shared__ int pnext[2];   // pivot of column j in pnext[j & 1] (written one column ahead)
-  double* lc = lcol;         // multipliers of the current column (indexed by row)
-  double* ln = lnext;        // multipliers of the next column
-  // warp 0: rows r = j + lane + 32 q of column j are in v[q] (q < nq); pivot,
-  // reciprocal and multipliers of column j
-  auto pick = [&](int j, const double (&v)[LU_RPL], double* lout, int nq) {
-    // lane-local candidate: largest |a| key, smallest row among equal keys
-    unsigned long long best = 0ull;
-    int bi = 0x7fffffff;
+// On GB300 the SM's FP64 unit takes one warp instruction every 19 cycles, a single
+// warp one every 60, and the trailing update is bound by it while more than about
+// 40 positions are left; below, a column's pivot chain (one FMA, the argmax, the
+// reciprocal, the multipliers) is a sequence of latencies that bounds the
+// factorisation.  So while the other warps eliminate b and
+// apply the rank-1 update of column j to columns j+2.., warp 0 alone takes
+// column j+1 through registers: lane l keeps positions n-1-l, n-33-l, n-65-l (a
+// position's row, its value in the current column and its multiplier), and only
+// the register blocks that still hold positions take part.  Rows are not moved:
+// the exchange swaps two rows' positions, in registers and in the list of rows
+// by position that warp 0 hands over with the multipliers (double-buffered, so
+// one barrier per column).  The pivot is the largest |a| by integer keys, ties to
+// the smaller position as in LAPACK.  The column itself is not written back (L is
+// not stored, and U needs only the rows above).
+// The loops are specialised by the number of register blocks: straight-line code
+// for three of them in one loop made a column of the smallest systems 2.0k cycles,
+// fetching instructions; 1.2k as it is.  Order 66: 126k cycles (153k with rows
+// exchanged in memory between barriers), order 15 18k (31k).  Four trailing
+// warps instead of seven, or several elements in flight per thread, are slower
+// (order 66: 160-350k).
+constexpr int LU_RPL = (IPM_MAXS + 31) / 32;   // register blocks of 32 positions
+struct LuShared {
+  double lb[2][IPM_MAXS];    // multipliers by position, of even and odd columns
+  int rows[2][IPM_MAXS];     // row by position, after the exchange of even and odd columns
+  int prow[IPM_MAXS];        // pivot rows
+};
+// warp 0's registers
+struct LuRegs {
+  double v[LU_RPL], l[LU_RPL];
+  int row[LU_RPL], pr;
+};
+
+// warp 0: R.v holds column j at positions j.. (in NQ register blocks); its pivot,
+// reciprocal, multipliers and the exchange of positions
+template <int NQ>
+__device__ __forceinline__ void lu_pick(LuRegs& R, LuShared& S, int j, int n, double* dinv,
+                                        int* ok_out) {
+  const int lane = threadIdx.x & 31, p0 = n - 1 - lane;
+  // lane-local candidate: largest |a| key, smallest position among equal keys
+  unsigned long long best = abs_key(R.v[0]);
+  int bp = p0;
 #pragma unroll
-    for (int q = 0; q < LU_RPL; ++q) {
-      const int i = j + lane + 32 * q;
-      if (q < nq && i < n) {
-        const unsigned long long kk = abs_key(v[q]);
-        if (bi == 0x7fffffff || kk > best) { best = kk; bi = i; }
-      }
-    }
-    // warp argmax by reduction instructions: high word, then low word among
-    // the lanes holding the top high word, then the smallest row among ties
-    const unsigned hi = (unsigned)(best >> 32), lo = (unsigned)best;
-    const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
-    const bool th = (bi != 0x7fffffff) && hi == mhi;
-    const unsigned mlo = __reduce_max_sync(0xffffffffu, th ? lo : 0u);
-    const bool tl = th && lo == mlo;
-    const unsigned mrow = __reduce_min_sync(0xffffffffu, tl ? (unsigned)bi : 0xffffffffu);
-    double bv;
-    if (mrow == 0xffffffffu) {
-      bi = j;
-      bv = A[(size_t)j * lda + j];
-    } else {
-      bi = (int)mrow;
-      const int off = bi - j;           // the row's owner lane and register
-      double sel = 0.0;
-#pragma unroll
-      for (int q = 0; q < LU_RPL; ++q) if (q == (off >> 5)) sel = v[q];
-      bv = __shfl_sync(0xffffffffu, sel, off & 31);
-    }
-    const double inv = (bv == 0.0) ? 1.0 : 1.0 / bv;
-#pragma unroll
-    for (int q = 0; q < LU_RPL; ++q) {
-      const int i = j + lane + 32 * q;
-      if (q < nq && i < n) lout[i] = v[q] * inv;
-    }
-    if (lane == 0) {
-      pnext[j & 1] = bi;
-      dinv[j] = inv;
-      if (bv == 0.0) *ok_out = 0;
-    }
-  };
-  if (tid == 0) *ok_out = 1;
-  __syncthreads();
-  if (tid < 32) {
-    double v[LU_RPL];
-#pragma unroll
-    for (int q = 0; q < LU_RPL; ++q) {
-      const int i = lane + 32 * q;
-      v[q] = (i < n) ? A[i] : 0.0;
-    }
-    pick(0, v, lc, LU_RPL);
+  for (int q = 1; q < NQ; ++q) {
+    const unsigned long long k = abs_key(R.v[q]);
+    if (p0 - 32 * q >= j && k >= best) { best = k; bp = p0 - 32 * q; }
   }
-  __syncthreads();
-  for (int j = 0; j < n; ++j) {
-    const int piv = pnext[j & 1];
-    // swap rows j and piv (columns j.., b and the multipliers of column j)
-    if (piv != j) {
-      for (int c = j + tid; c < n; c += blockDim.x) {
-        const double t = A[c * lda + j];
-        A[c * lda + j] = A[c * lda + piv];
-        A[c * lda + piv] = t;
-      }
-      if (tid == 0) {
-        const double t = b[j]; b[j] = b[piv]; b[piv] = t;
-        lc[piv] = lc[j];
-      }
-      __syncthreads();
+  // warp argmax by reduction instructions: high word, then low word among
+  // the lanes holding the top high word, then the smallest position among ties
+  const bool cand = bp >= j;
+  const unsigned hi = (unsigned)(best >> 32), lo = (unsigned)best;
+  const unsigned mhi = __reduce_max_sync(0xffffffffu, cand ? hi : 0u);
+  const bool th = cand && hi == mhi;
+  const unsigned mlo = __reduce_max_sync(0xffffffffu, th ? lo : 0u);
+  const int bi = (int)__reduce_min_sync(0xffffffffu, (th && lo == mlo) ? (unsigned)bp : 0x7fffffffu);
+  const int bo = n - 1 - bi, jo = n - 1 - j;      // their owner lanes and blocks
+  double bsel = R.v[0], jsel = R.v[NQ - 1];       // position j is in the last block
+  int brow = R.row[0], jrow = R.row[NQ - 1];
+#pragma unroll
+  for (int q = 1; q < NQ; ++q)
+    if (q == (bo >> 5)) { bsel = R.v[q]; brow = R.row[q]; }
+  const double bv = __shfl_sync(0xffffffffu, bsel, bo & 31);
+  R.pr = __shfl_sync(0xffffffffu, brow, bo & 31);
+  jsel = __shfl_sync(0xffffffffu, jsel, jo & 31);
+  jrow = __shfl_sync(0xffffffffu, jrow, jo & 31);
+  const bool zero = (abs_key(bv) == 0ull);
+  const double inv = recip_exact(zero ? 1.0 : bv);
+  double* lj = S.lb[j & 1];
+  int* rj = S.rows[j & 1];
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) {
+    const int p = p0 - 32 * q;
+    if (p == bi) { R.v[q] = jsel; R.row[q] = jrow; }
+    R.l[q] = R.v[q] * inv;
+    if (p > j) {
+      lj[p] = R.l[q];
+      rj[p] = R.row[q];
     }
-    const int w = n - j - 1;
-    if (w == 0) break;
-    if (tid < 32) {
-      // column j+1 for rows j+1.. (all loads first), then the look-ahead
-      const double* colj1 = A + (size_t)(j + 1) * lda;
-      const double ujn = colj1[j];
-      const int nq = (w + 31) >> 5;   // register blocks holding rows, warp-uniform
-      double a[LU_RPL], l[LU_RPL];
+  }
+  if (lane == 0) {
+    S.prow[j] = R.pr;
+    dinv[j] = inv;
+    if (zero) *ok_out = 0;
+  }
+}
+
+// columns j = j0.. while at most 32 NQ positions (and more than 32 (NQ - 1)) lie
+// behind them; returns the first column not done
+template <int NQ>
+__device__ __forceinline__ int lu_columns(double* A, int lda, double* b, int n, double* dinv,
+                                          LuShared& S, LuRegs& R, int j0, int* ok_out) {
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  int j = j0;
+  for (; j < n - 1 - 32 * (NQ - 1); ++j) {
+    if (wid == 0) {
+      // column j+1 at positions j+1.. (all loads first), then its pivot
+      const double* col = A + (j + 1) * lda;
+      const double u = col[R.pr];
+      double a[NQ];
 #pragma unroll
-      for (int q = 0; q < LU_RPL; ++q) {
-        const int i = j + 1 + lane + 32 * q;
-        a[q] = (q < nq && i < n) ? colj1[i] : 0.0;
-        l[q] = (q < nq && i < n) ? lc[i] : 0.0;
-      }
-      double v[LU_RPL];
+      for (int q = 0; q < NQ; ++q) a[q] = (n - 1 - lane - 32 * q > j) ? col[R.row[q]] : 0.0;
 #pragma unroll
-      for (int q = 0; q < LU_RPL; ++q) {
-        if (q < nq) {
-          const int i = j + 1 + lane + 32 * q;
-          v[q] = a[q] - l[q] * ujn;
-          if (i < n) A[(size_t)(j + 1) * lda + i] = v[q];
-        } else {
-          v[q] = 0.0;
-        }
-      }
-      pick(j + 1, v, ln, nq);
+      for (int q = 0; q < NQ; ++q) R.v[q] = a[q] - R.l[q] * u;
+      lu_pick<NQ>(R, S, j + 1, n, dinv, ok_out);
     } else {
-      const int nt = (int)blockDim.x - 32, t = tid - 32;
-      // b for rows j+1.. (forward elimination of the right-hand side)
-      if (t < w) {
-        const int i = j + 1 + t;
-        b[i] = b[i] - lc[i] * b[j];
+      const int pj = S.prow[j];
+      const double* lj = S.lb[j & 1];
+      const int* rj = S.rows[j & 1];
+      double l[NQ];
+      int r[NQ];
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        const int p = n - 1 - lane - 32 * q;
+        l[q] = (p > j) ? lj[p] : 0.0;
+        r[q] = (p > j) ? rj[p] : -1;
       }
-      if (w > 1) {
-        // columns j+2.. of rows j+1..: flat over warps 1..7, lanes along rows
-        const int cpp = nt / w;                 // columns per pass
-        const int cc = t / w, r = t - (t / w) * w;
-        if (cc < cpp) {
-          const int i = j + 1 + r;
-          const double li = lc[i];
-          for (int c = j + 2 + cc; c < n; c += cpp) {
-            double* col = A + (size_t)c * lda;
-            col[i] = col[i] - li * col[j];
-          }
-        }
+      // columns j+2.. dealt to warps 1..7, and b (forward elimination of the
+      // right-hand side) as one more column to the warp with the fewest
+      for (int c = j + 1 + wid; c <= n; c += IPM_BLOCK / 32 - 1) {
+        double* col = (c < n) ? A + c * lda : b;
+        const double u = col[pj];
+        double x[NQ];
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) x[q] = (r[q] >= 0) ? col[r[q]] : 0.0;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q)
+          if (r[q] >= 0) col[r[q]] = x[q] - l[q] * u;
       }
     }
     __syncthreads();
-    double* tsw = lc; lc = ln; ln = tsw;
+  }
+  return j;
+}
+
+// U x = b, columns j = j0 down to 32 (NQ - 1), by one warp: lane l keeps b at
+// positions l, l + 32, l + 64 in br; x_j = b_j * (1 / u_jj) with the pivot
+// reciprocal of the factorisation (as the multipliers), then every lane updates
+// its positions above j, the block that holds position j - 1 first.
+template <int NQ>
+__device__ __forceinline__ int lu_back(const double* A, int lda, const double* dinv, LuRegs& R,
+                                       int j0) {
+  const int lane = threadIdx.x & 31;
+  int j = j0;
+  for (; j >= 32 * (NQ - 1); --j) {
+    const double* colj = A + j * lda;
+    double u[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) u[q] = (lane + 32 * q < j) ? colj[R.row[q]] : 0.0;
+    const double bj = __shfl_sync(0xffffffffu, R.v[NQ - 1], j & 31) * dinv[j];
+#pragma unroll
+    for (int q = NQ - 1; q >= 0; --q) {
+      const int i = lane + 32 * q;
+      if (i == j) R.v[q] = bj;
+      else if (i < j) R.v[q] -= u[q] * bj;
+    }
+  }
+  return j;
+}
+
+__device__ void ipm_lu_solve(double* A, int lda, double* b, int n, double* dinv, int* ok_out) {
+  static_assert(LU_RPL == 3, "register blocks");
+  __shared__ LuShared S;
+  const int tid = threadIdx.x, lane = tid & 31;
+  LuRegs R;
+  if (tid == 0) *ok_out = 1;
+  __syncthreads();
+  if (tid < 32) {
+#pragma unroll
+    for (int q = 0; q < LU_RPL; ++q) {
+      R.row[q] = n - 1 - lane - 32 * q;
+      R.v[q] = (R.row[q] >= 0) ? A[R.row[q]] : 0.0;
+    }
+    if (n > 64) lu_pick<3>(R, S, 0, n, dinv, ok_out);
+    else if (n > 32) lu_pick<2>(R, S, 0, n, dinv, ok_out);
+    else lu_pick<1>(R, S, 0, n, dinv, ok_out);
   }
   __syncthreads();
-  // U x = b by one warp: lane l keeps b[l], b[l + 32], b[l + 64] in registers;
-  // x_j = b_j * (1 / u_jj) with the pivot reciprocal of the factorisation (as
-  // the multipliers), then every lane updates its rows above j.
+  int j = lu_columns<3>(A, lda, b, n, dinv, S, R, 0, ok_out);
+  j = lu_columns<2>(A, lda, b, n, dinv, S, R, j, ok_out);
+  j = lu_columns<1>(A, lda, b, n, dinv, S, R, j, ok_out);
   if (tid < 32) {
-    double br[LU_RPL];
 #pragma unroll
-    for (int q = 0; q < LU_RPL; ++q) br[q] = (lane + 32 * q < n) ? b[lane + 32 * q] : 0.0;
-    for (int j = n - 1; j >= 0; --j) {
-      const int oq = j >> 5, ol = j & 31;
-      double bj = 0.0;
-#pragma unroll
-      for (int q = 0; q < LU_RPL; ++q) if (q == oq) bj = br[q];
-      bj = __shfl_sync(0xffffffffu, bj, ol) * dinv[j];
-      const double* colj = A + (size_t)j * lda;
-#pragma unroll
-      for (int q = 0; q < LU_RPL; ++q) {
-        if (q <= oq) {   // blocks holding rows at or above j, warp-uniform
-          const int i = lane + 32 * q;
-          if (i == j) br[q] = bj;
-          else if (i < j) br[q] -= colj[i] * bj;
-        }
-      }
+    for (int q = 0; q < LU_RPL; ++q) {
+      R.row[q] = (lane + 32 * q < n) ? S.prow[lane + 32 * q] : 0;
+      R.v[q] = (lane + 32 * q < n) ? b[R.row[q]] : 0.0;
     }
+    j = lu_back<3>(A, lda, dinv, R, n - 1);
+    j = lu_back<2>(A, lda, dinv, R, j);
+    j = lu_back<1>(A, lda, dinv, R, j);
 #pragma unroll
-    for (int q = 0; q < LU_RPL; ++q) if (lane + 32 * q < n) b[lane + 32 * q] = br[q];
+    for (int q = 0; q < LU_RPL; ++q) if (lane + 32 * q < n) b[lane + 32 * q] = R.v[q];
   }
   __syncthreads();
 }
@@ -389,10 +432,10 @@ __global__ void __launch_bounds__(IPM_BLOCK, 1) ipm_kernel(const __grid_constant
   __shared__ IpmShared sh;
   __shared__ IpmScal sc;
   __shared__ double grid[256];
-  __shared__ int s_piv, s_ok;
+  __shared__ int s_ok;
+  __shared__ unsigned s_mask;
   if (A.skip && *A.skip) return;
   const int k = A.k, s = k * (k + 1) / 2, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int nw = IPM_BLOCK / 32;
   double* Q11 = dyn;            // s*s (mode 0)
   double* coeff = dyn + s * s;  // s*s
   double* sm = A.smalls;
@@ -548,11 +591,10 @@ __global__ void __launch_bounds__(IPM_BLOCK, 1) ipm_kernel(const __grid_constant
       }
     }
     // S^-1 (the reference's jnp.linalg.inv, solver/usbs.py:91)
-    for (int e = tid; e < k * k; e += IPM_BLOCK) sh.wk[e] = sh.S[e];
     __syncthreads();
     const double k1 = sc.k1, k2 = sc.k2, den = sc.den, ze = sc.ze;
     {
-      const bool okinv = cta_inverse(sh.wk, k, sh.Si, sh.lcol, &s_piv, sh.redv);
+      const bool okinv = cta_inverse(sh.S, k, sh.Si, coeff);
       if (!okinv && tid == 0) atomicOr(A.status, ST_SMALL_DENSE_FAIL);
     }
     __syncthreads();
@@ -605,7 +647,7 @@ __global__ void __launch_bounds__(IPM_BLOCK, 1) ipm_kernel(const __grid_constant
     }
     __syncthreads();
     if (tid == 0) { const long long c = clock64(); ph0 += c - tclk; tclk = c; }
-    ipm_lu_solve(coeff, s, sh.ord, s, sh.dinv, sh.lcol, &s_ok);
+    ipm_lu_solve(coeff, s, sh.ord, s, sh.dinv, &s_ok);
     if (tid == 0) { const long long c = clock64(); ph1 += c - tclk; tclk = c; }
     if (tid == 0 && !s_ok) atomicOr(A.status, ST_SMALL_DENSE_FAIL);
     // sh.ord now holds dsS
@@ -658,41 +700,41 @@ __global__ void __launch_bounds__(IPM_BLOCK, 1) ipm_kernel(const __grid_constant
     svec_inv_to(sh.dsT, k, s, sh.bi, sh.ci, sh.dT);
     __syncthreads();
     // ---- line search over the grid 0.9^j (solver/usbs.py:134-154): the largest
-    // grid step keeping S (lanes 0-15) and T (lanes 16-31) positive definite is the
-    // first positive-definite grid index ----
-    if (wid == 0) {
-      const int half = lane >> 4, sub = lane & 15;
-      const double* M = half ? sh.T : sh.S;
-      const double* dM = half ? sh.dT : sh.dS;
+    // grid step keeping S and T positive definite is the first positive-definite
+    // grid index ----
+    int firstS, firstT;
+    {
       // PD-ness of A + a dA is monotone along the grid (the PD steps form an
       // interval containing 0), so after the first 16 points the first PD
       // index is bracketed by testing every 16th point, then resolved inside
       // the bracket: at most three rounds of 16 tests per matrix.
+      const int half = tid >> 7, sub = (tid >> 3) & 15;
       auto gstep = [&](int j) { return (j < 256) ? grid[j] : pow(0.9, (double)j); };
-      int first = -1;
-      {
-        const bool pd = (sub < ngrid) && pd_test(M, dM, gstep(sub), k);
-        const unsigned bal = __ballot_sync(0xffffffffu, pd);
-        const unsigned mine = half ? (bal >> 16) : (bal & 0xffffu);
-        if (mine) first = __ffs(mine) - 1;
+      auto tests = [&](bool active, int j) {
+        return pd_tests(sh.S, sh.dS, sh.T, sh.dT, k, s, sh.bi, sh.ci, active,
+                        active ? gstep(j) : 0.0, coeff, &s_mask);
+      };
+      auto lowest = [](unsigned m) { return m ? __ffs(m) - 1 : -1; };
+      const unsigned m1 = tests(sub < ngrid, sub);
+      firstS = lowest(m1 & 0xffffu);
+      firstT = lowest(m1 >> 16);
+      if (ngrid > 16 && (firstS < 0 || firstT < 0)) {
+        __syncthreads();
+        const bool need2 = (half ? firstT : firstS) < 0;
+        const unsigned m2 = tests(need2 && 16 + 16 * sub < ngrid, min(31 + 16 * sub, ngrid - 1));
+        const int qS = lowest(m2 & 0xffffu), qT = lowest(m2 >> 16);
+        if (m2) {
+          __syncthreads();
+          const int q = half ? qT : qS;
+          const int j3 = 16 + 16 * max(q, 0) + sub, jq = min(31 + 16 * max(q, 0), ngrid - 1);
+          const unsigned m3 = tests(need2 && q >= 0 && j3 <= jq, j3);
+          const int fS = lowest(m3 & 0xffffu), fT = lowest(m3 >> 16);
+          if (firstS < 0 && qS >= 0 && fS >= 0) firstS = 16 + 16 * qS + fS;
+          if (firstT < 0 && qT >= 0 && fT >= 0) firstT = 16 + 16 * qT + fT;
+        }
       }
-      const bool need2 = (first < 0) && (ngrid > 16);
-      if (__any_sync(0xffffffffu, need2)) {
-        const int jc = min(31 + 16 * sub, ngrid - 1);
-        const bool pd = need2 && (16 + 16 * sub < ngrid) && pd_test(M, dM, gstep(jc), k);
-        const unsigned bal = __ballot_sync(0xffffffffu, pd);
-        const unsigned mine = half ? (bal >> 16) : (bal & 0xffffu);
-        const int q = mine ? (__ffs(mine) - 1) : -1;
-        const bool need3 = need2 && q >= 0;
-        const int j3 = 16 + 16 * (q < 0 ? 0 : q) + sub;
-        const int jq = min(31 + 16 * (q < 0 ? 0 : q), ngrid - 1);
-        const bool pd3 = need3 && j3 <= jq && pd_test(M, dM, gstep(j3), k);
-        const unsigned bal3 = __ballot_sync(0xffffffffu, pd3);
-        const unsigned mine3 = half ? (bal3 >> 16) : (bal3 & 0xffffu);
-        if (need3 && mine3) first = 16 + 16 * q + __ffs(mine3) - 1;
-      }
-      const int firstS = __shfl_sync(0xffffffffu, first, 0);
-      const int firstT = __shfl_sync(0xffffffffu, first, 16);
+    }
+    if (wid == 0) {
       if (lane == 0) {
         const double cS = (firstS < 0) ? 0.0 : (firstS < 256 ? grid[firstS] : pow(0.9, (double)firstS));
         const double cT = (firstT < 0) ? 0.0 : (firstT < 256 ? grid[firstT] : pow(0.9, (double)firstT));
@@ -926,13 +968,22 @@ __global__ void cholqr_kernel(CholQRArgs A) {
   for (int e = lane; e < k * k; e += 32) sm[A.o_Rinv + e] = Ri[e];
 }
 
+// Q11, then the Newton matrix, whose room the inverse of S (4 k^2) and the line
+// search (32 tests of s + IPM_MAXK) use before and after it
+static size_t ipm_dyn_doubles(int k) {
+  const size_t s = (size_t)k * (k + 1) / 2;
+  size_t w = s * s;
+  if (w < (size_t)4 * k * k) w = (size_t)4 * k * k;
+  if (w < 32 * (s + IPM_MAXK)) w = 32 * (s + IPM_MAXK);
+  return s * s + w;
+}
+
 int launch_ipm(const IpmArgs& a, cudaStream_t st) {
-  const int s = a.k * (a.k + 1) / 2;
-  const size_t dyn = (size_t)2 * s * s * sizeof(double);
+  const size_t dyn = ipm_dyn_doubles(a.k) * sizeof(double);
   static bool attr = false;
   if (!attr) {
     cudaFuncSetAttribute(ipm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         2 * IPM_MAXS * IPM_MAXS * (int)sizeof(double));
+                         (int)(ipm_dyn_doubles(IPM_MAXK) * sizeof(double)));
     attr = true;
   }
   ipm_kernel<<<1, IPM_BLOCK, dyn, st>>>(a);

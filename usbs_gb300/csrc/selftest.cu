@@ -12,6 +12,7 @@
 #include "../../include/usbs_gb300.h"
 #include "common.cuh"
 #include "internal.h"
+#include "recip.cuh"
 
 namespace usbs {
 
@@ -32,9 +33,30 @@ __global__ void selftest_wait_kernel(int which, int expected, unsigned long long
   __syncthreads();
 }
 
+// y = recip_exact(x), elementwise
+__global__ void selftest_recip_kernel(long long n, const double* __restrict__ x,
+                                      double* __restrict__ y) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
+       i += (long long)gridDim.x * blockDim.x)
+    y[i] = recip_exact(x[i]);
+}
+
 }  // namespace usbs
 
 using namespace usbs;
+
+extern "C" int usbs_selftest_recip(long long n, const double* x, double* y, void* stream) {
+  if (n < 1 || !x || !y) {
+    set_error("selftest_recip: n=%lld", n);
+    return -2;
+  }
+  selftest_recip_kernel<<<304, 256, 0, (cudaStream_t)stream>>>(n, x, y);
+  if (cudaGetLastError() != cudaSuccess) {
+    set_error("selftest_recip: launch failed");
+    return -5;
+  }
+  return 0;
+}
 
 extern "C" int usbs_selftest_wait_limits(int which, int nctas, long long limit_ns,
                                          unsigned int* counters, int* status, void* stream) {
