@@ -13,37 +13,110 @@
 
 namespace usbs {
 
-template <typename OT>
-__global__ void assemble_kernel(int nnz, const double* __restrict__ c_val, double alpha_c,
-                                const int* __restrict__ slot_ptr, const int* __restrict__ slot_tid,
-                                const int* __restrict__ con, const double* __restrict__ a,
-                                const double* __restrict__ w, OT* __restrict__ out) {
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < nnz; p += gridDim.x * blockDim.x) {
-    double v = (alpha_c != 0.0 && c_val) ? alpha_c * c_val[p] : 0.0;
-    if (w) {
+// (float)x rounded to nearest even, on the integer pipes for results that are
+// normal floats (or round to infinity): a conversion from FP64 takes the SM's FP64
+// unit 19 cycles per warp, like any FP64 instruction.
+__device__ __forceinline__ float to_float_rn(double x) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const unsigned long long m = b & 0x7fffffffffffffffull;
+  const unsigned ex = (unsigned)(m >> 52);
+  if (ex - 897u > 253u && m != 0ull) return (float)x;      // subnormal float, overflow, Inf, NaN
+  unsigned r = 0u;
+  if (m) r = (unsigned)((m + 0x0fffffffull + ((m >> 29) & 1ull)) >> 29) - (896u << 23);
+  return __uint_as_float(r | ((unsigned)(b >> 32) & 0x80000000u));
+}
+template <typename OT> __device__ __forceinline__ OT out_of(double v);
+template <> __device__ __forceinline__ double out_of<double>(double v) { return v; }
+template <> __device__ __forceinline__ float out_of<float>(double v) { return to_float_rn(v); }
+
+// alpha x without an FP64 instruction where alpha is 1 or -1 (sgn = 0 or the sign
+// bit; 1 otherwise), as the solvers' operators are
+__device__ __forceinline__ double scaled(double alpha, unsigned long long sgn, double x) {
+  return (sgn == 1ull) ? alpha * x
+                       : __longlong_as_double(__double_as_longlong(x) ^ (long long)sgn);
+}
+
+constexpr int AS_BLOCK = 256;
+
+// out = alpha_c C + A*(w) on the pattern.  Entries that no triple lands on (seven of
+// eight on a degree-7 graph) need no FP64 arithmetic; the others are listed per
+// block and taken by whole warps, because an FP64 instruction costs its warp the
+// same however few lanes have such an entry.  n = 10^6, 8.1e6 entries, FP32 out:
+// 50 us (87 with every entry scaled, added to and converted in place).
+template <typename OT, int AS_PER>      // AS_PER pattern entries per thread and round
+__global__ void __launch_bounds__(AS_BLOCK) assemble_kernel(
+    int nnz, const double* __restrict__ c_val, double alpha_c, unsigned long long sgn,
+    const int* __restrict__ slot_ptr, const int* __restrict__ slot_tid,
+    const int* __restrict__ con, const double* __restrict__ a, const double* __restrict__ w,
+    OT* __restrict__ out) {
+  __shared__ int list[AS_BLOCK * AS_PER];
+  __shared__ int count;
+  const bool has_c = alpha_c != 0.0 && c_val;
+  constexpr int CH = AS_BLOCK * AS_PER;
+  for (int base = blockIdx.x * CH; base < nnz; base += gridDim.x * CH) {
+    if (threadIdx.x == 0) count = 0;
+    __syncthreads();
+    double v[AS_PER];
+    int n0[AS_PER], n1[AS_PER];
+#pragma unroll
+    for (int u = 0; u < AS_PER; ++u) {
+      const int p = base + u * AS_BLOCK + threadIdx.x;
+      v[u] = (has_c && p < nnz) ? c_val[p] : 0.0;
+      n0[u] = n1[u] = 0;
+      if (w && p < nnz) { n0[u] = slot_ptr[p]; n1[u] = slot_ptr[p + 1]; }
+    }
+#pragma unroll
+    for (int u = 0; u < AS_PER; ++u) {
+      const int p = base + u * AS_BLOCK + threadIdx.x;
+      const bool more = n1[u] > n0[u];
+      const unsigned mb = __ballot_sync(0xffffffffu, more);
+      int at = 0;
+      if (mb && (threadIdx.x & 31) == 0) at = atomicAdd(&count, __popc(mb));
+      at = __shfl_sync(0xffffffffu, at, 0) + __popc(mb & ((1u << (threadIdx.x & 31)) - 1u));
+      if (more) list[at] = p;
+      else if (p < nnz) out[p] = out_of<OT>(has_c ? scaled(alpha_c, sgn, v[u]) : 0.0);
+    }
+    __syncthreads();
+    const int cnt = count;
+    for (int i = threadIdx.x; i < cnt; i += AS_BLOCK) {
+      const int p = list[i];
+      double x = has_c ? scaled(alpha_c, sgn, c_val[p]) : 0.0;
       const int e = slot_ptr[p + 1];
       for (int q = slot_ptr[p]; q < e; ++q) {
         const int t = slot_tid[q];
-        v += a[t] * w[con[t]];
+        x += a[t] * w[con[t]];
       }
+      out[p] = out_of<OT>(x);
     }
-    out[p] = (OT)v;
+    __syncthreads();
   }
+}
+
+template <typename OT>
+static void assemble_launch(int nnz, const double* c_val, double alpha_c, const int* slot_ptr,
+                            const int* slot_tid, const int* con, const double* a, const double* w,
+                            OT* out, cudaStream_t stream) {
+  const unsigned long long sgn = (alpha_c == 1.0) ? 0ull : (alpha_c == -1.0) ? 1ull << 63 : 1ull;
+  // four entries per thread once that still fills the GPU twice over
+  const int per = (nnz >= 152 * 2048) ? 4 : 1;
+  int blocks = (nnz + AS_BLOCK * per - 1) / (AS_BLOCK * per);
+  if (blocks > 152 * 16) blocks = 152 * 16;
+  if (per == 4)
+    assemble_kernel<OT, 4><<<blocks, AS_BLOCK, 0, stream>>>(nnz, c_val, alpha_c, sgn, slot_ptr,
+                                                            slot_tid, con, a, w, out);
+  else
+    assemble_kernel<OT, 1><<<blocks, AS_BLOCK, 0, stream>>>(nnz, c_val, alpha_c, sgn, slot_ptr,
+                                                            slot_tid, con, a, w, out);
 }
 
 int assemble_operator(int nnz, const double* c_val, double alpha_c, const int* slot_ptr,
                       const int* slot_tid, const int* con, const double* a, const double* w,
                       void* op_val, int prec, cudaStream_t stream) {
   if (nnz <= 0) return 0;
-  const int threads = 256;
-  int blocks = (nnz + threads - 1) / threads;
-  if (blocks > 152 * 16) blocks = 152 * 16;
   if (prec == 64)
-    assemble_kernel<double><<<blocks, threads, 0, stream>>>(nnz, c_val, alpha_c, slot_ptr,
-                                                            slot_tid, con, a, w, (double*)op_val);
+    assemble_launch(nnz, c_val, alpha_c, slot_ptr, slot_tid, con, a, w, (double*)op_val, stream);
   else
-    assemble_kernel<float><<<blocks, threads, 0, stream>>>(nnz, c_val, alpha_c, slot_ptr,
-                                                           slot_tid, con, a, w, (float*)op_val);
+    assemble_launch(nnz, c_val, alpha_c, slot_ptr, slot_tid, con, a, w, (float*)op_val, stream);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { set_error("assemble_operator: %s", cudaGetErrorString(e)); return -5; }
   return 0;
@@ -243,24 +316,67 @@ int gather_values(long long total, const int* map, const void* src, void* dst, i
   return 0;
 }
 
-// out[c] = sum_{t in constraint c} a_t * U[i_t, :] . U[j_t, :]    (one warp per constraint)
-__global__ void A_operator_kernel(int m, const int* __restrict__ con_ptr,
-                                  const int* __restrict__ t_row, const int* __restrict__ t_col,
-                                  const double* __restrict__ a, const double* __restrict__ U,
-                                  int ldu, int k, double* __restrict__ out) {
+// a_t U[i_t, :] . U[j_t, :]
+__device__ __forceinline__ double triple_value(int t, const int* __restrict__ t_row,
+                                               const int* __restrict__ t_col,
+                                               const double* __restrict__ a,
+                                               const double* __restrict__ U, int ldu, int k) {
+  const int i = t_row[t], j = t_col[t];
+  double d = 0.0;
+  for (int q = 0; q < k; ++q) d += U[(size_t)q * ldu + i] * U[(size_t)q * ldu + j];
+  return fma(a[t], d, 0.0);
+}
+
+// out[c] = sum_{t in constraint c} a_t * U[i_t, :] . U[j_t, :]: triples dealt to 32
+// accumulators (every 32nd to the same one) that are added pairwise at distance
+// 16, 8, 4, 2, 1.  Constraints of at most AO_SHORT triples take one thread each
+// (its few accumulators in registers, the tree's additions of nothing left out),
+// longer ones one warp.  With a warp for each of the QAP's 3.4e5 constraints, of
+// mostly two triples, the FP64 unit added zeros: 170 us at l = 30, k = 2; 18 now.
+constexpr int AO_SHORT = 8;
+__global__ void __launch_bounds__(256) A_operator_kernel(
+    int m, const int* __restrict__ con_ptr, const int* __restrict__ t_row,
+    const int* __restrict__ t_col, const double* __restrict__ a, const double* __restrict__ U,
+    int ldu, int k, double* __restrict__ out) {
   const int lane = threadIdx.x & 31;
-  const int warps = (gridDim.x * blockDim.x) >> 5;
-  for (int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < m; c += warps) {
-    double s = 0.0;
-    const int e = con_ptr[c + 1];
-    for (int t = con_ptr[c] + lane; t < e; t += 32) {
-      const int i = t_row[t], j = t_col[t];
-      double d = 0.0;
-      for (int q = 0; q < k; ++q) d += U[(size_t)q * ldu + i] * U[(size_t)q * ldu + j];
-      s += a[t] * d;
+  const int total = gridDim.x * blockDim.x, warps = total >> 5;
+  const int gid = blockIdx.x * blockDim.x + threadIdx.x, wid = gid >> 5;
+  // long constraints: each lane looks at one, far from its neighbours' (long ones
+  // come in runs), and the warp takes those it found one by one
+  for (long long c0 = wid; c0 < m; c0 += 32ll * warps) {
+    const long long c = c0 + (long long)lane * warps;
+    int b = 0, e = 0;
+    if (c < m) { b = con_ptr[c]; e = con_ptr[c + 1]; }
+    unsigned todo = __ballot_sync(0xffffffffu, e - b > AO_SHORT);
+    while (todo) {
+      const int src = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const int tb = __shfl_sync(0xffffffffu, b, src), te = __shfl_sync(0xffffffffu, e, src);
+      double s = 0.0;
+      for (int t = tb + lane; t < te; t += 32) {
+        const int i = t_row[t], j = t_col[t];
+        double d = 0.0;
+        for (int q = 0; q < k; ++q) d += U[(size_t)q * ldu + i] * U[(size_t)q * ldu + j];
+        s += a[t] * d;
+      }
+      s = warp_sum(s);
+      if (lane == 0) out[c0 + (long long)src * warps] = s;
     }
-    s = warp_sum(s);
-    if (lane == 0) out[c] = s;
+  }
+  for (int c = gid; c < m; c += total) {
+    const int b = con_ptr[c], cnt = con_ptr[c + 1] - b;
+    if (cnt > AO_SHORT) continue;
+    double v[AO_SHORT];
+#pragma unroll
+    for (int u = 0; u < AO_SHORT; ++u)
+      v[u] = (u < cnt) ? triple_value(b + u, t_row, t_col, a, U, ldu, k) : 0.0;
+#pragma unroll
+    for (int o = AO_SHORT / 2; o > 0; o >>= 1) {
+#pragma unroll
+      for (int u = 0; u < o; ++u)
+        if (u + o < cnt) v[u] += v[u + o];
+    }
+    out[c] = v[0];
   }
 }
 
@@ -269,30 +385,83 @@ int apply_A_operator(int m, const int* con_ptr, const int* t_row, const int* t_c
                      cudaStream_t stream) {
   if (m <= 0) return 0;
   const int threads = 256;
-  long long need = ((long long)m * 32 + threads - 1) / threads;
-  int blocks = (int)(need < 152 * 16 ? need : 152 * 16);
+  long long need = ((long long)m * 32 + threads - 1) / threads;       // a warp per constraint
+  int blocks = (int)(need < 152 * 8 ? need : 152 * 8);
   A_operator_kernel<<<blocks, threads, 0, stream>>>(m, con_ptr, t_row, t_col, a, U, ldu, k, out);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { set_error("apply_A_operator: %s", cudaGetErrorString(e)); return -5; }
   return 0;
 }
 
-// out[i, q] = sum_{t with row i} a_t z[c_t] U[j_t, q]    (one warp per row, lanes over triples)
-__global__ void A_adjoint_kernel(int n, const int* __restrict__ row_ptr,
-                                 const int* __restrict__ r_con, const int* __restrict__ r_col,
-                                 const double* __restrict__ r_a, const double* __restrict__ z,
-                                 const double* __restrict__ U, int ldu, int k,
-                                 double* __restrict__ out, int ldo) {
+// out[i, q] = sum_{t with row i} a_t z[c_t] U[j_t, q], summed as A_operator_kernel
+// sums: 32 accumulators, then pairwise.  Rows of at most AO_SHORT triples (one in
+// MaxCut) take one thread for all columns, longer ones (the QAP's hold about 900,
+// the lifted row several thousand) one warp per column, because a warp gets one
+// FP64 instruction per 60 cycles; four triples' loads in flight per lane.
+__global__ void __launch_bounds__(256) A_adjoint_kernel(
+    int n, const int* __restrict__ row_ptr, const int* __restrict__ r_con,
+    const int* __restrict__ r_col, const double* __restrict__ r_a, const double* __restrict__ z,
+    const double* __restrict__ U, int ldu, int k, double* __restrict__ out, int ldo) {
   const int lane = threadIdx.x & 31;
-  const int warps = (gridDim.x * blockDim.x) >> 5;
-  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
-    const int b = row_ptr[i], e = row_ptr[i + 1];
-    for (int q = 0; q < k; ++q) {
+  const int total = gridDim.x * blockDim.x, warps = total >> 5;
+  const int gid = blockIdx.x * blockDim.x + threadIdx.x, wid = gid >> 5;
+  const long long tasks = (long long)n * k;        // (row, column), column fastest
+  for (long long w0 = wid; w0 < tasks; w0 += 32ll * warps) {
+    const long long w = w0 + (long long)lane * warps;
+    int b = 0, e = 0;
+    if (w < tasks) { b = row_ptr[w / k]; e = row_ptr[w / k + 1]; }
+    unsigned todo = __ballot_sync(0xffffffffu, e - b > AO_SHORT);
+    while (todo) {
+      const int src = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const long long ws = w0 + (long long)src * warps;
+      const int i = (int)(ws / k), q = (int)(ws - (long long)i * k);
+      const int tb = __shfl_sync(0xffffffffu, b, src), te = __shfl_sync(0xffffffffu, e, src);
+      const double* Uq = U + (size_t)q * ldu;
       double s = 0.0;
-      for (int t = b + lane; t < e; t += 32)
-        s += r_a[t] * z[r_con[t]] * U[(size_t)q * ldu + r_col[t]];
+      for (int t = tb + lane; t < te; t += 128) {
+        double av[4], zv[4], uv[4];
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          const int th = min(t + 32 * h, te - 1);
+          av[h] = r_a[th];
+          zv[h] = z[r_con[th]];
+          uv[h] = Uq[r_col[th]];
+        }
+#pragma unroll
+        for (int h = 0; h < 4; ++h)
+          if (t + 32 * h < te) s += av[h] * zv[h] * uv[h];
+      }
       s = warp_sum(s);
       if (lane == 0) out[(size_t)q * ldo + i] = s;
+    }
+  }
+  for (int i = gid; i < n; i += total) {
+    const int b = row_ptr[i], cnt = row_ptr[i + 1] - b;
+    if (cnt > AO_SHORT) continue;
+    double az[AO_SHORT];
+    int col[AO_SHORT];
+#pragma unroll
+    for (int u = 0; u < AO_SHORT; ++u) {
+      az[u] = 0.0;
+      col[u] = 0;
+      if (u < cnt) {
+        az[u] = r_a[b + u] * z[r_con[b + u]];
+        col[u] = r_col[b + u];
+      }
+    }
+    for (int q = 0; q < k; ++q) {
+      const double* Uq = U + (size_t)q * ldu;
+      double v[AO_SHORT];
+#pragma unroll
+      for (int u = 0; u < AO_SHORT; ++u) v[u] = (u < cnt) ? fma(az[u], Uq[col[u]], 0.0) : 0.0;
+#pragma unroll
+      for (int o = AO_SHORT / 2; o > 0; o >>= 1) {
+#pragma unroll
+        for (int u = 0; u < o; ++u)
+          if (u + o < cnt) v[u] += v[u + o];
+      }
+      out[(size_t)q * ldo + i] = v[0];
     }
   }
 }
@@ -302,8 +471,9 @@ int apply_A_adjoint(int n, const int* row_ptr, const int* r_con, const int* r_co
                     double* out, int ldo, cudaStream_t stream) {
   if (n <= 0) return 0;
   const int threads = 256;
-  long long need = ((long long)n * 32 + threads - 1) / threads;
-  int blocks = (int)(need < 152 * 16 ? need : 152 * 16);
+  long long need = ((long long)n * k * 32 + threads - 1) / threads;   // a warp per (row, column)
+  if (need < 1) need = 1;
+  int blocks = (int)(need < 152 * 8 ? need : 152 * 8);
   A_adjoint_kernel<<<blocks, threads, 0, stream>>>(n, row_ptr, r_con, r_col, r_a, z, U, ldu, k,
                                                    out, ldo);
   cudaError_t e = cudaGetLastError();
