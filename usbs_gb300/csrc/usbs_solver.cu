@@ -101,6 +101,106 @@ __global__ void __launch_bounds__(RED_BLOCK) gram_kernel(GramArgs a) {
   if (tid == 0) *a.counter = 0u;
 }
 
+// gram_kernel for at most 256 entries (kx ky <= 256): the same tiles of the same
+// blocks and the same order of every sum, so the same result.  A block's row
+// tiles are staged four at a time, the next four's loads issued before this
+// four's FMAs: with nine entries over 3.4e5 rows (the QAP's A* projections) a
+// block's chain of dependent FMAs is the bound (60 cycles each, 36 us) and every
+// wait for a load between two of them adds to it (245 us).
+constexpr int GS_T = 4;              // tiles per stage
+constexpr int GS_MAXC = 16;          // widest operand staged this way
+__global__ void __launch_bounds__(RED_BLOCK) gram_small_kernel(GramArgs a) {
+  if (a.skip && *a.skip) return;
+  constexpr int SR = GS_T * GR_ROWS, LDS_R = SR + 2;
+  __shared__ __align__(16) double xs[GS_MAXC * LDS_R], ys[GS_MAXC * LDS_R];
+  __shared__ bool last;
+  const int E = a.kx * a.ky, tid = threadIdx.x;
+  const int p = tid / a.ky, q = tid - p * a.ky;
+  const bool own = tid < E;
+  double acc = 0.0;
+  const int ntiles = (a.n + GR_ROWS - 1) / GR_ROWS;
+  const bool same = a.X == a.Y && a.ldx == a.ldy && a.kx == a.ky;
+  const int ncol = a.kx + (same ? 0 : a.ky);           // operand columns to stage
+  constexpr int PER = 2 * GS_MAXC * SR / RED_BLOCK;     // most values per thread and stage
+  double v[PER];
+  auto fetch = [&](int tile0) {
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int e = tid + u * RED_BLOCK, c = e / SR, r = e - c * SR;
+      const int tile = tile0 + (r / GR_ROWS) * (int)gridDim.x;
+      const long long row = (long long)tile * GR_ROWS + (r % GR_ROWS);
+      v[u] = 0.0;
+      if (c < ncol && tile < ntiles && row < a.n)
+        v[u] = (c < a.kx) ? a.X[(size_t)c * a.ldx + row] : a.Y[(size_t)(c - a.kx) * a.ldy + row];
+    }
+  };
+  fetch(blockIdx.x);
+  for (int tile0 = blockIdx.x; tile0 < ntiles; tile0 += GS_T * (int)gridDim.x) {
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int e = tid + u * RED_BLOCK, c = e / SR, r = e - c * SR;
+      if (c < ncol) {
+        if (c < a.kx) xs[c * LDS_R + r] = v[u];
+        else ys[(c - a.kx) * LDS_R + r] = v[u];
+      }
+    }
+    __syncthreads();
+    if (tile0 + GS_T * (int)gridDim.x < ntiles) fetch(tile0 + GS_T * (int)gridDim.x);
+    if (own) {
+      const double* x = xs + p * LDS_R;
+      const double* y = (same ? xs : ys) + q * LDS_R;
+      // (tiles past the end hold zeros; like gram_kernel they are not added)
+      const int nt = min(GS_T, (ntiles - tile0 + (int)gridDim.x - 1) / (int)gridDim.x);
+      for (int t = 0; t < nt; ++t) {
+#pragma unroll
+        for (int r = 0; r < GR_ROWS; r += 2) {
+          const double2 xv = *(const double2*)(x + t * GR_ROWS + r);
+          const double2 yv = *(const double2*)(y + t * GR_ROWS + r);
+          acc += xv.x * yv.x;
+          acc += xv.y * yv.y;
+        }
+      }
+    }
+    __syncthreads();
+  }
+  if (own) a.partial[(size_t)blockIdx.x * E + tid] = acc;
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) last = (atomicAdd(a.counter, 1u) == gridDim.x - 1);
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  // gram_kernel's four chains over the blocks (4 j + chain), each on a group of
+  // threads of its own while the entries leave room: a warp's FP64 adds are 60
+  // cycles apart however independent they are
+  const int nb = (int)gridDim.x, full = nb & ~3;
+  const int GE = (E <= 64) ? 64 : (E <= 128) ? 128 : 256;     // threads per group
+  const int g = tid / GE, e = tid - g * GE, G = RED_BLOCK / GE;
+  double* part = xs;                                          // 4 x E sums
+  if (e < E) {
+    for (int ch = g; ch < 4; ch += G) {
+      const double* src = a.partial + (size_t)ch * E + e;
+      double s = 0.0;
+      int b = 0;
+      for (; b + 28 < full; b += 32) {
+        double w[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) w[u] = __ldcg(src + (size_t)(b + 4 * u) * E);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) s += w[u];
+      }
+      for (; b < full; b += 4) s += __ldcg(src + (size_t)b * E);
+      if (ch == 0)
+        for (b = full; b < nb; ++b) s += __ldcg(a.partial + (size_t)b * E + e);
+      part[ch * E + e] = s;
+    }
+  }
+  __syncthreads();
+  if (own)
+    a.out[tid] = (part[tid] + part[E + tid]) + (part[2 * E + tid] + part[3 * E + tid]);
+  if (tid == 0) *a.counter = 0u;
+}
+
 // Symmetric case G = X^T X of a wide X (create_Q_base): the same per-block
 // tiles and accumulation order as gram_kernel, for the upper triangle only
 // (x_p x_q and x_q x_p round alike, so the lower triangle is its mirror), and
@@ -265,6 +365,45 @@ __global__ void svec_project_kernel(int m, const int* __restrict__ con_ptr,
   }
 }
 
+// svec_project_kernel for small orders (s = k (k + 1) / 2 <= 15): one thread per
+// (constraint, svec entry), constraints along the lanes, each entry summed over
+// the constraint's triples in their order.  A warp per constraint has s of its
+// lanes at work: 345 us for the QAP's s = 3 and 3.4e5 constraints.  The triples
+// of long constraints are loaded four ahead.
+__global__ void __launch_bounds__(256) svec_project_small_kernel(
+    int m, const int* __restrict__ con_ptr, const int* __restrict__ t_row,
+    const int* __restrict__ t_col, const double* __restrict__ t_a, const double* __restrict__ V,
+    int ldv, int s, double* __restrict__ Pm, int ldm, const int* skip) {
+  if (skip && *skip) return;
+  int b = 0, q = blockIdx.y;                       // entry (b, q) of the lower triangle
+  while (q > b) { q -= b + 1; ++b; }
+  const double* Vb = V + (size_t)b * ldv;
+  const double* Vq = V + (size_t)q * ldv;
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < m; c += gridDim.x * blockDim.x) {
+    double acc = 0.0;
+    const int e = con_ptr[c + 1];
+    for (int t0 = con_ptr[c]; t0 < e; t0 += 4) {
+      double av[4], bi[4], bj[4], qi[4], qj[4];
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        const int t = min(t0 + h, e - 1);
+        const int i = t_row[t], j = t_col[t];
+        av[h] = t_a[t];
+        bi[h] = Vb[i]; bj[h] = Vb[j]; qi[h] = Vq[i]; qj[h] = Vq[j];
+      }
+#pragma unroll
+      for (int h = 0; h < 4; ++h)
+        if (t0 + h < e) {
+          double v;
+          if (b == q) v = bi[h] * bj[h];
+          else v = RSQ2_S * (qi[h] * bj[h]) + RSQ2_S * (bi[h] * qj[h]);
+          acc += av[h] * v;
+        }
+    }
+    Pm[(size_t)blockIdx.y * ldm + c] = acc;
+  }
+}
+
 // The three weight vectors of the A* projections side by side after Pm's s
 // columns: W[:, 0] = y, W[:, 1] = z_bar, W[:, 2] = b - upsilon (m each).
 __global__ void pack3_kernel(int m, const double* __restrict__ y, const double* __restrict__ zbar,
@@ -300,46 +439,98 @@ __global__ void sinit_kernel(int k, double v, double* __restrict__ S) {
 }
 
 // AF[c] = sum_t a_t V[i_t] S+ V[j_t]^T = A(F F^T)_c and AFc[c] with Sc+
-// (solver/usbs.py:411-412, 570-571, 627, 639).  One thread per constraint.
-__global__ void quadform_kernel(int m, const int* __restrict__ con_ptr,
-                                const int* __restrict__ t_row, const int* __restrict__ t_col,
-                                const double* __restrict__ t_a, const double* __restrict__ V,
-                                int ldv, int k, const double* __restrict__ Sp,
-                                const double* __restrict__ Scp, double* __restrict__ AF,
-                                double* __restrict__ AFc, const int* skip) {
+// (solver/usbs.py:411-412, 570-571, 627, 639).  A block takes QF_CON consecutive
+// constraints and their triples QF_TILE at a time: each thread forms
+// v_i S+ v_j^T and v_i Sc+ v_j^T of its triples, then warp 0 (for S+) and warp 1
+// (for Sc+) add each constraint's triples of the tile in order, one lane per
+// constraint.  The additions are a chain of FMAs, 60 cycles each whatever the
+// warp has besides, so the two sums go to two warps and a tile holds many
+// constraints' triples.  (One thread per constraint walking its triples left the
+// QAP's 60-triple rows and partial traces to a few warps: 310 us at l = 30,
+// where most of the 3.4e5 constraints have two; 210 us with tiles of 256 and both
+// sums on one thread.)  K: the bundle rank at compile time (0: at run time).
+constexpr int QF_BLOCK = 256, QF_TILE = 1024, QF_CON = 32;
+template <int K>
+__global__ void __launch_bounds__(QF_BLOCK) quadform_kernel(
+    int m, const int* __restrict__ con_ptr, const int* __restrict__ t_row,
+    const int* __restrict__ t_col, const double* __restrict__ t_a, const double* __restrict__ V,
+    int ldv, int k_run, const double* __restrict__ Sp, const double* __restrict__ Scp,
+    double* __restrict__ AF, double* __restrict__ AFc, const int* skip) {
   if (skip && *skip) return;
+  constexpr int KM = K ? K : IPM_MAXK;
+  const int k = K ? K : k_run;
   __shared__ double sp[IPM_MAXK * IPM_MAXK], scp[IPM_MAXK * IPM_MAXK];
-  for (int e = threadIdx.x; e < k * k; e += blockDim.x) { sp[e] = Sp[e]; scp[e] = Scp[e]; }
+  __shared__ double v1[QF_TILE], v2[QF_TILE], va[QF_TILE];
+  const int tid = threadIdx.x;
+  for (int e = tid; e < k * k; e += QF_BLOCK) { sp[e] = Sp[e]; scp[e] = Scp[e]; }
   __syncthreads();
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < m; c += gridDim.x * blockDim.x) {
-    double a1 = 0.0, a2 = 0.0;
-    const int e = con_ptr[c + 1];
-    for (int t = con_ptr[c]; t < e; ++t) {
-      const int i = t_row[t], j = t_col[t];
-      double u[IPM_MAXK], w[IPM_MAXK];
+  for (int c0 = blockIdx.x * QF_CON; c0 < m; c0 += gridDim.x * QF_CON) {
+    const int c1 = min(c0 + QF_CON, m), c = c0 + (tid & 31);
+    const int T0 = con_ptr[c0], T1 = con_ptr[c1];
+    int b = 0, e = 0;
+    if (tid < 64 && c < c1) { b = con_ptr[c]; e = con_ptr[c + 1]; }
+    const double* vs = (tid < 32) ? v1 : v2;
+    double acc = 0.0;
+    for (int t0 = T0; t0 < T1; t0 += QF_TILE) {
+      const int tn = min(QF_TILE, T1 - t0);
+      for (int x = tid; x < tn; x += QF_BLOCK) {
+        const int i = t_row[t0 + x], j = t_col[t0 + x];
+        va[x] = t_a[t0 + x];
+        double u[KM], w[KM];
 #pragma unroll
-      for (int q = 0; q < IPM_MAXK; ++q) {
-        u[q] = (q < k) ? V[(size_t)q * ldv + i] : 0.0;
-        w[q] = (q < k) ? V[(size_t)q * ldv + j] : 0.0;
-      }
-      double s1 = 0.0, s2 = 0.0;
-#pragma unroll
-      for (int p = 0; p < IPM_MAXK; ++p) {
-        if (p < k) {
-          double r1 = 0.0, r2 = 0.0;
-#pragma unroll
-          for (int q = 0; q < IPM_MAXK; ++q)
-            if (q < k) { r1 += sp[p * k + q] * w[q]; r2 += scp[p * k + q] * w[q]; }
-          s1 += u[p] * r1;
-          s2 += u[p] * r2;
+        for (int q = 0; q < KM; ++q) {
+          u[q] = (q < k) ? V[(size_t)q * ldv + i] : 0.0;
+          w[q] = (q < k) ? V[(size_t)q * ldv + j] : 0.0;
         }
+        double s1 = 0.0, s2 = 0.0;
+#pragma unroll
+        for (int p = 0; p < KM; ++p) {
+          if (p < k) {
+            double r1 = 0.0, r2 = 0.0;
+#pragma unroll
+            for (int q = 0; q < KM; ++q)
+              if (q < k) { r1 += sp[p * k + q] * w[q]; r2 += scp[p * k + q] * w[q]; }
+            s1 += u[p] * r1;
+            s2 += u[p] * r2;
+          }
+        }
+        v1[x] = s1;
+        v2[x] = s2;
       }
-      a1 += t_a[t] * s1;
-      a2 += t_a[t] * s2;
+      __syncthreads();
+      const int lo = max(b - t0, 0), hi = min(e - t0, tn);
+#pragma unroll 4
+      for (int x = lo; x < hi; ++x) acc += va[x] * vs[x];
+      __syncthreads();
     }
-    AF[c] = a1;
-    if (AFc) AFc[c] = a2;
+    if (tid < 64 && c < c1) {
+      if (tid < 32) AF[c] = acc;
+      else if (AFc) AFc[c] = acc;
+    }
   }
+}
+
+static int launch_quadform(int m, const int* con_ptr, const int* t_row, const int* t_col,
+                           const double* t_a, const double* V, int ldv, int k, const double* Sp,
+                           const double* Scp, double* AF, double* AFc, int sm_count,
+                           cudaStream_t st) {
+  int blocks = (m + QF_CON - 1) / QF_CON;
+  if (blocks > sm_count * 8) blocks = sm_count * 8;
+  if (blocks < 1) blocks = 1;
+  auto go = [&](auto kern) {
+    kern<<<blocks, QF_BLOCK, 0, st>>>(m, con_ptr, t_row, t_col, t_a, V, ldv, k, Sp, Scp, AF, AFc,
+                                     nullptr);
+  };
+  switch (k) {
+    case 1: go(quadform_kernel<1>); break;
+    case 2: go(quadform_kernel<2>); break;
+    case 3: go(quadform_kernel<3>); break;
+    case 4: go(quadform_kernel<4>); break;
+    default: go(quadform_kernel<0>); break;
+  }
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) { set_error("quadform: %s", cudaGetErrorString(e)); return -5; }
+  return 0;
 }
 
 // ---------------------------------------------------------------- m-vector passes
@@ -365,11 +556,18 @@ struct MvecArgs {
   const int* skip;
 };
 
+// Per-block results v[NR], then the last block's sums (in block order) or maxima
+// over the blocks, in red[0..NR-1] of that block (which gets true).  The last
+// block's threads read all partials at once; the NR sums are then chains of
+// dependent FP64 adds over shared memory (60 cycles a block, 9 us for 304
+// blocks; 36 us with a global load in front of each add).
+constexpr int MV_MAXB = 512;         // most blocks (mgrid is at most two per SM)
 template <int NR>
 __device__ __forceinline__ bool mvec_finish(const MvecArgs& a, double (&v)[NR], const bool* is_max,
                                             double* red) {
   __shared__ bool last;
-  const int tid = threadIdx.x;
+  __shared__ double all[NR * MV_MAXB];
+  const int tid = threadIdx.x, nb = (int)gridDim.x;
   for (int r = 0; r < NR; ++r) {
     double t = is_max[r] ? block_max(v[r], red) : block_sum(v[r], red);
     if (tid == 0) a.partial[(size_t)blockIdx.x * NR + r] = t;
@@ -381,11 +579,31 @@ __device__ __forceinline__ bool mvec_finish(const MvecArgs& a, double (&v)[NR], 
   __syncthreads();
   if (!last) return false;
   __threadfence();
+  const bool fits = nb <= MV_MAXB;
+  if (fits)
+    for (int e = tid; e < nb * NR; e += RED_BLOCK) all[e] = __ldcg(a.partial + e);
+  __syncthreads();
+  double mx[NR];
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    mx[r] = 0.0;
+    if (is_max[r]) {                 // a maximum does not depend on the order
+      for (int bk = tid; bk < nb; bk += RED_BLOCK)
+        mx[r] = fmax(mx[r], fits ? all[bk * NR + r] : __ldcg(a.partial + (size_t)bk * NR + r));
+      mx[r] = block_max(mx[r], red);
+      __syncthreads();
+    }
+  }
   if (tid < NR) {
-    double s = is_max[tid] ? 0.0 : 0.0;
-    for (int bk = 0; bk < (int)gridDim.x; ++bk) {
-      const double t = __ldcg(a.partial + (size_t)bk * NR + tid);
-      s = is_max[tid] ? fmax(s, t) : s + t;
+    double s = 0.0;
+    bool mine_max = false;
+#pragma unroll
+    for (int r = 0; r < NR; ++r)
+      if (tid == r && is_max[r]) { s = mx[r]; mine_max = true; }
+    if (!mine_max) {
+#pragma unroll 8
+      for (int bk = 0; bk < nb; ++bk)
+        s += fits ? all[bk * NR + tid] : __ldcg(a.partial + (size_t)bk * NR + tid);
     }
     red[tid] = s;
   }
@@ -918,7 +1136,9 @@ struct Solver {
       gram_sym_reduce_kernel<<<(et + 127) / 128, 128, 0, st>>>(a.partial, blocks, kx, out, nullptr);
       return kerr("gram");
     }
-    if (kx * ky <= RED_BLOCK) gram_kernel<1><<<blocks, RED_BLOCK, 0, st>>>(a);
+    if (kx * ky <= RED_BLOCK && kx <= GS_MAXC && ky <= GS_MAXC)
+      gram_small_kernel<<<blocks, RED_BLOCK, 0, st>>>(a);
+    else if (kx * ky <= RED_BLOCK) gram_kernel<1><<<blocks, RED_BLOCK, 0, st>>>(a);
     else if (kx * ky <= 4 * RED_BLOCK) gram_kernel<4><<<blocks, RED_BLOCK, 0, st>>>(a);
     else gram_kernel<(IPM_MAXS * IPM_MAXS + RED_BLOCK - 1) / RED_BLOCK><<<blocks, RED_BLOCK, 0, st>>>(a);
     return kerr("gram");
@@ -1094,11 +1314,17 @@ static int body(Solver& X, int t) {
     CK(kerr("mvec_pre"));
   }
   {
-    int blocks = (int)(((long long)L.m * 32 + 255) / 256);
-    if (blocks > X.di.sm_count * 16) blocks = X.di.sm_count * 16;
     ++X.launches;
-    svec_project_kernel<<<blocks, 256, 0, st>>>(L.m, P->con_ptr, P->t_row, P->t_col, P->t_a, V,
-                                                L.ld, L.k, L.Pm, L.m, nullptr);
+    if (L.s <= 15) {
+      const int blocks = (L.m + 255) / 256;
+      svec_project_small_kernel<<<dim3((unsigned)blocks, (unsigned)L.s), 256, 0, st>>>(
+          L.m, P->con_ptr, P->t_row, P->t_col, P->t_a, V, L.ld, L.s, L.Pm, L.m, nullptr);
+    } else {
+      int blocks = (int)(((long long)L.m * 32 + 255) / 256);
+      if (blocks > X.di.sm_count * 16) blocks = X.di.sm_count * 16;
+      svec_project_kernel<<<blocks, 256, 0, st>>>(L.m, P->con_ptr, P->t_row, P->t_col, P->t_a, V,
+                                                  L.ld, L.k, L.Pm, L.m, nullptr);
+    }
     CK(kerr("svec_project"));
     CK(X.gram(L.Pm, L.m, L.s, L.Pm, L.m, L.s, L.m, L.smalls + L.o_QB));   // create_Q_base
   }
@@ -1115,7 +1341,6 @@ static int body(Solver& X, int t) {
   ea.o_Sout = L.o_Sout; ea.o_GC = L.o_GC; ea.o_W = L.o_W; ea.o_Splus = L.o_Splus;
   ea.o_Scplus = L.o_Scplus; ea.o_Wpast = L.o_Wpast; ea.o_VtO = L.o_VtO; ea.o_M = L.o_M;
   ea.o_Mc = L.o_Mc; ea.status = L.status; ea.skip = nullptr;
-  const int qblocks = X.mgrid();
   for (int pass = 0; pass < Pa->subprob_max_iters; ++pass) {
     CK(X.run_ipm(0));
     ++X.launches;
@@ -1129,10 +1354,9 @@ static int body(Solver& X, int t) {
       CK(kerr("rows_update"));
     } else {
       ++X.launches;
-      quadform_kernel<<<qblocks, 256, 0, st>>>(L.m, P->con_ptr, P->t_row, P->t_col, P->t_a, V,
-                                               L.ld, L.k, L.smalls + L.o_Splus,
-                                               L.smalls + L.o_Scplus, L.AF, L.AFc, nullptr);
-      CK(kerr("quadform"));
+      CK(launch_quadform(L.m, P->con_ptr, P->t_row, P->t_col, P->t_a, V, L.ld, L.k,
+                         L.smalls + L.o_Splus, L.smalls + L.o_Scplus, L.AF, L.AFc, X.di.sm_count,
+                         st));
     }
     if (!P->has_ineq) break;       // upsilon stays 0: the loop ends after one pass
     MvecArgs ma = X.margs();
