@@ -342,6 +342,34 @@ __device__ inline bool cta_jacobi_f32(float* A, float* A2, int lda, int n, float
   return ok;
 }
 
+// 2 (sqrt(sum sa) + sqrt(sum aa) sqrt(sum rr)) over the CTA's threads, of which
+// those at or past `count` hold zeros.  The sums are block_sum's (warps in
+// order; warps of zeros add nothing), but only warps with values take part, the
+// three run on three lanes, and so do the square roots: as three block_sums by
+// every thread they took the SM's FP64 unit 8k cycles.
+__device__ __forceinline__ double cta_refine_delta(double sa, double aa, double rr, int count) {
+  __shared__ double part[3][32], out;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int nw = min((int)(blockDim.x >> 5), (count + 31) / 32);
+  if (wid < nw) {
+    sa = warp_sum(sa);
+    aa = warp_sum(aa);
+    rr = warp_sum(rr);
+    if (lane == 0) { part[0][wid] = sa; part[1][wid] = aa; part[2][wid] = rr; }
+  }
+  __syncthreads();
+  if (wid == 0) {
+    double s = 0.0;
+    if (lane < 3)
+      for (int w = 0; w < nw; ++w) s += part[lane][w];
+    s = sqrt(s);
+    const double r1 = __shfl_sync(0xffffffffu, s, 1), r2 = __shfl_sync(0xffffffffu, s, 2);
+    if (lane == 0) out = 2.0 * (s + r1 * r2);
+  }
+  __syncthreads();
+  return out;
+}
+
 // One step of the iterative refinement of a symmetric eigen-decomposition of
 // Ogita & Aishima ("Iterative refinement for symmetric eigenvalue
 // decomposition", Japan J. Indust. Appl. Math. 35, 2018), FP64, whole CTA.
@@ -352,7 +380,7 @@ __device__ inline bool cta_jacobi_f32(float* A, float* A2, int lda, int n, float
 // A, X, R, S, W: n x n row-major with leading dimension ld (shared memory);
 // A is multiplied as a dense matrix.  lam receives the refined eigenvalues.
 __device__ inline void cta_refine_eig(const double* A, double* X, double* R, double* S,
-                                      double* W, double* lam, double* red, int n, int ld) {
+                                      double* W, double* lam, int n, int ld) {
   const int tid = threadIdx.x, nt = blockDim.x;
   // W = A X
   for (int e = tid; e < n * n; e += nt) {
@@ -388,12 +416,7 @@ __device__ inline void cta_refine_eig(const double* A, double* X, double* R, dou
     aa += A[i * ld + j] * A[i * ld + j];
     rr += R[i * ld + j] * R[i * ld + j];
   }
-  sa = block_sum(sa, red);
-  __syncthreads();
-  aa = block_sum(aa, red);
-  __syncthreads();
-  rr = block_sum(rr, red);
-  const double delta = 2.0 * (sqrt(sa) + sqrt(aa) * sqrt(rr));
+  const double delta = cta_refine_delta(sa, aa, rr, n * n);
   // E into W
   for (int e = tid; e < n * n; e += nt) {
     const int i = e / n, j = e - i * n;

@@ -147,7 +147,7 @@ __device__ unsigned pd_tests(const double* S, const double* dS, const double* T,
 
 struct IpmScal {
   double eta, zeta, omega, mu, step, trS, k1, k2, den, ze, F2, d_eta, d_omega, d_zeta, st, cS,
-      cT, q22, h2, t1, t2, t3, t4, rden;
+      cT, q22, h2, t1, t2, t3, t4, rden, mow, moe, lbc;
   int cont, it;
 };
 
@@ -557,11 +557,12 @@ __global__ void __launch_bounds__(IPM_BLOCK, 1) ipm_kernel(const __grid_constant
     if (!sc.cont) break;
     const double mu = sc.mu, eta_ = sc.eta, zeta = sc.zeta, omega = sc.omega, tIS = sc.trS;
     // ---- Newton system ----
-    // The step's scalar coefficients are chains of FP64 divisions, each
-    // holding an SM sub-partition's FP64 pipe for hundreds of cycles: the last
-    // warp forms them once (k1, k2, den, ze, F2, 1/den and, for the quadratic
-    // subproblem, t1 and t2), while the other warps form F1 = Q11 svec(S) + ...
-    // They are read after the barrier that follows the copy of S below.
+    // The step's scalar coefficients are chains of FP64 divisions of about 600
+    // cycles each: the last warp forms them, independent quotients on lanes of
+    // their own (k1, ze, mu/omega and mu/eta together, then 1/den and, for the
+    // quadratic subproblem, t1 and t2, for the lower bound its coefficient and t1),
+    // while the other warps form F1 = Q11 svec(S) + ...  They are read after the
+    // barrier that precedes the inverse below.
     if (wid == IPM_BLOCK / 32 - 1) {
       double F2 = 0.0;
       if (A.mode == 0) {
@@ -569,17 +570,37 @@ __global__ void __launch_bounds__(IPM_BLOCK, 1) ipm_kernel(const __grid_constant
         F2 = d + eta_ * q22 + h2;
         F2 = F2 + (-zeta + omega);
       }
+      F2 = __shfl_sync(0xffffffffu, F2, 0);
+      const double q4 = (lane == 0 ? 1 - tIS - eta_ : lane == 1 ? zeta : mu) /
+                        ((lane & 1) ? eta_ : omega);
+      const double k1 = __shfl_sync(0xffffffffu, q4, 0), ze = __shfl_sync(0xffffffffu, q4, 1);
+      const double mow = __shfl_sync(0xffffffffu, q4, 2), moe = __shfl_sync(0xffffffffu, q4, 3);
+      const double k2 = ze + q22;
+      const double den = fma(k1, k2, 1.0);
+      double num, dv;
+      if (A.mode == 0) {
+        const double lin = mow + tIS + eta_ - 1;
+        num = (lane == 1) ? fma(k1, F2 - moe + zeta, lin)
+            : (lane == 2) ? fma(-k2, lin, F2 - moe + zeta) : 1.0;
+        dv = den;
+      } else {
+        num = (lane == 1) ? ze * (fma(-k1, moe - h2 - omega, mow) + tIS + eta_ - 1)
+            : (lane == 2) ? ze : 1.0;
+        dv = (lane == 1) ? fma(-k1, ze, -1.0) : (lane == 2) ? fma(k1, ze, 1.0) : den;
+      }
+      const double q3 = num / dv;
+      const double t1 = __shfl_sync(0xffffffffu, q3, 1), t2 = __shfl_sync(0xffffffffu, q3, 2);
       if (lane == 0) {
-        const double k1 = (1 - tIS - eta_) / omega;
-        const double k2 = zeta / eta_ + q22;
-        const double den = k1 * k2 + 1;
-        const double ze = zeta / eta_;
         sc.k1 = k1; sc.k2 = k2; sc.den = den; sc.ze = ze;
         sc.F2 = F2;
-        sc.rden = 1.0 / den;
+        sc.mow = mow; sc.moe = moe;
+        sc.rden = q3;
+        sc.t1 = t1;
         if (A.mode == 0) {
-          sc.t1 = (mu / omega + tIS + eta_ - 1 + k1 * (F2 - mu / eta_ + zeta)) / den;
-          sc.t2 = (F2 - mu / eta_ + zeta - k2 * (mu / omega + tIS + eta_ - 1)) / den;
+          sc.t2 = t2;
+        } else {
+          sc.lbc = t2;
+          sc.t2 = h2 - moe;
         }
       }
     }
@@ -603,7 +624,7 @@ __global__ void __launch_bounds__(IPM_BLOCK, 1) ipm_kernel(const __grid_constant
     // coefficient matrix, every entry computed (S^-1 is not exactly symmetric in
     // floating point; mirroring one triangle measurably degrades the Newton
     // steps once the system is ill-conditioned near the end of the IPM)
-    const double lbc = (A.mode == 1) ? (ze / (k1 * ze + 1)) : 0.0;
+    const double lbc = (A.mode == 1) ? sc.lbc : 0.0;
     const double rden = sc.rden;
     if (A.mode == 0) {
       for (int a2 = tid; a2 < s; a2 += IPM_BLOCK) {
@@ -626,10 +647,6 @@ __global__ void __launch_bounds__(IPM_BLOCK, 1) ipm_kernel(const __grid_constant
         v += lbc * (sh.sI[a] * sh.sI[a2]);
       }
       coeff[a2 * s + a] = v;
-    }
-    if (tid == 0 && A.mode == 1) {
-      sc.t1 = ze * (-k1 * (mu / eta_ - h2 - omega) + mu / omega + tIS + eta_ - 1) / (-k1 * ze - 1);
-      sc.t2 = h2 - mu / eta_;
     }
     __syncthreads();
     for (int a = tid; a < s; a += IPM_BLOCK) {
@@ -665,21 +682,30 @@ __global__ void __launch_bounds__(IPM_BLOCK, 1) ipm_kernel(const __grid_constant
       }
       t1 = warp_sum(t1);
       if (A.mode == 0) { t2 = warp_sum(t2); t3 = warp_sum(t3); }
+      // (every lane the same, but for one quotient per lane)
+      const double mow = sc.mow, moe = sc.moe;
+      double d_eta, d_omega, d_zeta;
+      if (A.mode == 0) {
+        const double ne = fma(k1, -F2 + moe - zeta, -t1 - mow - tIS - eta_ + 1);
+        const double no = fma(k2, mow + tIS + eta_ - 1, -F2 + moe - zeta) - t2;
+        const double qd = (lane == 0 ? ne : no) / den;
+        d_eta = __shfl_sync(0xffffffffu, qd, 0);
+        d_omega = __shfl_sync(0xffffffffu, qd, 1);
+        d_zeta = fma(d_eta, q22, t3) + d_omega + F2;
+      } else {
+        d_eta = (fma(-k1, moe - h2 - omega, t1) + mow + tIS + eta_ - 1) / fma(-k1, ze, -1.0);
+        d_omega = fma(-ze, d_eta, moe);
+        d_omega = d_omega + (-h2 - omega);
+        d_zeta = d_omega - zeta + h2 + omega;
+      }
+      // step size from the linear variables (solver/usbs.py:128-132)
+      const double qr = (lane == 0 ? d_eta : lane == 1 ? d_zeta : d_omega) /
+                        (lane == 0 ? eta_ : lane == 1 ? zeta : omega);
+      const double r = nanmin2(nanmin2(__shfl_sync(0xffffffffu, qr, 0),
+                                       __shfl_sync(0xffffffffu, qr, 1)),
+                               __shfl_sync(0xffffffffu, qr, 2));
       if (lane == 0) {
-        double d_eta, d_omega, d_zeta;
-        if (A.mode == 0) {
-          d_eta = (-t1 - (mu / omega) - tIS - eta_ + 1 + k1 * (-F2 + mu / eta_ - zeta)) / den;
-          d_omega = (-F2 + mu / eta_ - zeta + k2 * (mu / omega + tIS + eta_ - 1) - t2) / den;
-          d_zeta = t3 + d_eta * q22 + d_omega + F2;
-        } else {
-          d_eta = (t1 - k1 * (mu / eta_ - h2 - omega) + mu / omega + tIS + eta_ - 1) / (-k1 * ze - 1);
-          d_omega = -ze * d_eta + mu / eta_;
-          d_omega = d_omega + (-h2 - omega);
-          d_zeta = d_omega - zeta + h2 + omega;
-        }
         sc.d_eta = d_eta; sc.d_omega = d_omega; sc.d_zeta = d_zeta;
-        // step size from the linear variables (solver/usbs.py:128-132)
-        const double r = nanmin2(nanmin2(d_eta / eta_, d_zeta / zeta), d_omega / omega);
         double st = -1.0 / r;
         if (!isnan(st) && st > 1.0) st = 1.0;
         sc.st = 0.99 * ((st <= 0.0) ? 1.0 : st);
@@ -809,7 +835,7 @@ __global__ void __launch_bounds__(IPM_BLOCK) eigS_kernel(EigSArgs A) {
   if (A.skip && *A.skip) return;
   constexpr int L = 16;                               // ld of the FP64 k x k blocks
   __shared__ double Sd[L * L], Z[L * L], R[L * L], S2[L * L], Wb[L * L], lam[L];
-  __shared__ double GW[IPM_MAXK * IPM_MAXK], red[IPM_BLOCK / 32];
+  __shared__ double GW[IPM_MAXK * IPM_MAXK];
   __shared__ float Af[2 * (L + 1) + L * L + L], Af2[2 * (L + 1) + L * L + L], Zf[L * (L + 1)];
   __shared__ float wf[L], redf[32];
   __shared__ int order[L];
@@ -830,8 +856,8 @@ __global__ void __launch_bounds__(IPM_BLOCK) eigS_kernel(EigSArgs A) {
     Z[r * L + c] = (double)Zf[r * (L + 1) + c];
   }
   __syncthreads();
-  cta_refine_eig(Sd, Z, R, S2, Wb, lam, red, k, L);
-  cta_refine_eig(Sd, Z, R, S2, Wb, lam, red, k, L);
+  cta_refine_eig(Sd, Z, R, S2, Wb, lam, k, L);
+  cta_refine_eig(Sd, Z, R, S2, Wb, lam, k, L);
   if (tid < k) {
     const double v = lam[tid];
     int r = 0;

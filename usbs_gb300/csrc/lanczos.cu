@@ -393,7 +393,7 @@ __device__ __forceinline__ void cl_share(double* p, int C, double v) {
 // them to every CTA.  The products are 4 n^3 FP64 FMAs at 2 per clock and SM:
 // done by every CTA redundantly they took 170k cycles per step (n = 32).
 __device__ inline void cl_refine_eig(const double* A, double* X, double* R, double* S, double* W,
-                                     double* lam, double* red, int n, int ld, int rank, int C) {
+                                     double* lam, int n, int ld, int rank, int C) {
   const int tid = threadIdx.x, nt = blockDim.x, nn = n * n;
   const int e0 = nn * rank / C, e1 = nn * (rank + 1) / C;
   // W = A X
@@ -430,12 +430,7 @@ __device__ inline void cl_refine_eig(const double* A, double* X, double* R, doub
     aa += A[i * ld + j] * A[i * ld + j];
     rr += R[i * ld + j] * R[i * ld + j];
   }
-  sa = block_sum(sa, red);
-  __syncthreads();
-  aa = block_sum(aa, red);
-  __syncthreads();
-  rr = block_sum(rr, red);
-  const double delta = 2.0 * (sqrt(sa) + sqrt(aa) * sqrt(rr));
+  const double delta = cta_refine_delta(sa, aa, rr, nn);
   // E into W (every CTA is past its last read of the old W)
   for (int e = e0 + tid; e < e1; e += nt) {
     const int i = e / n, j = e - i * n;
@@ -549,9 +544,9 @@ __device__ void restart_select(const D& P, LzShared<VT>& sh, int k, bool write_o
     if constexpr (LOCAL_YS) cl_sync();
     for (int it = 0; it < 2; ++it) {
       if constexpr (LOCAL_YS)
-        cl_refine_eig(T, X, sh.u.rs.R, sh.u.rs.S, sh.u.rs.W, sh.ritz, sh.red, m, MP1, rank, C);
+        cl_refine_eig(T, X, sh.u.rs.R, sh.u.rs.S, sh.u.rs.W, sh.ritz, m, MP1, rank, C);
       else
-        cta_refine_eig(T, X, sh.u.rs.R, sh.u.rs.S, sh.u.rs.W, sh.ritz, sh.red, m, MP1);
+        cta_refine_eig(T, X, sh.u.rs.R, sh.u.rs.S, sh.u.rs.W, sh.ritz, m, MP1);
     }
     select_order(sh.ritz, m, sh.order);
     __syncthreads();

@@ -3,9 +3,10 @@
 // On GB300 a dependent FP64 instruction takes 60 cycles (150 while all eight warps
 // of a CTA use the SM's FP64 unit), and 1 / x is a chain of them: 350 cycles alone,
 // 660 with eight warps.  The integer pipes are otherwise idle in the kernels
-// that wait for one pivot's reciprocal: 310 and 370 cycles here.  Newton's iteration for 1/d in fixed point from the FP32
-// hardware approximation (about 2^-22), then the exact remainder decides the
-// rounding, so the result is that of an IEEE division.
+// that wait for one pivot's reciprocal: 310 and 370 cycles here.  Newton's
+// iteration for 1/d in fixed point from the FP32 hardware approximation (about
+// 2^-22), then the exact remainder decides the rounding, so the result is that of
+// an IEEE division.
 #pragma once
 #include <stdint.h>
 
