@@ -55,10 +55,32 @@ __device__ inline bool warp_syev(double* A, int lda, int n, double* w, double* Z
     __syncwarp();
     if (lane == r0) { A[r0 * lda + j] = nrm; A[j * lda + r0] = nrm; }
     if (lane > r0 && lane < n) { A[lane * lda + j] = 0.0; A[j * lda + lane] = 0.0; }
-    // Z <- Z (I - beta v v^T): row i of Z: z_i -= beta (z_i . v) v^T
-    for (int i = 0; i < n; ++i) {
-      double zv = warp_sum((lane < n) ? Z[i * ldz + lane] * vi : 0.0);
-      if (lane < n) Z[i * ldz + lane] -= beta * zv * vi;
+    // Z <- Z (I - beta v v^T): row i of Z: z_i -= beta (z_i . v) v^T, the rows'
+    // dots 16 at a time by a butterfly whose payload halves (lanes 2 i and
+    // 2 i + 1 end with row i's, summed as by a warp sum)
+    for (int i0 = 0; i0 < n; i0 += 16) {
+      double zr[16], x[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        zr[i] = (lane < n && i0 + i < n) ? Z[(i0 + i) * ldz + lane] : 0.0;
+        x[i] = (lane < n && i0 + i < n) ? zr[i] * vi : 0.0;
+      }
+#pragma unroll
+      for (int h = 16, w = 8; w >= 1; h >>= 1, w >>= 1) {
+        const bool up = (lane & h) != 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          if (i < w) {
+            const double send = up ? x[i] : x[i + w], keep = up ? x[i + w] : x[i];
+            x[i] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+          }
+      }
+      const double bz = beta * (x[0] + __shfl_xor_sync(0xffffffffu, x[0], 1));
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const double b = __shfl_sync(0xffffffffu, bz, 2 * i);
+        if (lane < n && i0 + i < n) Z[(i0 + i) * ldz + lane] = fma(-b, vi, zr[i]);
+      }
     }
     __syncwarp();
   }
@@ -84,17 +106,21 @@ __device__ inline bool warp_syev(double* A, int lda, int n, double* w, double* Z
         continue;
       }
     }
-    // start p of the unreduced block ending at hi
-    int p = hi - 1;
-    while (p > 0) {
-      double e = A[p * lda + p - 1];
-      if (fabs(e) <= eps * (fabs(d[p - 1]) + fabs(d[p])) || fabs(e) < 1e-300) {
-        __syncwarp();
-        if (lane == 0) A[p * lda + p - 1] = 0.0;
-        __syncwarp();
-        break;
+    // start p of the unreduced block ending at hi: the last negligible
+    // subdiagonal below it (lane p looks at p, p - 1), which becomes zero
+    int p = 0;
+    {
+      bool neg = false;
+      if (lane >= 1 && lane < hi) {
+        const double e = A[lane * lda + lane - 1];
+        neg = fabs(e) <= eps * (fabs(d[lane - 1]) + fabs(d[lane])) || fabs(e) < 1e-300;
       }
-      --p;
+      const unsigned nb = __ballot_sync(0xffffffffu, neg);
+      if (nb) {
+        p = 31 - __clz(nb);
+        if (lane == p) A[p * lda + p - 1] = 0.0;
+        __syncwarp();
+      }
     }
     if (++iters > maxit) return false;
     // Wilkinson shift from the trailing 2x2
@@ -105,8 +131,9 @@ __device__ inline bool warp_syev(double* A, int lda, int n, double* w, double* Z
     double x = d[p] - mu, z = A[(p + 1) * lda + p];
     for (int k = p; k < hi; ++k) {
       double r = hypot(x, z);
-      double c = (r == 0.0) ? 1.0 : x / r;
-      double s = (r == 0.0) ? 0.0 : z / r;
+      // (both quotients in one division, on even and odd lanes)
+      const double cs = (r == 0.0) ? ((lane & 1) ? 0.0 : 1.0) : ((lane & 1) ? z : x) / r;
+      const double c = __shfl_sync(0xffffffffu, cs, 0), s = __shfl_sync(0xffffffffu, cs, 1);
       double ak = d[k], ak1 = d[k + 1], bk = A[(k + 1) * lda + k];
       double f = (k + 1 < hi) ? A[(k + 2) * lda + k + 1] : 0.0;
       // new 2x2 block

@@ -116,40 +116,90 @@ __global__ void __launch_bounds__(RD_BLOCK) rd_gram_kernel(int n, int s, int ld,
   }
 }
 
-// one CTA: sums the Gram partials in block order, then warp 0 forms rho, L,
-// M^T M and its eigen-decomposition, T and Lambda (see the file comment)
-__global__ void __launch_bounds__(RD_BLOCK) rd_small_kernel(int n, int s, int nblocks,
-                                                            double eps,
-                                                            const double* __restrict__ gpart,
+// Sums of the Gram partials in four interleaved chains over the blocks, four
+// threads per entry, one chain each: the chains are dependent FP64 adds (60
+// cycles), and all of them on one SM took its FP64 unit 40 us.  gsum: 3 s^2.
+constexpr int RD_RED = 64;
+__global__ void __launch_bounds__(RD_RED) rd_reduce_kernel(int E, int nblocks,
+                                                           const double* __restrict__ gpart,
+                                                           double* __restrict__ gsum) {
+  const int t = blockIdx.x * RD_RED + threadIdx.x, e = t >> 2, ch = t & 3;
+  double a = 0.0;
+  if (e < E) {
+    const int full = nblocks & ~3;
+    const double* src = gpart + (size_t)ch * E + e;
+    int b = 0;
+    for (; b + 28 < full; b += 32) {
+      double w[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) w[u] = src[(size_t)(b + 4 * u) * E];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) a += w[u];
+    }
+    for (; b < full; b += 4) a += src[(size_t)b * E];
+    if (ch == 0)
+      for (b = full; b < nblocks; ++b) a += gpart[(size_t)b * E + e];
+  }
+  a += __shfl_xor_sync(0xffffffffu, a, 1);         // (a0 + a1) and (a2 + a3)
+  a += __shfl_xor_sync(0xffffffffu, a, 2);
+  if (e < E && ch == 0) gsum[e] = a;
+}
+
+// one CTA: rho from the largest eigenvalue of P^T P, then warp 0 forms L, M^T M
+// and its eigen-decomposition, T and Lambda (see the file comment).  The largest
+// eigenvalue alone comes from the FP32 Jacobi refined to FP64 by two
+// Ogita-Aishima steps (on the matrix scaled by a power of two); the
+// decomposition of M^T M keeps the QR iteration, whose vectors' signs are the
+// result's.  Bound by the QR iteration's chain of FP64 instructions on one warp: 297 us
+// at s = 10 (593 with both decompositions by QR and the partials summed here).
+__global__ void __launch_bounds__(RD_BLOCK) rd_small_kernel(int n, int s, double eps,
+                                                            const double* __restrict__ gsum,
                                                             double* __restrict__ small) {
   __shared__ double G[3 * RD_MAXS * RD_MAXS];
   __shared__ double A[RD_MAXS * RD_LD], Lm[RD_MAXS * RD_LD], K[RD_MAXS * RD_LD];
-  __shared__ double Z[RD_MAXS * RD_LD], w[RD_MAXS];
+  __shared__ double Z[RD_MAXS * RD_LD], X[RD_MAXS * RD_LD], w[RD_MAXS];
+  __shared__ float wf[RD_MAXS], redf[2];
+  __shared__ unsigned emax;
   const int tid = threadIdx.x, lane = tid & 31, s2 = s * s, E = 3 * s2;
+  if (tid == 0) emax = 0u;
+  __syncthreads();
   for (int e = tid; e < E; e += RD_BLOCK) {
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-    int b = 0;
-    for (; b + 3 < nblocks; b += 4) {
-      a0 += gpart[(size_t)b * E + e];
-      a1 += gpart[(size_t)(b + 1) * E + e];
-      a2 += gpart[(size_t)(b + 2) * E + e];
-      a3 += gpart[(size_t)(b + 3) * E + e];
-    }
-    for (; b < nblocks; ++b) a0 += gpart[(size_t)b * E + e];
-    G[e] = (a0 + a1) + (a2 + a3);
+    const double g = gsum[e];
+    G[e] = g;
+    if (e < s2) atomicMax(&emax, (unsigned)((__double_as_longlong(g) >> 52) & 0x7ff));
   }
   __syncthreads();
+  bool conv = true;
+  double lmax;
+  {
+    // P^T P scaled to entries below 2 (exact, but for entries that underflow)
+    const int sh = (emax == 0u || emax == 0x7ffu) ? 0 : 1023 - (int)emax;
+    const double f = scalbn(1.0, sh);
+    float* Af = (float*)Lm;                          // each of 33^2 doubles' room
+    float* Bf = (float*)K;
+    float* Zf = (float*)Z;
+    for (int e = tid; e < s2; e += RD_BLOCK) {
+      const int i = e / s, j = e - i * s;
+      const double g = G[e] * f;
+      A[i * RD_LD + j] = g;
+      Af[i * RD_LD + j] = (float)g;
+    }
+    __syncthreads();
+    if (s <= 16) conv = cta_jacobi_f32<16>(Af, Bf, RD_LD, s, wf, Zf, RD_LD, redf);
+    else conv = cta_jacobi_f32<32>(Af, Bf, RD_LD, s, wf, Zf, RD_LD, redf);
+    for (int e = tid; e < s2; e += RD_BLOCK) {
+      const int i = e / s, j = e - i * s;
+      X[i * RD_LD + j] = (double)Zf[i * RD_LD + j];
+    }
+    __syncthreads();
+    for (int it = 0; it < 2; ++it) cta_refine_eig(A, X, Lm, K, Z, w, s, RD_LD);
+    lmax = warp_max(w[lane < s ? lane : 0]) * scalbn(1.0, -sh);
+    __syncthreads();
+  }
   if (tid >= 32) return;
   const double* PtP = G;
   const double* OtP = G + s2;
   const double* OtO = G + 2 * s2;
-  // ||P||_2 from the largest eigenvalue of P^T P
-  for (int i = 0; i < s; ++i)
-    if (lane < s) A[i * RD_LD + lane] = PtP[i * s + lane];
-  __syncwarp();
-  bool conv = warp_syev(A, RD_LD, s, w, Z, RD_LD);
-  __syncwarp();
-  const double lmax = w[s - 1];
   const double rho = sqrt((double)n) * eps * sqrt(lmax > 0.0 ? lmax : 0.0);
   // B = sym(Omega^T P + rho Omega^T Omega) into Lm, then its Cholesky factor
   for (int i = 0; i < s; ++i)
@@ -215,22 +265,14 @@ __global__ void __launch_bounds__(RD_BLOCK) rd_small_kernel(int n, int s, int nb
       const double sig2 = w[src];
       const double rh = sqrt(sig2 > 0.0 ? sig2 : 0.0);
       const double inv = rh > 0.0 ? 1.0 / rh : 0.0;
-      double t[RD_MAXS];
-#pragma unroll
-      for (int i = RD_MAXS - 1; i >= 0; --i) {
-        if (i < s) {
-          double v = Z[i * RD_LD + src];
-#pragma unroll
-          for (int k = i + 1; k < RD_MAXS; ++k)
-            if (k < s) v -= Lm[k * RD_LD + i] * t[k];
-          t[i] = v / Lm[i * RD_LD + i];
-        } else {
-          t[i] = 0.0;
-        }
+      // (column `lane` of K holds t: loops of s steps, where 32 guarded ones
+      // unrolled were mostly instruction fetches)
+      for (int i = s - 1; i >= 0; --i) {
+        double v = Z[i * RD_LD + src];
+        for (int k = i + 1; k < s; ++k) v -= Lm[k * RD_LD + i] * K[k * RD_LD + lane];
+        K[i * RD_LD + lane] = v / Lm[i * RD_LD + i];
       }
-#pragma unroll
-      for (int i = 0; i < RD_MAXS; ++i)
-        if (i < s) small[RD_T + i * RD_MAXS + lane] = t[i] * inv;
+      for (int i = 0; i < s; ++i) small[RD_T + i * RD_MAXS + lane] = K[i * RD_LD + lane] * inv;
       const double lam = rh * rh - rho;
       small[RD_LAM + lane] = lam > 0.0 ? lam : 0.0;
     }
@@ -246,28 +288,32 @@ __global__ void __launch_bounds__(RD_BLOCK) rd_small_kernel(int n, int s, int nb
   }
 }
 
-// E = P_rho T (optional) and the sign word of each row (bit j: E[r, j] > 0)
-__global__ void __launch_bounds__(RD_BLOCK) rd_sign_kernel(int n, int s, int ld,
-                                                           const double* __restrict__ P,
-                                                           const double* __restrict__ Om,
-                                                           const double* __restrict__ small,
-                                                           unsigned* __restrict__ bits,
-                                                           double* __restrict__ E, int lde) {
-  __shared__ double T[RD_MAXS * RD_MAXS];
-  for (int e = threadIdx.x; e < s * RD_MAXS; e += RD_BLOCK) T[e] = small[RD_T + e];
+// E = P_rho T (optional) and the sign word of each row (bit j: E[r, j] > 0).  One
+// thread per row, small blocks so that a sketch of 10^4 rows reaches every SM's
+// FP64 unit (30 us with 40 blocks of 256).  MS >= s: register rows.
+constexpr int RD_SIGN = 64;
+template <int MS>
+__global__ void __launch_bounds__(RD_SIGN) rd_sign_kernel(int n, int s, int ld,
+                                                          const double* __restrict__ P,
+                                                          const double* __restrict__ Om,
+                                                          const double* __restrict__ small,
+                                                          unsigned* __restrict__ bits,
+                                                          double* __restrict__ E, int lde) {
+  __shared__ double T[MS * RD_MAXS];
+  for (int e = threadIdx.x; e < s * RD_MAXS; e += RD_SIGN) T[e] = small[RD_T + e];
   __syncthreads();
   const double rho = small[RD_RHO];
   const bool ok = small[RD_OK] != 0.0;
-  for (int r = blockIdx.x * RD_BLOCK + threadIdx.x; r < n; r += gridDim.x * RD_BLOCK) {
-    double pr[RD_MAXS];
+  for (int r = blockIdx.x * RD_SIGN + threadIdx.x; r < n; r += gridDim.x * RD_SIGN) {
+    double pr[MS];
 #pragma unroll
-    for (int i = 0; i < RD_MAXS; ++i)
+    for (int i = 0; i < MS; ++i)
       pr[i] = (i < s) ? P[(size_t)i * ld + r] + rho * Om[(size_t)i * ld + r] : 0.0;
     unsigned word = 0u;
     for (int j = 0; j < s; ++j) {
       double e = 0.0;
 #pragma unroll
-      for (int i = 0; i < RD_MAXS; ++i)
+      for (int i = 0; i < MS; ++i)
         if (i < s) e += pr[i] * T[i * RD_MAXS + j];
       if (ok && e > 0.0) word |= 1u << j;
       if (E) E[(size_t)j * lde + r] = e;
@@ -470,9 +516,14 @@ static int rd_reconstruct(int n, int s, const double* Om, const double* P, int l
   if (E3 <= RD_BLOCK) rd_gram_kernel<1><<<gb, RD_BLOCK, 0, st>>>(n, s, ld, P, Om, w.gpart);
   else if (E3 <= 4 * RD_BLOCK) rd_gram_kernel<4><<<gb, RD_BLOCK, 0, st>>>(n, s, ld, P, Om, w.gpart);
   else rd_gram_kernel<12><<<gb, RD_BLOCK, 0, st>>>(n, s, ld, P, Om, w.gpart);
-  rd_small_kernel<<<1, RD_BLOCK, 0, st>>>(n, s, gb, eps, w.gpart, w.small);
-  const int sb = rd_blocks(n, RD_BLOCK, 4 * 152);
-  rd_sign_kernel<<<sb, RD_BLOCK, 0, st>>>(n, s, ld, P, Om, w.small, w.bits, E, lde);
+  // (the cut partials' buffer is free until the cut pass)
+  rd_reduce_kernel<<<(4 * E3 + RD_RED - 1) / RD_RED, RD_RED, 0, st>>>(E3, gb, w.gpart, w.cpart);
+  rd_small_kernel<<<1, RD_BLOCK, 0, st>>>(n, s, eps, w.cpart, w.small);
+  const int sb = (int)(((long long)n + RD_SIGN - 1) / RD_SIGN < 16 * 152
+                           ? ((long long)n + RD_SIGN - 1) / RD_SIGN : 16 * 152);
+  if (s <= 8) rd_sign_kernel<8><<<sb, RD_SIGN, 0, st>>>(n, s, ld, P, Om, w.small, w.bits, E, lde);
+  else if (s <= 16) rd_sign_kernel<16><<<sb, RD_SIGN, 0, st>>>(n, s, ld, P, Om, w.small, w.bits, E, lde);
+  else rd_sign_kernel<32><<<sb, RD_SIGN, 0, st>>>(n, s, ld, P, Om, w.small, w.bits, E, lde);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_error("reconstruct_from_sketch: launch failed: %s", cudaGetErrorString(e));
