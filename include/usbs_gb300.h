@@ -63,6 +63,14 @@ int usbs_operator_apply(int n, long long nnz, const int* rowptr, const int* col,
                         const void* op_val, const void* x, void* y, int precision,
                         void* stream);
 
+/* y = (c_scale C + A*(w)) x in one pass: usbs_assemble_operator and
+ * usbs_operator_apply without the assembled values (same result, bit for bit). */
+int usbs_operator_apply_direct(int n, long long nnz, const int* rowptr, const int* col,
+                               const double* c_val, double c_scale, const int* slot_ptr,
+                               const int* slot_tid, const int* t_con, const double* t_a,
+                               const double* w, const void* x, void* y, int precision,
+                               void* stream);
+
 /* y = Op x with the operator in the sliced-ELL layout built by
  * usbs_gb300.problem.sell_layout: rows in windows of 256, sorted by length
  * inside a window and cut into 32-row slices; slice s holds its entries

@@ -25,24 +25,33 @@ from .arrays import as_torch, shape_of, to_device
 from .problem import DeviceProblem, layout
 
 
+_checked_torch = None      # torch, once a CUDA device has been seen
+
+
 def _torch():
-    import torch
-    if not torch.cuda.is_available():
-        raise RuntimeError("usbs_gb300 needs a CUDA device (GB300, sm_103a); none is visible")
-    return torch
+    global _checked_torch
+    if _checked_torch is None:
+        import torch
+        if not torch.cuda.is_available():
+            raise RuntimeError("usbs_gb300 needs a CUDA device (GB300, sm_103a); none is visible")
+        _checked_torch = torch
+    return _checked_torch
 
 
 def _p(t):
-    return ctypes.c_void_p(int(t.data_ptr())) if t is not None else ctypes.c_void_p(0)
+    """A tensor's address as the ctypes signatures take it (None: a null pointer)."""
+    return t.data_ptr() if t is not None else None
 
 
 def _stream():
-    torch = _torch()
-    return ctypes.c_void_p(int(torch.cuda.current_stream().cuda_stream))
+    return _torch().cuda.current_stream().cuda_stream
 
 
 def _dev(x, dtype, device):
-    _torch()
+    torch = _torch()
+    # the common case, a resident tensor of the right kind, without the conversions
+    if type(x) is torch.Tensor and x.dtype is dtype and x.device == device and x.is_contiguous():
+        return x
     return to_device(x, dtype, device)
 
 
@@ -105,12 +114,19 @@ def _problem_for(C, A_data, A_indices, m, device, *, make=None):
 
 def _cols(U, n, device):
     """Column-major device copy of an (n,) or (n, k) array: returns (tensor[k, ld], ld, k)."""
-    torch = _torch()
-    Ut = _dev(U, torch.float64, device)
+    Ut = _dev_any(U, device)
     if Ut.dim() == 1:
         Ut = Ut.reshape(n, 1)
-    k = Ut.shape[1]
-    return Ut.t().contiguous(), n, k
+    Ut = Ut.t()
+    return Ut if Ut.is_contiguous() else Ut.contiguous(), n, Ut.shape[0]
+
+
+def _dev_any(U, device):
+    """U as a float64 tensor on `device`; one that already is keeps its strides."""
+    torch = _torch()
+    if type(U) is torch.Tensor and U.dtype is torch.float64 and U.device == device:
+        return U
+    return to_device(U, torch.float64, device)
 
 
 def apply_A_operator_batched(m, A_data, A_indices, vecs, *, problem=None, n=None, device="cuda"):
@@ -120,8 +136,9 @@ def apply_A_operator_batched(m, A_data, A_indices, vecs, *, problem=None, n=None
     if problem is None:
         nn = n if n is not None else int(shape_of(vecs)[0])
         problem = _problem_for(sp.csr_matrix((nn, nn)), A_data, A_indices, m, device)
-    Ucm, ld, k = _cols(vecs, problem.n, problem.device)
-    out = torch.empty(m, dtype=torch.float64, device=problem.device)
+    dev = problem.c_val.device
+    Ucm, ld, k = _cols(vecs, problem.n, dev)
+    out = torch.empty(m, dtype=torch.float64, device=dev)
     _lib.check(lib.usbs_apply_A_operator(m, k, _p(problem.con_ptr), _p(problem.t_row),
                                          _p(problem.t_col), _p(problem.t_a), _p(Ucm), ld,
                                          _p(out), _stream()), "usbs_apply_A_operator")
@@ -137,11 +154,12 @@ def apply_A_adjoint_batched(n, A_data, A_indices, z, vecs, *, problem=None, devi
     """[A*(z) v_j]_j for the columns of ``vecs`` -> (n, k) float64."""
     torch = _torch()
     lib = _lib.load()
-    zz = _dev(z, torch.float64, device if problem is None else problem.device)
+    zz = _dev(z, torch.float64, device if problem is None else problem.c_val.device)
     if problem is None:
         problem = _problem_for(sp.csr_matrix((n, n)), A_data, A_indices, zz.numel(), device)
-    Ucm, ld, k = _cols(vecs, n, problem.device)
-    out = torch.empty((k, n), dtype=torch.float64, device=problem.device)
+    dev = problem.c_val.device
+    Ucm, ld, k = _cols(vecs, n, dev)
+    out = torch.empty((k, n), dtype=torch.float64, device=dev)
     _lib.check(lib.usbs_apply_A_adjoint(n, k, _p(problem.row_ptr), _p(problem.r_con),
                                         _p(problem.r_col), _p(problem.r_a), _p(zz), _p(Ucm), ld,
                                         _p(out), n, _stream()), "usbs_apply_A_adjoint")
@@ -158,18 +176,15 @@ def operator_apply(problem, c_scale, w, x, precision=64):
     torch = _torch()
     lib = _lib.load()
     vt = _vt(precision)
-    dev = problem.device
-    op = torch.empty(max(problem.nnz, 1), dtype=vt, device=dev)
+    dev = problem.c_val.device
     wt = _dev(w, torch.float64, dev) if w is not None else None
-    _lib.check(lib.usbs_assemble_operator(problem.nnz, _p(problem.c_val), float(c_scale),
-                                          _p(problem.slot_ptr), _p(problem.slot_tid),
-                                          _p(problem.t_con), _p(problem.t_a0), _p(wt), _p(op),
-                                          precision, _stream()), "usbs_assemble_operator")
     xt = _dev(x, vt, dev)
     y = torch.empty(problem.n, dtype=vt, device=dev)
-    _lib.check(lib.usbs_operator_apply(problem.n, problem.nnz, _p(problem.rowptr),
-                                       _p(problem.col), _p(op), _p(xt), _p(y), precision,
-                                       _stream()), "usbs_operator_apply")
+    _lib.check(lib.usbs_operator_apply_direct(
+        problem.n, problem.nnz, _p(problem.rowptr), _p(problem.col), _p(problem.c_val),
+        float(c_scale), _p(problem.slot_ptr), _p(problem.slot_tid), _p(problem.t_con),
+        _p(problem.t_a0), _p(wt), _p(xt), _p(y), precision, _stream()),
+        "usbs_operator_apply_direct")
     return y
 
 

@@ -155,6 +155,25 @@ int usbs_operator_apply(int n, long long nnz, const int* rowptr, const int* col,
                   (cudaStream_t)stream);
 }
 
+int usbs_operator_apply_direct(int n, long long nnz, const int* rowptr, const int* col,
+                               const double* c_val, double c_scale, const int* slot_ptr,
+                               const int* slot_tid, const int* t_con, const double* t_a,
+                               const double* w, const void* x, void* y, int precision,
+                               void* stream) {
+  if (precision != 32 && precision != 64) { set_error("precision must be 32 or 64"); return -2; }
+  if (n < 0) { set_error("n < 0"); return -2; }
+  if (nnz < 0 || nnz > 0x7fffffffLL) { set_error("nnz %lld out of range", nnz); return -2; }
+  if (w && (!slot_ptr || !slot_tid || !t_con || !t_a)) {
+    set_error("operator_apply_direct: w given without the slot map / triples");
+    return -2;
+  }
+  DeviceInfo di;
+  int rc = get_device_info(&di);
+  if (rc) return rc;
+  return fused_apply(n, nnz, rowptr, col, c_val, c_scale, slot_ptr, slot_tid, t_con, t_a, w, x, y,
+                     precision, di.sm_count, (cudaStream_t)stream);
+}
+
 int usbs_operator_apply_sell(int n, const int* sl_ptr, const int* sl_col, const void* sl_val,
                              const unsigned char* sl_row, const void* x, void* y, int precision,
                              void* stream) {

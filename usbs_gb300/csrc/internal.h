@@ -70,6 +70,10 @@ int assemble_operator(int nnz, const double* c_val, double alpha_c, const int* s
                       const int* slot_tid, const int* con, const double* a, const double* w,
                       void* op_val, int prec, cudaStream_t stream);
 // y = M x  for CSR M (values double or float), optional per-row partial dots
+int fused_apply(int n, long long nnz, const int* rowptr, const int* col, const double* c_val,
+                double alpha_c, const int* slot_ptr, const int* slot_tid, const int* con,
+                const double* a, const double* w, const void* x, void* y, int prec, int sm_count,
+                cudaStream_t stream);
 int csr_spmv(int n, long long nnz, const int* rowptr, const int* col, const void* val,
              const void* x, void* y, int prec, int sm_count, cudaStream_t stream);
 // y = M x for M in the sliced-ELL layout (windows of 256 rows, 32-row slices)

@@ -36,6 +36,10 @@ __device__ __forceinline__ double scaled(double alpha, unsigned long long sgn, d
                        : __longlong_as_double(__double_as_longlong(x) ^ (long long)sgn);
 }
 
+static unsigned long long sign_of_scale(double alpha) {
+  return (alpha == 1.0) ? 0ull : (alpha == -1.0) ? 1ull << 63 : 1ull;
+}
+
 constexpr int AS_BLOCK = 256;
 
 // out = alpha_c C + A*(w) on the pattern.  Entries that no triple lands on (seven of
@@ -96,7 +100,7 @@ template <typename OT>
 static void assemble_launch(int nnz, const double* c_val, double alpha_c, const int* slot_ptr,
                             const int* slot_tid, const int* con, const double* a, const double* w,
                             OT* out, cudaStream_t stream) {
-  const unsigned long long sgn = (alpha_c == 1.0) ? 0ull : (alpha_c == -1.0) ? 1ull << 63 : 1ull;
+  const unsigned long long sgn = sign_of_scale(alpha_c);
   // four entries per thread once that still fills the GPU twice over
   const int per = (nnz >= 152 * 2048) ? 4 : 1;
   int blocks = (nnz + AS_BLOCK * per - 1) / (AS_BLOCK * per);
@@ -171,6 +175,97 @@ int csr_spmv(int n, long long nnz, const int* rowptr, const int* col, const void
                          (const float*)x, (float*)y);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { set_error("csr_spmv: %s", cudaGetErrorString(e)); return -5; }
+  return 0;
+}
+
+// y = (alpha_c C + A*(w)) x without storing the operator: each entry's value is
+// formed as assemble_kernel forms it (rounded to VT), and the row is summed as
+// csr_spmv_kernel sums it, so the result is that of the two kernels.  One apply
+// then reads the pattern once and writes y, one launch: n = 10^6, 8.1e6 entries,
+// FP32: 81 us (87 as two kernels); n = 800, degree 48, FP64: 16 us a call (37 as two
+// launches and an allocation for the values).  (The Lanczos path applies one operator a hundred
+// times and keeps the assembled values.)
+template <typename VT, int L>
+__global__ void __launch_bounds__(256) fused_apply_kernel(
+    int n, const int* __restrict__ rowptr, const int* __restrict__ col,
+    const double* __restrict__ c_val, double alpha_c, unsigned long long sgn,
+    const int* __restrict__ slot_ptr, const int* __restrict__ slot_tid,
+    const int* __restrict__ con, const double* __restrict__ a, const double* __restrict__ w,
+    const VT* __restrict__ x, VT* __restrict__ y) {
+  const bool has_c = alpha_c != 0.0 && c_val;
+  const int lanes_total = gridDim.x * blockDim.x;
+  const int gid = blockIdx.x * blockDim.x + threadIdx.x;
+  const int lig = gid % L;
+  const int lane = threadIdx.x & 31;
+  const unsigned gmask = (L == 32) ? 0xffffffffu : (((1u << L) - 1u) << (lane & ~(L - 1)));
+  constexpr int U = 2;                             // entries in flight per lane
+  for (int row = gid / L; row < n; row += lanes_total / L) {
+    VT s = (VT)0;
+    const int e = rowptr[row + 1];
+    for (int p0 = rowptr[row] + lig; p0 < e; p0 += U * L) {
+      double v[U];
+      VT xv[U];
+      int b[U], f[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int p = min(p0 + u * L, e - 1);
+        v[u] = has_c ? scaled(alpha_c, sgn, c_val[p]) : 0.0;
+        xv[u] = x[col[p]];
+        b[u] = f[u] = 0;
+        if (w) { b[u] = slot_ptr[p]; f[u] = slot_ptr[p + 1]; }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (p0 + u * L < e) {
+          for (int q = b[u]; q < f[u]; ++q) {
+            const int t = slot_tid[q];
+            v[u] += a[t] * w[con[t]];
+          }
+          s += out_of<VT>(v[u]) * xv[u];
+        }
+    }
+#pragma unroll
+    for (int o = L >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(gmask, s, o, L);
+    if (lig == 0) y[row] = s;
+  }
+}
+
+template <typename VT>
+static void fused_dispatch(int L, int blocks, cudaStream_t st, int n, const int* rp, const int* c,
+                           const double* cv, double alpha, unsigned long long sgn, const int* sp,
+                           const int* sid, const int* con, const double* a, const double* w,
+                           const VT* x, VT* y) {
+  auto go = [&](auto kern) {
+    kern<<<blocks, 256, 0, st>>>(n, rp, c, cv, alpha, sgn, sp, sid, con, a, w, x, y);
+  };
+  switch (L) {
+    case 1: go(fused_apply_kernel<VT, 1>); break;
+    case 2: go(fused_apply_kernel<VT, 2>); break;
+    case 4: go(fused_apply_kernel<VT, 4>); break;
+    case 8: go(fused_apply_kernel<VT, 8>); break;
+    case 16: go(fused_apply_kernel<VT, 16>); break;
+    default: go(fused_apply_kernel<VT, 32>); break;
+  }
+}
+
+int fused_apply(int n, long long nnz, const int* rowptr, const int* col, const double* c_val,
+                double alpha_c, const int* slot_ptr, const int* slot_tid, const int* con,
+                const double* a, const double* w, const void* x, void* y, int prec, int sm_count,
+                cudaStream_t stream) {
+  if (n <= 0) return 0;
+  const int L = lanczos_lanes(n, nnz);
+  const unsigned long long sgn = sign_of_scale(alpha_c);
+  const long long need = ((long long)n * L + 255) / 256;
+  int blocks = (int)(need < (long long)sm_count * 32 ? need : (long long)sm_count * 32);
+  if (blocks < 1) blocks = 1;
+  if (prec == 64)
+    fused_dispatch<double>(L, blocks, stream, n, rowptr, col, c_val, alpha_c, sgn, slot_ptr,
+                           slot_tid, con, a, w, (const double*)x, (double*)y);
+  else
+    fused_dispatch<float>(L, blocks, stream, n, rowptr, col, c_val, alpha_c, sgn, slot_ptr,
+                          slot_tid, con, a, w, (const float*)x, (float*)y);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) { set_error("fused_apply: %s", cudaGetErrorString(e)); return -5; }
   return 0;
 }
 
@@ -397,7 +492,7 @@ int apply_A_operator(int m, const int* con_ptr, const int* t_row, const int* t_c
 // sums: 32 accumulators, then pairwise.  Rows of at most AO_SHORT triples (one in
 // MaxCut) take one thread for all columns, longer ones (the QAP's hold about 900,
 // the lifted row several thousand) one warp per column, because a warp gets one
-// FP64 instruction per 60 cycles; four triples' loads in flight per lane.
+// FP64 instruction per 60 cycles; eight triples' loads in flight per lane.
 __global__ void __launch_bounds__(256) A_adjoint_kernel(
     int n, const int* __restrict__ row_ptr, const int* __restrict__ r_con,
     const int* __restrict__ r_col, const double* __restrict__ r_a, const double* __restrict__ z,
@@ -419,17 +514,17 @@ __global__ void __launch_bounds__(256) A_adjoint_kernel(
       const int tb = __shfl_sync(0xffffffffu, b, src), te = __shfl_sync(0xffffffffu, e, src);
       const double* Uq = U + (size_t)q * ldu;
       double s = 0.0;
-      for (int t = tb + lane; t < te; t += 128) {
-        double av[4], zv[4], uv[4];
+      for (int t = tb + lane; t < te; t += 256) {
+        double av[8], zv[8], uv[8];
 #pragma unroll
-        for (int h = 0; h < 4; ++h) {
+        for (int h = 0; h < 8; ++h) {
           const int th = min(t + 32 * h, te - 1);
           av[h] = r_a[th];
           zv[h] = z[r_con[th]];
           uv[h] = Uq[r_col[th]];
         }
 #pragma unroll
-        for (int h = 0; h < 4; ++h)
+        for (int h = 0; h < 8; ++h)
           if (t + 32 * h < te) s += av[h] * zv[h] * uv[h];
       }
       s = warp_sum(s);

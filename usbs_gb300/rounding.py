@@ -23,11 +23,17 @@ import scipy.sparse as sp
 from . import _lib
 
 
+_checked_torch = None      # torch, once a CUDA device has been seen
+
+
 def _torch():
-    import torch
-    if not torch.cuda.is_available():
-        raise RuntimeError("usbs_gb300.rounding needs a CUDA device (GB300); none is visible")
-    return torch
+    global _checked_torch
+    if _checked_torch is None:
+        import torch
+        if not torch.cuda.is_available():
+            raise RuntimeError("usbs_gb300.rounding needs a CUDA device (GB300); none is visible")
+        _checked_torch = torch
+    return _checked_torch
 
 
 class DeviceCSR:
