@@ -1470,6 +1470,362 @@ __global__ void __launch_bounds__(LZ_BLOCK) st_rotate_kernel(const __grid_consta
   }
 }
 
+// ---------------------------------------------------------------- wave path
+// A team-size problem (too large for one cluster, x of at most 160 KB) that has
+// the GPU's launches to itself runs the team kernel's arithmetic as four
+// ordinary launches per Lanczos step, like the stream path:
+//   A1  y = Op x, Q[:, i] = x
+//   A2  partial h1 = Q^T y
+//   B   q1 = y - Q h1, partial h2 = Q^T q1
+//   C   q2 = q1 - Q h2, partial ||q2||^2, the step's state
+// Every sum is the team kernel's: rank r of its R CTAs owns up to four 256-row
+// tiles, thread t accumulates a column over row t of each in turn, and the R
+// partial sums of a column are added by lanes r, r + 32, ... and a butterfly.  Here
+// a rank is four CTAs (a cluster in B and C).  CTA j takes the rows of tile j for
+// the updates, and columns j, j + 4, ... of the dots over all four tiles (their
+// vector, in B, from the other CTAs' shared memory).  So four times as many
+// SMs work, a step has four kernel boundaries where the team kernel has three
+// grid barriers of about 20k cycles, and the results are the same bits.
+// ER n = 30,011 of degree 12, FP32, 10 restarts: 14.4 ms per call as one
+// cooperative launch of 30 CTAs, 5.3 with A1 and A2 as one kernel.
+constexpr int WV_C = 4;                  // CTAs (tiles) per rank
+constexpr int WV_U = 8;                  // columns per CTA: c = j + 4 u
+
+struct WvPlace { int rank, j, tile, t0, nt; };
+template <typename VT>
+__device__ __forceinline__ WvPlace wv_place(const TeamDesc<VT>& P) {
+  WvPlace w;
+  const int ntiles = (P.n + LZ_BLOCK - 1) / LZ_BLOCK;
+  w.rank = blockIdx.x / WV_C;
+  w.j = blockIdx.x % WV_C;               // (its rank in the cluster, where there is one)
+  w.t0 = (int)((long long)ntiles * w.rank / P.nctas);
+  w.nt = (int)((long long)ntiles * (w.rank + 1) / P.nctas) - w.t0;
+  w.tile = w.t0 + w.j;
+  return w;
+}
+
+template <typename VT>
+struct WvShared {
+  union {
+    struct {
+      double ys[LZ_BLOCK];
+      double wred[LZ_NW][MP1];
+    } st;
+  } u;
+  double h[MP1];
+  __align__(16) VT hv[MP1 + 3];
+  VT xv[LZ_BLOCK];                       // the tile's vector, read by the rank's other CTAs
+  int last;
+};
+
+// sh.h[c], sh.hv[c] = sum over the R ranks of part[c][r], c < nv <= 32: warp w
+// takes columns 4 w .. 4 w + 3
+template <typename VT>
+__device__ __forceinline__ void wv_reduce(const double* part, int R, int nv, WvShared<VT>& sh) {
+  const int lane = threadIdx.x & 31, c0 = 4 * (threadIdx.x >> 5);
+  if (c0 < nv) {
+    double a[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) a[u] = 0.0;
+    for (int r = lane; r < R; r += 32)
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (c0 + u < nv) a[u] += __ldcg(part + (size_t)(c0 + u) * R + r);
+#pragma unroll
+    for (int h = 16, w = 2; w >= 1; h >>= 1, w >>= 1) {
+      const bool up = (lane & h) != 0;
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+        if (u < w) {
+          const double send = up ? a[u] : a[u + w], keep = up ? a[u + w] : a[u];
+          a[u] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+        }
+    }
+    double v = a[0];
+#pragma unroll
+    for (int h = 4; h >= 1; h >>= 1) v += __shfl_xor_sync(0xffffffffu, v, h);
+    const int c = c0 + (lane >> 3);
+    if ((lane & 7) == 0 && c < nv) { sh.h[c] = v; sh.hv[c] = (VT)v; }
+  }
+  __syncthreads();
+}
+
+// this CTA's columns of the rank's rows (0 past nv or the last row)
+template <typename VT>
+__device__ __forceinline__ void wv_load(const TeamDesc<VT>& P, const WvPlace& w, int nv,
+                                        VT (&q)[WV_C][WV_U]) {
+#pragma unroll
+  for (int t = 0; t < WV_C; ++t) {
+    const int row = (w.t0 + t) * LZ_BLOCK + threadIdx.x;
+    const bool in = t < w.nt && row < P.n;
+#pragma unroll
+    for (int u = 0; u < WV_U; ++u) {
+      const int c = w.j + WV_C * u;
+      q[t][u] = (in && c < nv) ? __ldg(P.Q + (size_t)c * P.ld + row) : (VT)0;
+    }
+  }
+}
+
+// partial dots of the CTA's columns with the rank's vector y
+template <typename VT>
+__device__ __forceinline__ void wv_dots(const TeamDesc<VT>& P, const WvPlace& w, WvShared<VT>& sh,
+                                        int nv, const VT (&q)[WV_C][WV_U], const VT (&y)[WV_C],
+                                        double* part) {
+  typedef typename Acc<VT>::type AT;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  AT acc[WV_U];
+#pragma unroll
+  for (int u = 0; u < WV_U; ++u) acc[u] = (AT)0;
+#pragma unroll
+  for (int t = 0; t < WV_C; ++t)
+    if (t < w.nt && (w.t0 + t) * LZ_BLOCK + tid < P.n) {
+#pragma unroll
+      for (int u = 0; u < WV_U; ++u)
+        if (w.j + WV_C * u < nv) acc[u] += (AT)q[t][u] * (AT)y[t];
+    }
+#pragma unroll
+  for (int h = 16, x = WV_U / 2; x >= 1; h >>= 1, x >>= 1) {
+    const bool up = (lane & h) != 0;
+#pragma unroll
+    for (int u = 0; u < WV_U / 2; ++u)
+      if (u < x) {
+        const AT send = up ? acc[u] : acc[u + x], keep = up ? acc[u + x] : acc[u];
+        acc[u] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+      }
+  }
+  AT v = acc[0];
+#pragma unroll
+  for (int h = 2; h >= 1; h >>= 1) v += __shfl_xor_sync(0xffffffffu, v, h);
+  if ((lane & 3) == 0) sh.u.st.wred[wid][lane >> 2] = (double)v;
+  __syncthreads();
+  const int c = w.j + WV_C * tid;
+  if (tid < WV_U && c < nv) {
+    double s = 0.0;
+#pragma unroll
+    for (int k = 0; k < LZ_NW; ++k) s += sh.u.st.wred[k][tid];
+    part[(size_t)c * P.nctas + w.rank] = s;
+  }
+}
+
+// the thread's row of its tile: its vector entry and basis row, loaded before h is
+// known, then x - sum_{c < nv} Q[row, c] h[c]
+template <typename VT>
+struct WvRow {
+  VT x, q[MAXM];
+  __device__ __forceinline__ void load(const TeamDesc<VT>& P, int row, bool in, int nv,
+                                       const VT* v) {
+    x = in ? __ldcg(v + row) : (VT)0;
+#pragma unroll
+    for (int c = 0; c < MAXM; ++c)
+      q[c] = (in && c < nv) ? __ldg(P.Q + (size_t)c * P.ld + row) : (VT)0;
+  }
+  __device__ __forceinline__ VT update(const WvShared<VT>& sh, int nv) const {
+    VT s = (VT)0;
+#pragma unroll
+    for (int c = 0; c < MAXM; ++c)
+      if (c < nv) s += q[c] * sh.hv[c];
+    return x - s;
+  }
+};
+
+// A1, 64 rows per CTA, L lanes per row (spmv_tile's sums).  Breakdown
+// (solver/lanczos.py:107-117): the replacement vector in y's place.
+constexpr int WV_ROWS = 64;
+template <typename VT, int L>
+__device__ __forceinline__ void wv_spmv_rows(const TeamDesc<VT>& P, const VT* x, VT xscale, VT* v) {
+  typedef typename Acc<VT>::type AT;
+  constexpr int GPP = LZ_BLOCK / L, NP = (WV_ROWS + GPP - 1) / GPP;
+  const int g = threadIdx.x / L, lig = threadIdx.x - (threadIdx.x / L) * L;
+  const int base = blockIdx.x * WV_ROWS;
+  int pb[NP], pe[NP], c0[NP];
+  VT v0[NP], x0[NP];
+#pragma unroll
+  for (int q = 0; q < NP; ++q) {
+    const int lr = q * GPP + g;
+    pb[q] = pe[q] = 0;
+    if (lr < WV_ROWS && base + lr < P.n) {
+      pb[q] = __ldg(P.rowptr + base + lr) + lig;
+      pe[q] = __ldg(P.rowptr + base + lr + 1);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < NP; ++q) {
+    c0[q] = 0;
+    v0[q] = (VT)0;
+    if (pb[q] < pe[q]) { c0[q] = __ldg(P.col + pb[q]); v0[q] = __ldg(P.val + pb[q]); }
+  }
+#pragma unroll
+  for (int q = 0; q < NP; ++q) x0[q] = __ldg(x + c0[q]);
+#pragma unroll
+  for (int q = 0; q < NP; ++q) {
+    AT s = (AT)v0[q] * (AT)x0[q];
+    for (int p = pb[q] + L; p < pe[q]; p += L)
+      s += (AT)__ldg(P.val + p) * (AT)__ldg(x + __ldg(P.col + p));
+#pragma unroll
+    for (int o = L >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    const int lr = q * GPP + g;
+    if (lig == 0 && lr < WV_ROWS && base + lr < P.n) v[base + lr] = (VT)s * xscale;
+  }
+}
+template <typename VT>
+__global__ void __launch_bounds__(LZ_BLOCK) wv_spmv_kernel(const __grid_constant__ TeamDesc<VT> P,
+                                                           StreamCtl* ctl) {
+  st_pdl_prologue();
+  int i, nv, buf;
+  const int mode = st_mode(ctl, P.m, &i, &nv, &buf);
+  if (mode == SM_SKIP) return;
+  const size_t ld = (size_t)P.ld;
+  const int row = blockIdx.x * WV_ROWS + threadIdx.x;
+  const bool own = threadIdx.x < WV_ROWS && row < P.n;
+  VT* v = P.vbuf + (size_t)buf * ld;
+  if (mode == SM_BREAKDOWN) {
+    if (own) v[row] = (VT)hash_normal((uint64_t)i, (uint64_t)row);
+    return;
+  }
+  const int k = __ldg(&ctl->k);
+  const bool wq = i > k;
+  const VT* x = wq ? P.vbuf + (size_t)(buf ^ 1) * ld : P.Q + (size_t)k * ld;
+  const VT xscale = wq ? (VT)__ldg(&ctl->invb) : (VT)1;
+  if (wq && own) P.Q[(size_t)i * ld + row] = __ldg(x + row) * xscale;
+  switch (P.lanes) {
+    case 1: wv_spmv_rows<VT, 1>(P, x, xscale, v); break;
+    case 2: wv_spmv_rows<VT, 2>(P, x, xscale, v); break;
+    case 4: wv_spmv_rows<VT, 4>(P, x, xscale, v); break;
+    case 8: wv_spmv_rows<VT, 8>(P, x, xscale, v); break;
+    case 16: wv_spmv_rows<VT, 16>(P, x, xscale, v); break;
+    default: wv_spmv_rows<VT, 32>(P, x, xscale, v); break;
+  }
+}
+
+// A2
+template <typename VT>
+__global__ void __launch_bounds__(LZ_BLOCK) wv_dot_kernel(const __grid_constant__ TeamDesc<VT> P,
+                                                          StreamCtl* ctl) {
+  st_pdl_prologue();
+  __shared__ WvShared<VT> sh;
+  int i, nv, buf;
+  if (st_mode(ctl, P.m, &i, &nv, &buf) == SM_SKIP) return;
+  const WvPlace w = wv_place(P);
+  const VT* v = P.vbuf + (size_t)buf * P.ld;
+  VT q[WV_C][WV_U], y[WV_C];
+  wv_load(P, w, nv, q);
+#pragma unroll
+  for (int t = 0; t < WV_C; ++t) {
+    const int row = (w.t0 + t) * LZ_BLOCK + threadIdx.x;
+    y[t] = (t < w.nt && row < P.n) ? __ldg(v + row) : (VT)0;
+  }
+  wv_dots(P, w, sh, nv, q, y, P.part);
+}
+
+// B
+template <typename VT>
+__global__ void __launch_bounds__(LZ_BLOCK) wv_update_dot_kernel(
+    const __grid_constant__ TeamDesc<VT> P, StreamCtl* ctl) {
+  st_pdl_prologue();
+  __shared__ WvShared<VT> sh;
+  int i, nv, buf;
+  if (st_mode(ctl, P.m, &i, &nv, &buf) == SM_SKIP) return;
+  const WvPlace w = wv_place(P);
+  const int tid = threadIdx.x, row = w.tile * LZ_BLOCK + tid;
+  const bool in = w.j < w.nt && row < P.n;
+  VT* v = P.vbuf + (size_t)buf * P.ld;
+  WvRow<VT> r;
+  r.load(P, row, in, nv, v);
+  wv_reduce(P.part, P.nctas, nv, sh);
+  if (blockIdx.x == 0 && tid < nv) ctl->h1[tid] = sh.h[tid];
+  if (in) {
+    const VT x = r.update(sh, nv);
+    v[row] = x;
+    sh.xv[tid] = x;
+  }
+  VT q[WV_C][WV_U], y[WV_C];
+  wv_load(P, w, nv, q);
+  cl_sync();
+#pragma unroll
+  for (int t = 0; t < WV_C; ++t) {
+    y[t] = (VT)0;
+    if (t < w.nt) y[t] = cl_ld(cl_map(&sh.xv[tid], (unsigned)t), (VT)0);
+  }
+  wv_dots(P, w, sh, nv, q, y, P.part + (size_t)MP1 * P.nctas);
+  cl_sync();       // no CTA leaves while another reads its vector
+}
+
+// C; the last rank to finish advances the state (solver/lanczos.py:95-105, and the
+// breakdown test of :107)
+template <typename VT>
+__global__ void __launch_bounds__(LZ_BLOCK) wv_update_norm_kernel(
+    const __grid_constant__ TeamDesc<VT> P, StreamCtl* ctl) {
+  st_pdl_prologue();
+  typedef typename Acc<VT>::type AT;
+  __shared__ WvShared<VT> sh;
+  int i, nv, buf;
+  const int mode = st_mode(ctl, P.m, &i, &nv, &buf);
+  if (mode == SM_SKIP) return;
+  const WvPlace w = wv_place(P);
+  const int tid = threadIdx.x, lane = tid & 31, row = w.tile * LZ_BLOCK + tid, R = P.nctas;
+  const bool in = w.j < w.nt && row < P.n;
+  VT* v = P.vbuf + (size_t)buf * P.ld;
+  WvRow<VT> r;
+  r.load(P, row, in, nv, v);
+  wv_reduce(P.part + (size_t)MP1 * R, R, nv, sh);
+  if (in) {
+    const VT x = r.update(sh, nv);
+    v[row] = x;
+    sh.xv[tid] = x;
+  }
+  cl_sync();
+  AT nrm = (AT)0;
+  if (w.j == 0) {
+#pragma unroll
+    for (int t = 0; t < WV_C; ++t)
+      if (t < w.nt && (w.t0 + t) * LZ_BLOCK + tid < P.n) {
+        const VT x = cl_ld(cl_map(&sh.xv[tid], (unsigned)t), (VT)0);
+        nrm += (AT)x * (AT)x;
+      }
+  }
+  cl_sync();
+  if (w.j != 0) return;
+  nrm = warp_sum(nrm);
+  if (lane == 0) sh.u.st.wred[tid >> 5][0] = (double)nrm;
+  __syncthreads();
+  double* part = P.part + (size_t)2 * MP1 * R;
+  if (tid == 0) {
+    double s = 0.0;
+#pragma unroll
+    for (int k = 0; k < LZ_NW; ++k) s += sh.u.st.wred[k][0];
+    part[w.rank] = s;
+    __threadfence();
+    sh.last = (atomicAdd(&ctl->ticket[2], 1u) == (unsigned)R - 1u) ? 1 : 0;
+    if (sh.last) __threadfence();
+  }
+  __syncthreads();
+  if (!sh.last || tid >= 32) return;
+  double a = 0.0;
+  for (int r = lane; r < R; r += 32) a += __ldcg(part + r);
+  a = warp_sum(a);
+  if (lane == 0) {
+    const double b = sqrt(a);
+    if (mode == SM_STEP) {
+      ctl->alpha[i] = __ldcg(&ctl->h1[i]) + sh.h[i];
+      ctl->beta[i] = b;
+      ctl->steps += 1;
+      ctl->sum_nv += i + 1;
+      ctl->cur = buf ^ 1;
+      ctl->i = i + 1;
+      if (b < 1e-15) {
+        ctl->bd = 1;
+        ctl->breakdowns += 1;
+      } else {
+        ctl->invb = 1.0 / b;
+      }
+    } else {
+      ctl->invb = 1.0 / b;
+      ctl->bd = 0;
+    }
+    ctl->ticket[2] = 0u;
+  }
+}
+
 // ---------------------------------------------------------------- cluster path
 // A problem of at most CL_MAX_CTAS x rc rows runs as one thread-block cluster.
 // CTA r of the cluster owns rows [r rc, (r+1) rc) and keeps, for the whole
@@ -2429,7 +2785,21 @@ int lanczos_stream_occupancy(int prec) {
   return b;
 }
 
-// Stream path of one problem.  The host enqueues a cycle's steps (m - i of
+// Whether a problem runs on the wave path: a team-size problem whose ranks hold at
+// most four tiles, outside a stream capture (the loop state is read back once per
+// restart).
+template <typename VT>
+static bool wave_fits(const LanczosProblem& p, int nctas, cudaStream_t stream) {
+  if (p.m > MAXM || p.m < 1 || p.n < 1 || p.ld < p.n) return false;
+  const int tiles = (p.n + LZ_BLOCK - 1) / LZ_BLOCK;
+  if (nctas < 1 || (tiles + nctas - 1) / nctas > WV_C) return false;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &cs) != cudaSuccess) { cudaGetLastError(); return false; }
+  return cs == cudaStreamCaptureStatusNone;
+}
+
+// Stream path of one problem (wave = 0), or its wave path over `wave` ranks.  The
+// host enqueues a cycle's steps (m - i of
 // them, one more after a breakdown), the restart and the rotation, then reads
 // the control block back once (a synchronisation of `stream`) to learn where
 // the next cycle starts and whether the loop has ended.  The loop state is
@@ -2437,23 +2807,28 @@ int lanczos_stream_occupancy(int prec) {
 // a stream kernel launched with programmatic stream serialisation (see
 // st_pdl_prologue)
 template <typename... KArgs, typename... Args>
-static cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, size_t smem,
+static cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int cluster, size_t smem,
                               cudaStream_t stream, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3(LZ_BLOCK);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = (unsigned)cluster;
+  at[1].val.clusterDim.y = 1;
+  at[1].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 template <typename VT>
-static int run_stream(const DeviceInfo& di, const LanczosProblem& p, cudaStream_t stream) {
+static int run_stream(const DeviceInfo& di, const LanczosProblem& p, cudaStream_t stream,
+                      int wave = 0) {
   if (p.m > MAXM || p.m < 1 || p.n < 1 || p.ld < p.n) {
     set_error("lanczos: unsupported sizes n=%d ld=%d m=%d (m must be in [1, %d])", p.n, p.ld,
               p.m, MAXM);
@@ -2466,7 +2841,8 @@ static int run_stream(const DeviceInfo& di, const LanczosProblem& p, cudaStream_
     return -2;
   }
   const int ntiles = (p.n + LZ_BLOCK - 1) / LZ_BLOCK;
-  const int G = lanczos_team_size(di, p.n, sizeof(VT) == 8 ? 64 : 32, true);   // partials per pass
+  // partials per pass
+  const int G = wave ? wave : lanczos_team_size(di, p.n, sizeof(VT) == 8 ? 64 : 32, true);
   const int* occ = stream_occ<VT>();
   // each kernel: at most one wave, and every CTA the same number of row
   // chunks (A2 and C use 4 rows per thread, B 8 bytes per thread), so no
@@ -2476,7 +2852,7 @@ static int run_stream(const DeviceInfo& di, const LanczosProblem& p, cudaStream_
     const int rows = (j == 1) ? (8 / (int)sizeof(VT)) * LZ_BLOCK : (j == 3 ? LZ_BLOCK : ST_ROWS);
     const int nch = (p.n + rows - 1) / rows;
     int gmax = di.sm_count * occ[j];
-    if (gmax > G) gmax = G;
+    if (gmax > G && !wave) gmax = G;
     if (gmax < 1) gmax = 1;
     const int per = (nch + gmax - 1) / gmax;
     g[j] = (nch + per - 1) / per;
@@ -2498,21 +2874,23 @@ static int run_stream(const DeviceInfo& di, const LanczosProblem& p, cudaStream_
   t.Ybuf = (double*)w; w += align256((size_t)MAXM * MAXM * sizeof(double));
   t.bar = nullptr;
   w += 256;
-  const int ns = (p.n + 31) / 32;
-  t.wcap = sell_wcap(p.n, p.nnz);
-  if ((long long)ns * 32 * t.wcap > 0x7fffffffLL) {
-    set_error("lanczos: n=%d is too large for the stream path's operator layout", p.n);
-    return -2;
-  }
-  t.sl_ptr = (int*)w; w += align256((size_t)(ns + 1) * sizeof(int));
-  t.sl_row = (unsigned char*)w; w += align256((size_t)ns * 32);
-  t.sl_col = (int*)w; w += align256((size_t)ns * 32 * t.wcap * sizeof(int));
-  t.sl_val = (VT*)w;
   t.alpha = p.alpha; t.beta = p.beta; t.ctl = p.ctl; t.status = p.status;
-  st_sell_order_kernel<VT><<<ntiles, LZ_BLOCK, 0, stream>>>(t);
-  st_sell_scan_kernel<<<1, 1024, 0, stream>>>(ns, t.sl_ptr);
-  st_sell_fill_kernel<VT><<<ntiles, LZ_BLOCK, 0, stream>>>(t);
-  t_launches += 3;
+  if (!wave) {
+    const int ns = (p.n + 31) / 32;
+    t.wcap = sell_wcap(p.n, p.nnz);
+    if ((long long)ns * 32 * t.wcap > 0x7fffffffLL) {
+      set_error("lanczos: n=%d is too large for the stream path's operator layout", p.n);
+      return -2;
+    }
+    t.sl_ptr = (int*)w; w += align256((size_t)(ns + 1) * sizeof(int));
+    t.sl_row = (unsigned char*)w; w += align256((size_t)ns * 32);
+    t.sl_col = (int*)w; w += align256((size_t)ns * 32 * t.wcap * sizeof(int));
+    t.sl_val = (VT*)w;
+    st_sell_order_kernel<VT><<<ntiles, LZ_BLOCK, 0, stream>>>(t);
+    st_sell_scan_kernel<<<1, 1024, 0, stream>>>(ns, t.sl_ptr);
+    st_sell_fill_kernel<VT><<<ntiles, LZ_BLOCK, 0, stream>>>(t);
+    t_launches += 3;
+  }
   if (cudaMemsetAsync(ctl, 0, sizeof(StreamCtl), stream) != cudaSuccess ||
       cudaMemsetAsync(p.ctl, 0, 16 * sizeof(int), stream) != cudaSuccess) {
     set_error("lanczos: memset failed");
@@ -2529,14 +2907,26 @@ static int run_stream(const DeviceInfo& di, const LanczosProblem& p, cudaStream_
     const int slots = (p.m - i_host) + (bd_host ? 1 : 0);
     cudaError_t e = cudaSuccess;
     for (int j = 0; j < slots && e == cudaSuccess; ++j) {
-      e = launch_pdl(st_sell_spmv_kernel<VT>, ntiles, 0, stream, t, ctl);
-      if (e == cudaSuccess) e = launch_pdl(st_dot_kernel<VT>, g[0], st_sacc_bytes<VT>(), stream, t, ctl);
+      if (wave) {
+        e = launch_pdl(wv_spmv_kernel<VT>, (p.n + WV_ROWS - 1) / WV_ROWS, 1, 0, stream, t, ctl);
+        if (e == cudaSuccess)
+          e = launch_pdl(wv_dot_kernel<VT>, WV_C * wave, 1, 0, stream, t, ctl);
+        if (e == cudaSuccess)
+          e = launch_pdl(wv_update_dot_kernel<VT>, WV_C * wave, WV_C, 0, stream, t, ctl);
+        if (e == cudaSuccess)
+          e = launch_pdl(wv_update_norm_kernel<VT>, WV_C * wave, WV_C, 0, stream, t, ctl);
+        continue;
+      }
+      e = launch_pdl(st_sell_spmv_kernel<VT>, ntiles, 1, 0, stream, t, ctl);
       if (e == cudaSuccess)
-        e = launch_pdl(st_update_dot1_kernel<VT>, g[1], st_sacc_bytes<VT>(), stream, t, ctl);
-      if (e == cudaSuccess) e = launch_pdl(st_update_norm_kernel<VT>, g[2], 0, stream, t, ctl);
+        e = launch_pdl(st_dot_kernel<VT>, g[0], 1, st_sacc_bytes<VT>(), stream, t, ctl);
+      if (e == cudaSuccess)
+        e = launch_pdl(st_update_dot1_kernel<VT>, g[1], 1, st_sacc_bytes<VT>(), stream, t, ctl);
+      if (e == cudaSuccess)
+        e = launch_pdl(st_update_norm_kernel<VT>, g[2], 1, 0, stream, t, ctl);
     }
-    if (e == cudaSuccess) e = launch_pdl(st_restart_kernel<VT>, 1, 0, stream, t, ctl);
-    if (e == cudaSuccess) e = launch_pdl(st_rotate_kernel<VT>, g[3], 0, stream, t, ctl);
+    if (e == cudaSuccess) e = launch_pdl(st_restart_kernel<VT>, 1, 1, 0, stream, t, ctl);
+    if (e == cudaSuccess) e = launch_pdl(st_rotate_kernel<VT>, g[3], 1, 0, stream, t, ctl);
     t_launches += 4 * slots + 2;
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) {
@@ -2575,6 +2965,26 @@ static int run_noncluster(const DeviceInfo& di, const LanczosProblem* probs, int
       }
     }
     if (nt) {
+      // a few team-size problems: one after another on the wave path (2.7 against
+      // 14 ms for one at n = 30,000), with the team sizes, and so the results, of
+      // the shared launch, which would run four in about 14 ms; more, or teams
+      // shrunk to fit one launch, share it
+      const int occ = (sizeof(VT) == 8) ? di.lanczos_occ64 : di.lanczos_occ32;
+      const int maxc = (di.sm_count > 4 ? di.sm_count - 2 : di.sm_count) * (occ > 0 ? occ : 1);
+      int want[MAX_TEAMS], total = 0;
+      bool wave = nt <= 4;
+      for (int i = 0; i < nt; ++i) {
+        want[i] = lanczos_team_size(di, team[i].n, sizeof(VT) == 8 ? 64 : 32);
+        total += want[i];
+        wave = wave && wave_fits<VT>(team[i], want[i], stream);
+      }
+      if (wave && total <= maxc) {
+        for (int i = 0; i < nt; ++i) {
+          const int rc = run_stream<VT>(di, team[i], stream, want[i]);
+          if (rc) return rc;
+        }
+        continue;
+      }
       const int rc = run_typed<VT>(di, team, nt, stream);
       if (rc) return rc;
     }
