@@ -851,7 +851,8 @@ struct __align__(16) StreamCtl {
   int i, k, bd, cur;           // step, saved vectors, breakdown pending, work vector in use
   int stop, rot, stepped;      // loop ended; rotation pending; the finished cycle had steps
   int restarts, breakdowns, steps, sum_nv, sum_kn, nconv;
-  unsigned ticket[4];          // last-CTA tickets of A2, B, C and the rotation
+  unsigned ticket[4];          // last-CTA tickets of (unused), B, C and the rotation
+  unsigned dticket[4];         // of A2's column groups
   double invb;                 // 1 / beta of the latest unnormalised vector
   double h1[MP1], h2[MP1];
   double alpha[MAXM], beta[MAXM];
@@ -1032,29 +1033,6 @@ __device__ __forceinline__ Row4<VT> st_combine(const VT* Q, size_t ld, int r4, i
   return s;
 }
 
-// sacc[c][tid] += sum_j Q[r4 + j, c] * x.v[j], c < nv (a per-thread column of
-// shared memory), st_batch() loads in flight at a time
-template <typename VT, typename AT>
-__device__ __forceinline__ void st_dots(const VT* Q, size_t ld, int r4, int n, int nv,
-                                        const Row4<VT>& x, AT* sacc) {
-  constexpr int NB = st_batch<VT>();
-#pragma unroll 1
-  for (int c0 = 0; c0 < nv; c0 += NB) {
-    Row4<VT> q[NB];
-#pragma unroll
-    for (int b = 0; b < NB; ++b)
-      if (c0 + b < nv) q[b] = ld4(Q + (size_t)(c0 + b) * ld, r4, n);
-#pragma unroll
-    for (int b = 0; b < NB; ++b)
-      if (c0 + b < nv) {
-        AT d = (AT)0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) d += (AT)q[b].v[j] * (AT)x.v[j];
-        sacc[(c0 + b) * LZ_BLOCK + threadIdx.x] += d;
-      }
-  }
-}
-
 // out[c * R] = sum over the CTA's threads of sacc[c][t], c < nv: warp w takes
 // columns w, w + 8, ...; lane l sums threads l, l + 32, ... in order
 template <typename AT>
@@ -1070,7 +1048,7 @@ __device__ __forceinline__ void st_block_cols(const AT* sacc, int nv, double* ou
   }
 }
 
-// the per-thread dot accumulators of A2 and B (dynamic shared memory)
+// the threads' dot accumulators of B (dynamic shared memory, for their sums)
 template <typename VT>
 constexpr size_t st_sacc_bytes() {
   return (size_t)MP1 * LZ_BLOCK * sizeof(typename Acc<VT>::type);
@@ -1230,32 +1208,97 @@ __global__ void __launch_bounds__(LZ_BLOCK, 8) st_sell_spmv_kernel(
   }
 }
 
-// A2: h1[c] = Q[:, c] . v for c < nv (v = the step's y, or the breakdown vector)
+// A2: h1[c] = Q[:, c] . v for c < nv (v = the step's y, or the breakdown vector).
+// The grid is DOT_G x R: the R row blocks of the partial sums, each shared by DOT_G
+// CTAs that take columns g, g + DOT_G, ...  One CTA per row block left SMs with
+// three or four of them (489 blocks at n = 10^6) and one CTA to add all columns'
+// partials at the end; a group's last CTA adds its own columns.
+constexpr int DOT_G = 4, DOT_U = MAXM / DOT_G;
 template <typename VT>
 __global__ void __launch_bounds__(LZ_BLOCK) st_dot_kernel(const __grid_constant__ TeamDesc<VT> P,
                                                            StreamCtl* ctl) {
   st_pdl_prologue();
   typedef typename Acc<VT>::type AT;
   __shared__ StShared<VT> sh;
+  __shared__ AT sacc[DOT_U * LZ_BLOCK];
   int i, nv, buf;
   if (st_mode(ctl, P.m, &i, &nv, &buf) == SM_SKIP) return;
-  const int R = gridDim.x;
+  const int R = gridDim.x / DOT_G, g = blockIdx.x % DOT_G, rb = blockIdx.x / DOT_G;
+  const int mine = (nv - g + DOT_G - 1) / DOT_G;            // columns g, g + DOT_G, ... < nv
+  if (mine <= 0) return;
   const size_t ld = (size_t)P.ld;
-  int c0, c1;
-  st_chunks(P.n, &c0, &c1);
+  const int nch = (P.n + ST_ROWS - 1) / ST_ROWS;
+  const int c0 = (int)((long long)nch * rb / R), c1 = (int)((long long)nch * (rb + 1) / R);
   const VT* v = P.vbuf + (size_t)buf * ld;
-  extern __shared__ __align__(16) unsigned char st_dyn[];
-  AT* sacc = (AT*)st_dyn;
-  for (int c = 0; c < nv; ++c) sacc[c * LZ_BLOCK + threadIdx.x] = (AT)0;
+  AT acc[DOT_U];
+#pragma unroll
+  for (int u = 0; u < DOT_U; ++u) acc[u] = (AT)0;
   for (int ch = c0; ch < c1; ++ch) {
     const int r4 = ch * ST_ROWS + 4 * threadIdx.x;
-    if (r4 < P.n) st_dots(P.Q, ld, r4, P.n, nv, ld4<VT, false>(v, r4, P.n), sacc);
+    if (r4 < P.n) {
+      constexpr int B = st_batch<VT>();
+#pragma unroll
+      for (int u0 = 0; u0 < DOT_U; u0 += B) {
+        if (u0 < mine) {
+          Row4<VT> q[B];
+#pragma unroll
+          for (int u = 0; u < B; ++u)
+            if (u0 + u < mine) q[u] = ld4(P.Q + (size_t)(g + DOT_G * (u0 + u)) * ld, r4, P.n);
+          const Row4<VT> x = ld4<VT, false>(v, r4, P.n);
+#pragma unroll
+          for (int u = 0; u < B; ++u)
+            if (u0 + u < mine) {
+              AT d = (AT)0;
+#pragma unroll
+              for (int j = 0; j < 4; ++j) d += (AT)q[u].v[j] * (AT)x.v[j];
+              acc[u0 + u] += d;
+            }
+        }
+      }
+    }
   }
-  st_block_cols(sacc, nv, P.part + blockIdx.x, R);
-  if (!st_last_cta(&ctl->ticket[0], sh)) return;
-  st_reduce<VT>(P.part, R, nv, sh);
-  for (int c = threadIdx.x; c < nv; c += LZ_BLOCK) ctl->h1[c] = sh.h[c];
-  if (threadIdx.x == 0) ctl->ticket[0] = 0u;
+#pragma unroll
+  for (int u = 0; u < DOT_U; ++u)
+    if (u < mine) sacc[u * LZ_BLOCK + threadIdx.x] = acc[u];
+  __syncthreads();
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (w < mine) {                                            // one column per warp
+    AT s = (AT)0;
+#pragma unroll
+    for (int k = 0; k < LZ_BLOCK / 32; ++k) s += sacc[w * LZ_BLOCK + lane + 32 * k];
+    s = warp_sum(s);
+    if (lane == 0) P.part[(size_t)(g + DOT_G * w) * R + rb] = (double)s;
+  }
+  // the group's last CTA
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) sh.last = (atomicAdd(&ctl->dticket[g], 1u) == (unsigned)R - 1u) ? 1 : 0;
+  __syncthreads();
+  if (!sh.last) return;
+  __threadfence();
+  // st_reduce's sums of columns g + DOT_G w: lane l adds partials l, l + 64, ... and
+  // l + 32, l + 96, ..., then a butterfly
+  if (w < mine) {
+    const double* p = P.part + (size_t)(g + DOT_G * w) * R;
+    double a0 = 0.0, a1 = 0.0;
+    for (int r0 = 0; r0 < R; r0 += 512) {
+      double x[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) {
+        const int r = r0 + lane + 32 * u;
+        x[u] = (r < R) ? __ldcg(p + r) : 0.0;
+      }
+      const int left = (R - r0 + 31) / 32;
+#pragma unroll
+      for (int u = 0; u < 16; u += 2) {
+        if (u < left) a0 += x[u];
+        if (u + 1 < left) a1 += x[u + 1];
+      }
+    }
+    const double a = warp_sum(a0 + a1);
+    if (lane == 0) ctl->h1[g + DOT_G * w] = a;
+  }
+  if (threadIdx.x == 0) ctl->dticket[g] = 0u;
 }
 
 // B, one pass over Q: each thread keeps its rows of the nv basis columns in
@@ -1277,7 +1320,9 @@ __global__ void __launch_bounds__(LZ_BLOCK, 2) st_update_dot1_kernel(
   for (int c = threadIdx.x; c < nv; c += LZ_BLOCK) sh.hv[c] = (VT)__ldg(&ctl->h1[c]);
   extern __shared__ __align__(16) unsigned char st_dyn[];
   AT* sacc = (AT*)st_dyn;
-  for (int c = 0; c < nv; ++c) sacc[c * LZ_BLOCK + threadIdx.x] = (AT)0;
+  AT acc[MAXM];
+#pragma unroll
+  for (int c = 0; c < MAXM; ++c) acc[c] = (AT)0;
   __syncthreads();
   const int nch = (n + CROWS - 1) / CROWS;
   const int c0 = (int)((long long)nch * blockIdx.x / R);
@@ -1287,9 +1332,9 @@ __global__ void __launch_bounds__(LZ_BLOCK, 2) st_update_dot1_kernel(
     const int r0 = ch * CROWS + RW * threadIdx.x;
     if (r0 >= n) continue;
     const bool full = r0 + RW <= n;
-    VT q[MP1][RW];
+    VT q[MAXM][RW];
 #pragma unroll
-    for (int c = 0; c < MP1; ++c)
+    for (int c = 0; c < MAXM; ++c)
       if (c < nv) {
         const VT* src = P.Q + (size_t)c * ld + r0;
         if constexpr (RW == 2) {
@@ -1310,7 +1355,7 @@ __global__ void __launch_bounds__(LZ_BLOCK, 2) st_update_dot1_kernel(
       s[j] = (VT)0;
     }
 #pragma unroll
-    for (int c = 0; c < MP1; ++c)
+    for (int c = 0; c < MAXM; ++c)
       if (c < nv) {
         const VT h = sh.hv[c];
 #pragma unroll
@@ -1322,14 +1367,17 @@ __global__ void __launch_bounds__(LZ_BLOCK, 2) st_update_dot1_kernel(
       if (r0 + j < n) v[r0 + j] = x[j];
     }
 #pragma unroll
-    for (int c = 0; c < MP1; ++c)
+    for (int c = 0; c < MAXM; ++c)
       if (c < nv) {
         AT d = (AT)0;
 #pragma unroll
         for (int j = 0; j < RW; ++j) d += (AT)q[c][j] * (AT)x[j];
-        sacc[c * LZ_BLOCK + threadIdx.x] += d;
+        acc[c] += d;
       }
   }
+#pragma unroll
+  for (int c = 0; c < MAXM; ++c)
+    if (c < nv) sacc[c * LZ_BLOCK + threadIdx.x] = acc[c];
   double* part = P.part + (size_t)MP1 * R;
   st_block_cols(sacc, nv, part + blockIdx.x, R);
   if (!st_last_cta(&ctl->ticket[1], sh)) return;
@@ -2780,31 +2828,20 @@ static int run_typed(const DeviceInfo& di, const LanczosProblem* probs, int coun
   return 0;
 }
 
-// CTAs per SM of each partial-sum kernel of the stream path (A2, B, C, the
-// rotation), measured once per precision; each kernel runs one wave of its
-// own size.  Sets the dot kernels' dynamic shared memory limit on the way.
+// Row blocks per SM of the stream path's partial-sum kernels and the rotation (A2,
+// B, C, rotation).  They fix which rows share a partial sum, and with that the
+// last bits of every dot, so they are numbers of their own and not the kernels'
+// occupancies (which they were when each row block was one CTA of one wave).
+// Sets the dynamic shared memory limit of B on the way.
 template <typename VT>
 static const int* stream_occ() {
-  static int occ[4] = {0, 0, 0, 0};
+  static const int blocks[4] = {sizeof(VT) == 4 ? 4 : 3, 2, 4, sizeof(VT) == 4 ? 3 : 2};
   static std::once_flag once;
   std::call_once(once, [] {
-    const void* ks[] = {(const void*)st_dot_kernel<VT>, (const void*)st_update_dot1_kernel<VT>,
-                        (const void*)st_update_norm_kernel<VT>,
-                        (const void*)st_rotate_kernel<VT>};
-    const size_t dyn[] = {st_sacc_bytes<VT>(), st_sacc_bytes<VT>(), 0, 0};
-    for (int j = 0; j < 4; ++j) {
-      if (dyn[j])
-        cudaFuncSetAttribute(ks[j], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn[j]);
-      int o = 0;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, ks[j], LZ_BLOCK, dyn[j]) !=
-          cudaSuccess) {
-        cudaGetLastError();
-        o = 1;
-      }
-      occ[j] = o < 1 ? 1 : o;
-    }
+    cudaFuncSetAttribute((const void*)st_update_dot1_kernel<VT>,
+                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)st_sacc_bytes<VT>());
   });
-  return occ;
+  return blocks;
 }
 // the largest of them (sizes the partial-sum buffers)
 int lanczos_stream_occupancy(int prec) {
@@ -2948,7 +2985,7 @@ static int run_stream(const DeviceInfo& di, const LanczosProblem& p, cudaStream_
       }
       e = launch_pdl(st_sell_spmv_kernel<VT>, ntiles, 1, 0, stream, t, ctl);
       if (e == cudaSuccess)
-        e = launch_pdl(st_dot_kernel<VT>, g[0], 1, st_sacc_bytes<VT>(), stream, t, ctl);
+        e = launch_pdl(st_dot_kernel<VT>, DOT_G * g[0], 1, 0, stream, t, ctl);
       if (e == cudaSuccess)
         e = launch_pdl(st_update_dot1_kernel<VT>, g[1], 1, st_sacc_bytes<VT>(), stream, t, ctl);
       if (e == cudaSuccess)
