@@ -851,7 +851,7 @@ struct __align__(16) StreamCtl {
   int i, k, bd, cur;           // step, saved vectors, breakdown pending, work vector in use
   int stop, rot, stepped;      // loop ended; rotation pending; the finished cycle had steps
   int restarts, breakdowns, steps, sum_nv, sum_kn, nconv;
-  unsigned ticket[4];          // last-CTA tickets of (unused), B, C and the rotation
+  unsigned ticket[3];          // last-CTA tickets of B, C and the rotation
   unsigned dticket[4];         // of A2's column groups
   double invb;                 // 1 / beta of the latest unnormalised vector
   double h1[MP1], h2[MP1];
@@ -1048,7 +1048,7 @@ __device__ __forceinline__ void st_block_cols(const AT* sacc, int nv, double* ou
   }
 }
 
-// the threads' dot accumulators of B (dynamic shared memory, for their sums)
+// the per-thread dot accumulators of B (dynamic shared memory)
 template <typename VT>
 constexpr size_t st_sacc_bytes() {
   return (size_t)MP1 * LZ_BLOCK * sizeof(typename Acc<VT>::type);
@@ -1320,9 +1320,7 @@ __global__ void __launch_bounds__(LZ_BLOCK, 2) st_update_dot1_kernel(
   for (int c = threadIdx.x; c < nv; c += LZ_BLOCK) sh.hv[c] = (VT)__ldg(&ctl->h1[c]);
   extern __shared__ __align__(16) unsigned char st_dyn[];
   AT* sacc = (AT*)st_dyn;
-  AT acc[MAXM];
-#pragma unroll
-  for (int c = 0; c < MAXM; ++c) acc[c] = (AT)0;
+  for (int c = 0; c < nv; ++c) sacc[c * LZ_BLOCK + threadIdx.x] = (AT)0;
   __syncthreads();
   const int nch = (n + CROWS - 1) / CROWS;
   const int c0 = (int)((long long)nch * blockIdx.x / R);
@@ -1332,9 +1330,9 @@ __global__ void __launch_bounds__(LZ_BLOCK, 2) st_update_dot1_kernel(
     const int r0 = ch * CROWS + RW * threadIdx.x;
     if (r0 >= n) continue;
     const bool full = r0 + RW <= n;
-    VT q[MAXM][RW];
+    VT q[MP1][RW];
 #pragma unroll
-    for (int c = 0; c < MAXM; ++c)
+    for (int c = 0; c < MP1; ++c)
       if (c < nv) {
         const VT* src = P.Q + (size_t)c * ld + r0;
         if constexpr (RW == 2) {
@@ -1355,7 +1353,7 @@ __global__ void __launch_bounds__(LZ_BLOCK, 2) st_update_dot1_kernel(
       s[j] = (VT)0;
     }
 #pragma unroll
-    for (int c = 0; c < MAXM; ++c)
+    for (int c = 0; c < MP1; ++c)
       if (c < nv) {
         const VT h = sh.hv[c];
 #pragma unroll
@@ -1367,25 +1365,22 @@ __global__ void __launch_bounds__(LZ_BLOCK, 2) st_update_dot1_kernel(
       if (r0 + j < n) v[r0 + j] = x[j];
     }
 #pragma unroll
-    for (int c = 0; c < MAXM; ++c)
+    for (int c = 0; c < MP1; ++c)
       if (c < nv) {
         AT d = (AT)0;
 #pragma unroll
         for (int j = 0; j < RW; ++j) d += (AT)q[c][j] * (AT)x[j];
-        acc[c] += d;
+        sacc[c * LZ_BLOCK + threadIdx.x] += d;
       }
   }
-#pragma unroll
-  for (int c = 0; c < MAXM; ++c)
-    if (c < nv) sacc[c * LZ_BLOCK + threadIdx.x] = acc[c];
   double* part = P.part + (size_t)MP1 * R;
   st_block_cols(sacc, nv, part + blockIdx.x, R);
-  if (!st_last_cta(&ctl->ticket[1], sh)) return;
+  if (!st_last_cta(&ctl->ticket[0], sh)) return;
   st_reduce<VT>(part, R, nv, sh);
   for (int c = threadIdx.x; c < nv; c += LZ_BLOCK) ctl->h2[c] = sh.h[c];
   if (threadIdx.x == 0) {
     if (mode == SM_STEP) ctl->alpha[i] = __ldcg(&ctl->h1[i]) + sh.h[i];
-    ctl->ticket[1] = 0u;
+    ctl->ticket[0] = 0u;
   }
 }
 
@@ -1422,7 +1417,7 @@ __global__ void __launch_bounds__(LZ_BLOCK) st_update_norm_kernel(
   }
   double* part = P.part + (size_t)2 * MP1 * R;
   block_reduce_cols(nrm, 1, sh, part + blockIdx.x, R);
-  if (!st_last_cta(&ctl->ticket[2], sh)) return;
+  if (!st_last_cta(&ctl->ticket[1], sh)) return;
   st_reduce<VT>(part, R, 1, sh);
   if (threadIdx.x == 0) {
     const double nrm2 = sh.h[0];
@@ -1444,7 +1439,7 @@ __global__ void __launch_bounds__(LZ_BLOCK) st_update_norm_kernel(
       ctl->invb = 1.0 / sqrt(nrm2);
       ctl->bd = 0;
     }
-    ctl->ticket[2] = 0u;
+    ctl->ticket[1] = 0u;
   }
 }
 
@@ -1539,11 +1534,11 @@ __global__ void __launch_bounds__(LZ_BLOCK) st_rotate_kernel(const __grid_consta
       if (kn != m) P.Q[(size_t)m * ld + row] = xl;
     }
   }
-  if (!st_last_cta(&ctl->ticket[3], sh)) return;
+  if (!st_last_cta(&ctl->ticket[2], sh)) return;
   if (threadIdx.x == 0) {
     ctl->i = kn;     // the next cycle starts from Q[:, kn]
     ctl->rot = 0;
-    ctl->ticket[3] = 0u;
+    ctl->ticket[2] = 0u;
   }
 }
 
@@ -1872,7 +1867,7 @@ __global__ void __launch_bounds__(LZ_BLOCK) wv_update_norm_kernel(
     for (int k = 0; k < LZ_NW; ++k) s += sh.u.st.wred[k][0];
     part[w.rank] = s;
     __threadfence();
-    sh.last = (atomicAdd(&ctl->ticket[2], 1u) == (unsigned)R - 1u) ? 1 : 0;
+    sh.last = (atomicAdd(&ctl->ticket[1], 1u) == (unsigned)R - 1u) ? 1 : 0;
     if (sh.last) __threadfence();
   }
   __syncthreads();
@@ -1899,7 +1894,7 @@ __global__ void __launch_bounds__(LZ_BLOCK) wv_update_norm_kernel(
       ctl->invb = 1.0 / b;
       ctl->bd = 0;
     }
-    ctl->ticket[2] = 0u;
+    ctl->ticket[1] = 0u;
   }
 }
 
