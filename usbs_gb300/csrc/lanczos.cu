@@ -2014,6 +2014,7 @@ struct ClCtx {
   int rank, C, n, m, rc, r0, rows;
   int lanes, lp;        // accumulators per row of the SpMV, threads per row (lp <= lanes)
   bool staged;          // CSR slice in shared memory
+  bool short_rows;      // not staged, few entries per lane: four rows at a time
   int rp, cg, vs;       // its row bounds (rows+1 ints, from the slice's start), columns, values
   int xs;               // the whole x, copied at the start of each SpMV (or -1)
   const int* g_rowptr;  // the operator in global memory (slices that do not fit)
@@ -2117,6 +2118,68 @@ __device__ __forceinline__ VT cl_row_sum(const ClCtx<VT>& X, int lr, int lig, in
   return (VT)r;
 }
 
+// Row sums of a slice in global memory with short rows (lp = lanes: one accumulator
+// per thread): four rows per thread group at a time, whose bounds, first two entries
+// and gathers are in flight together, so a group waits for three round trips to L2
+// per four rows and for two more per further entry of a lane.  cl_row_sum takes one
+// row at a time, three round trips for up to eight entries of a lane.
+template <typename VT, bool XS>
+__device__ __forceinline__ void cl_spmv_global(const ClCtx<VT>& X, int xo, VT xscale, int vout) {
+  typedef typename Acc<VT>::type AT;
+  constexpr int R = 4, U = 2;                      // rows, entries of each in flight
+  const int L = X.lanes, gpp = LZ_BLOCK / L;
+  const int g = threadIdx.x / L, lig = threadIdx.x & (L - 1);
+  VT* D = cl_dyn_words<VT>();
+  auto gather = [&](int gc) -> VT {
+    if constexpr (XS) {
+      return D[X.xs + gc];
+    } else {
+      const int o = gc / X.rc;
+      return cl_ld(cl_map(D + xo + (gc - o * X.rc), (unsigned)o), (VT)0);
+    }
+  };
+  for (int base = 0; base < X.rows; base += R * gpp) {
+    int pb[R], pe[R], c[R][U];
+    VT v[R][U], xv[R][U];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int lr = base + r * gpp + g;
+      pb[r] = pe[r] = 0;
+      if (lr < X.rows) {
+        pb[r] = X.g_rowptr[X.r0 + lr] + lig;
+        pe[r] = X.g_rowptr[X.r0 + lr + 1];
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int p = pb[r] + u * L;
+        c[r][u] = (p < pe[r]) ? X.g_col[p] : -1;
+        v[r][u] = (p < pe[r]) ? X.g_val[p] : (VT)0;
+      }
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        xv[r][u] = (VT)0;
+        if (c[r][u] >= 0) xv[r][u] = gather(c[r][u]);
+      }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      AT s = (AT)0;
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (c[r][u] >= 0) s += (AT)v[r][u] * (AT)xv[r][u];
+      for (int p = pb[r] + U * L; p < pe[r]; p += L)
+        s += (AT)X.g_val[p] * (AT)gather(X.g_col[p]);
+      for (int o = L >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      const int lr = base + r * gpp + g;
+      if (lig == 0 && lr < X.rows) D[vout + lr] = (VT)s * xscale;
+    }
+  }
+}
+
 // vout = Op x * xscale for own rows; x and vout are offsets, the gathers read the
 // owner CTA's copy of x (or this CTA's copy of all of it)
 template <typename VT, int NL, bool XS>
@@ -2130,6 +2193,10 @@ __device__ __forceinline__ void cl_spmv_rows(const ClCtx<VT>& X, int xo, VT xsca
 }
 template <typename VT, bool XS>
 __device__ __forceinline__ void cl_spmv(const ClCtx<VT>& X, int xo, VT xscale, int vout) {
+  if (X.short_rows) {
+    cl_spmv_global<VT, XS>(X, xo, xscale, vout);
+    return;
+  }
   switch (X.lanes / X.lp) {
     case 1: cl_spmv_rows<VT, 1, XS>(X, xo, xscale, vout); break;
     case 2: cl_spmv_rows<VT, 2, XS>(X, xo, xscale, vout); break;
@@ -2463,6 +2530,11 @@ lanczos_cluster_kernel(const __grid_constant__ ClusterBatch<VT> batch) {
   const int p0 = (X.rows > 0) ? P.rowptr[X.r0] : 0;
   const int p1 = (X.rows > 0) ? P.rowptr[X.r0 + X.rows] : 0;
   X.staged = (p1 - p0) <= P.csr_cap;
+  // up to 3.5 entries per lane and row on average; kilocycles of a step's SpMV, 16
+  // CTAs, four rows at a time / one row at a time: ER n = 7000 of degree 80 (2.5 per
+  // lane) 52 / 71, n = 5000 of degree 100 (3.1) 46 / 54, of degree 130 (4.1) 59 / 55,
+  // n = 4000 of degree 200 (6.3) 70 / 44
+  X.short_rows = !X.staged && 2ll * (p1 - p0) <= 7ll * X.lanes * X.rows;
   X.lp = 1;
   // (a slice read from global memory keeps one thread per accumulator: its
   // consecutive entries are then consecutive lanes')
