@@ -3215,8 +3215,16 @@ static int run_cluster(const LanczosProblem* probs, int count, cudaStream_t stre
   ClusterBatch<VT> batch;
   batch.count = count;
   size_t dyn = 0;
+  // the largest operators first: clusters start in launch order and a long one
+  // started last runs alone
+  int order[MAX_TEAMS];
   for (int i = 0; i < count; ++i) {
-    const LanczosProblem& p = probs[i];
+    int j = i;
+    for (; j > 0 && probs[order[j - 1]].nnz < probs[i].nnz; --j) order[j] = order[j - 1];
+    order[j] = i;
+  }
+  for (int i = 0; i < count; ++i) {
+    const LanczosProblem& p = probs[order[i]];
     if (p.m > MAXM || p.m < 1 || p.n < 1 || p.ld < p.n) return 1;
     const int rc = (p.n + csize - 1) / csize;
     const ClLayout base = cl_layout<VT>(p.m, rc, 0);
