@@ -1558,8 +1558,8 @@ __global__ void __launch_bounds__(LZ_BLOCK) st_rotate_kernel(const __grid_consta
 // vector, in B, from the other CTAs' shared memory).  So four times as many
 // SMs work, a step has four kernel boundaries where the team kernel has three
 // grid barriers of about 20k cycles, and the results are the same bits.
-// ER n = 30,011 of degree 12, FP32, 10 restarts: 14.4 ms per call as one
-// cooperative launch of 30 CTAs, 5.3 with A1 and A2 as one kernel.
+// ER n = 30,011 of degree 12, FP32, 10 restarts: 4.8 ms per call (14.4 as one
+// cooperative launch of 30 CTAs, 5.3 with A1 and A2 as one kernel).
 constexpr int WV_C = 4;                  // CTAs (tiles) per rank
 constexpr int WV_U = 8;                  // columns per CTA: c = j + 4 u
 
@@ -1963,10 +1963,10 @@ __host__ __device__ inline ClLayout cl_layout(int m, int rc, int csr_cap) {
 // h[c] = sum over the cluster's CTAs r = 0..C-1 of part_r[c], c < nv, summed
 // as a fixed pairwise tree over 16 slots (slots r >= C hold 0): level one adds
 // slots r and r+8, level two r and r+4, level three r and r+2, level four r and
-// r+1.  An FP64 add holds its SM sub-partition's FP64 pipe for ~64 cycles, so
-// warps 0..3 (one per sub-partition) each form one level-two sum
-// R_w = (v_w + v_{w+8}) + (v_{w+4} + v_{w+12}), and warp 0 then forms
-// (R_0 + R_2) + (R_1 + R_3): the tree's association, spread over four pipes.
+// r+1.  A warp gets one FP64 add per ~60 cycles, dependent or not, while the SM's
+// FP64 unit takes one from any warp every 19, so warps 0..3 each form one
+// level-two sum R_w = (v_w + v_{w+8}) + (v_{w+4} + v_{w+12}), and warp 0 then forms
+// (R_0 + R_2) + (R_1 + R_3): the tree's association, spread over four warps.
 // With norm set (nv = 1), lane 0 also forms sh.bnorm = sqrt(h[0]) and
 // sh.binv = 1 / bnorm once for the CTA (FP64 square roots and divisions are
 // long dependent chains on this part's narrow FP64 pipe).
@@ -2029,7 +2029,7 @@ struct ClCtx {
 // need no shuffle; the sums do not depend on lp.  lp is chosen so that one pass
 // of the CTA covers its rows: with one row per warp (lanes = 32, 62 FP64 rows of
 // 49 entries per CTA) the shuffle tree's FP64 adds took 50k cycles per step,
-// because an FP64 warp instruction holds its pipe for 64 cycles however few
+// because an FP64 warp instruction costs the SM's one unit 19 cycles however few
 // lanes carry a row.
 // XS: x is read from the CTA's copy and cg holds byte offsets in it; else cg
 // holds the shared::cluster address of the entry's row in its owner's Q[:, 0].
@@ -2276,8 +2276,8 @@ __device__ __forceinline__ void cl_block_cols(LzShared<VT>& sh, int nrw, int nv,
 }
 
 // A thread's rows are taken RT at a time (lr, lr + 256, ...).  In FP32 the loads
-// and FMA chains of three rows overlap (CTAs of at most 256 rows: one); in FP64 one row's chain already
-// keeps its pipe busy (64 cycles per instruction).
+// and FMA chains of three rows overlap (CTAs of at most 256 rows: one); in FP64 the
+// CTA's warps already keep the SM's FP64 unit busy (19 cycles per instruction).
 template <typename VT> constexpr int cl_rt() { return sizeof(VT) == 4 ? 3 : 1; }
 
 // G columns c0 .. of a thread's RT rows; with PART, those at or past nv as 0.
@@ -2340,8 +2340,8 @@ __device__ __forceinline__ void cl_dot_rows(const ClCtx<VT>& X, int lr, int nv, 
 // Partial dots Q[:, c] . vec, c < nv <= 32, over the CTA's rows.  Lane l of
 // row-warp w accumulates rows 32 w + l, 32 w + l + 256, ...; CTAs with at most
 // 128, 64 or 32 rows have 4, 2 or 1 row-warps and give each 2, 4 or 8 warps,
-// which split the columns, so that all four SM sub-partitions (and their FP64
-// pipes) work.  vec may just have been written by other threads.
+// which split the columns, so that all eight warps work.  vec may just have been
+// written by other threads.
 template <int CW, typename VT>
 __device__ __forceinline__ void cl_dots_w(const ClCtx<VT>& X, LzShared<VT>& sh, int nv, int vec,
                                           double* part_out) {
@@ -3098,14 +3098,16 @@ static int run_noncluster(const DeviceInfo& di, const LanczosProblem* probs, int
       }
     }
     if (nt) {
-      // a few team-size problems: one after another on the wave path (2.7 against
-      // 14 ms for one at n = 30,000), with the team sizes, and so the results, of
-      // the shared launch, which would run four in about 14 ms; more, or teams
-      // shrunk to fit one launch, share it
+      // one or two team-size problems: one after another on the wave path, with the
+      // team sizes, and so the results, of the shared launch.  ms for one, two,
+      // three and four on it / in a shared launch, whose time hardly depends on
+      // their number: FP32 n = 30,011 4.9, 9.7, 14.6, 19.0 / 14.5 - 15.1; FP64
+      // n = 20,000 8.7, 17.4, 25.8, 34.5 / 22.3 - 22.7, n = 12,100 8.2, 16.2, 24.0,
+      // 31.8 / 20.0 - 20.2.  More, or teams shrunk to fit one launch, share it
       const int occ = (sizeof(VT) == 8) ? di.lanczos_occ64 : di.lanczos_occ32;
       const int maxc = (di.sm_count > 4 ? di.sm_count - 2 : di.sm_count) * (occ > 0 ? occ : 1);
       int want[MAX_TEAMS], total = 0;
-      bool wave = nt <= 4;
+      bool wave = nt <= 2;
       for (int i = 0; i < nt; ++i) {
         want[i] = lanczos_team_size(di, team[i].n, sizeof(VT) == 8 ? 64 : 32);
         total += want[i];
@@ -3133,9 +3135,9 @@ constexpr size_t cl_budget() { return 227 * 1024 - sizeof(LzShared<VT>) - 1024; 
 // target number of rows per CTA.  Each step's phases scale with the rows per
 // CTA and its cluster reductions with the CTAs, and clusters of one launch
 // (or of concurrent solves) compete for the SMs: on GB300 a lone problem runs
-// fastest spread over 16 CTAs (FP32 n = 5000: 4.8 ms at 16 CTAs, 8.7 ms at 8),
-// while 48 problems in one launch run fastest packed at 640 rows per CTA
-// (17 ms against 27 ms spread).  A caller that knows its launch shares the
+// fastest spread over 16 CTAs (FP32 n = 5000: 4.8 ms at 16 CTAs, 8.7 ms at 8 when
+// the line was drawn), while 48 problems in one launch run fastest packed at 640
+// rows per CTA (17 ms against 27 ms spread then; 8.65 ms packed now).  A caller that knows its launch shares the
 // GPU (a solve service) passes its own rows per CTA in the problem; otherwise
 // the class's measured choice is used (usbs_lanczos_autotune times the
 // candidates on a caller's batch and records the fastest for its precision,
