@@ -105,8 +105,10 @@ __global__ void __launch_bounds__(RED_BLOCK) gram_kernel(GramArgs a) {
 // blocks and the same order of every sum, so the same result.  A block's row
 // tiles are staged four at a time, the next four's loads issued before this
 // four's FMAs: with nine entries over 3.4e5 rows (the QAP's A* projections) a
-// block's chain of dependent FMAs is the bound (1820 of 60 cycles, 55 of the 98 us)
-// and every wait for a load between two of them adds to it (245 us).
+// block's chain of dependent FMAs is the bound (1820 of 60 cycles, 55 of the 89 us)
+// and every wait for a load between two of them adds to it (245 us; 98 with the
+// staged operands read right before their FMAs, 161 with a tile of them read ahead
+// in straight-line code).
 constexpr int GS_T = 4;              // tiles per stage
 constexpr int GS_MAXC = 16;          // widest operand staged this way
 __global__ void __launch_bounds__(RED_BLOCK) gram_small_kernel(GramArgs a) {
@@ -151,14 +153,17 @@ __global__ void __launch_bounds__(RED_BLOCK) gram_small_kernel(GramArgs a) {
       const double* y = (same ? xs : ys) + q * LDS_R;
       // (tiles past the end hold zeros; like gram_kernel they are not added)
       const int nt = min(GS_T, (ntiles - tile0 + (int)gridDim.x - 1) / (int)gridDim.x);
-      for (int t = 0; t < nt; ++t) {
-#pragma unroll
-        for (int r = 0; r < GR_ROWS; r += 2) {
-          const double2 xv = *(const double2*)(x + t * GR_ROWS + r);
-          const double2 yv = *(const double2*)(y + t * GR_ROWS + r);
-          acc += xv.x * yv.x;
-          acc += xv.y * yv.y;
-        }
+      // the next rows' operands are in registers before this pair's FMAs
+      const double2* x2 = (const double2*)x;
+      const double2* y2 = (const double2*)y;
+      double2 xc = x2[0], yc = y2[0];
+#pragma unroll 1
+      for (int r = 0; r < nt * (GR_ROWS / 2); ++r) {
+        const double2 xn = x2[r + 1], yn = y2[r + 1];   // (after the last: the padding)
+        acc += xc.x * yc.x;
+        acc += xc.y * yc.y;
+        xc = xn;
+        yc = yn;
       }
     }
     __syncthreads();
