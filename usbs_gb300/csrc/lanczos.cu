@@ -1914,9 +1914,9 @@ __global__ void __launch_bounds__(LZ_BLOCK) wv_update_norm_kernel(
 // identical results), which needs no broadcast; its FP64 refinement is shared
 // out.  A cluster is co-scheduled by the hardware, so there is no software
 // barrier and no spin-wait.
-// Bound by latency: FP32 torus n = 10^4 runs 20k cycles per step (SpMV and dots
-// 5.9k, second projection 5.6k, norm pass 2.6k, reductions 4.5k, barriers 1.7k)
-// and 160k per restart, 2.22 ms per call of 131 steps (3.53 ms with one
+// Bound by latency: FP32 torus n = 10^4 runs 19k cycles per step (SpMV and dots
+// 5.9k, second projection 4.2k, norm pass 2.6k, reductions 4.5k, barriers 1.7k)
+// and 153k per restart, 2.13 ms per call of 131 steps (3.53 ms with one
 // gather, one column and one shuffle level at a time); FP64 ER n = 800 of
 // degree 48 3.06 ms (8.25 ms).
 constexpr int CL_MAX_CTAS = 16;
@@ -2043,7 +2043,7 @@ __device__ __forceinline__ VT cl_row_sum(const ClCtx<VT>& X, int lr, int lig, in
   if (lr < X.rows) {
     constexpr int B = NL < 8 ? NL : 8;           // entries in flight per round trip ...
     constexpr int U = NL < 8 ? 8 / NL : 1;       // ... over U trips round the accumulators
-    if (X.staged) {
+    if ((NL > 1 && sizeof(VT) == 4) || X.staged) {
       const VT* D = cl_dyn_words<VT>();
       const int* rp = cl_dyn_words<int>() + X.rp;
       const uint32_t* cg = cl_dyn_words<uint32_t>() + X.cg;
@@ -2076,7 +2076,7 @@ __device__ __forceinline__ VT cl_row_sum(const ClCtx<VT>& X, int lr, int lig, in
           }
         }
       }
-    } else {
+    } else if constexpr (NL == 1 || sizeof(VT) == 8) {
       const int e = X.g_rowptr[X.r0 + lr + 1];
       for (int p0 = X.g_rowptr[X.r0 + lr] + lig; p0 < e; p0 += U * L) {
 #pragma unroll
@@ -2180,6 +2180,16 @@ __device__ __forceinline__ void cl_spmv_global(const ClCtx<VT>& X, int xo, VT xs
   }
 }
 
+// the same out of line.  In FP32 the staged path's kernel is then faster (torus
+// n = 10^4: 2.13 against 2.23 ms per call, its second projection 4.2 against 5.5
+// kilocycles per step), while slices in global memory lose up to a fifth of their
+// SpMV (n = 7000 of degree 80: 62 against 51); in FP64 inline is the faster form
+// (ER n = 800: 2.92 against 2.97 ms).
+template <typename VT, bool XS>
+__device__ __noinline__ void cl_spmv_global_call(const ClCtx<VT> X, int xo, VT xscale, int vout) {
+  cl_spmv_global<VT, XS>(X, xo, xscale, vout);
+}
+
 // vout = Op x * xscale for own rows; x and vout are offsets, the gathers read the
 // owner CTA's copy of x (or this CTA's copy of all of it)
 template <typename VT, int NL, bool XS>
@@ -2194,7 +2204,8 @@ __device__ __forceinline__ void cl_spmv_rows(const ClCtx<VT>& X, int xo, VT xsca
 template <typename VT, bool XS>
 __device__ __forceinline__ void cl_spmv(const ClCtx<VT>& X, int xo, VT xscale, int vout) {
   if (X.short_rows) {
-    cl_spmv_global<VT, XS>(X, xo, xscale, vout);
+    if constexpr (sizeof(VT) == 4) cl_spmv_global_call<VT, XS>(X, xo, xscale, vout);
+    else cl_spmv_global<VT, XS>(X, xo, xscale, vout);
     return;
   }
   switch (X.lanes / X.lp) {
@@ -2531,8 +2542,8 @@ lanczos_cluster_kernel(const __grid_constant__ ClusterBatch<VT> batch) {
   const int p1 = (X.rows > 0) ? P.rowptr[X.r0 + X.rows] : 0;
   X.staged = (p1 - p0) <= P.csr_cap;
   // up to 3.5 entries per lane and row on average; kilocycles of a step's SpMV, 16
-  // CTAs, four rows at a time / one row at a time: ER n = 7000 of degree 80 (2.5 per
-  // lane) 52 / 71, n = 5000 of degree 100 (3.1) 46 / 54, of degree 130 (4.1) 59 / 55,
+  // CTAs, four rows at a time (inlined) / one row at a time: ER n = 7000 of degree 80
+  // (2.5 per lane) 52 / 71, n = 5000 of degree 100 (3.1) 46 / 54, of degree 130 (4.1) 59 / 55,
   // n = 4000 of degree 200 (6.3) 70 / 44
   X.short_rows = !X.staged && 2ll * (p1 - p0) <= 7ll * X.lanes * X.rows;
   X.lp = 1;
@@ -3137,7 +3148,7 @@ constexpr size_t cl_budget() { return 227 * 1024 - sizeof(LzShared<VT>) - 1024; 
 // (or of concurrent solves) compete for the SMs: on GB300 a lone problem runs
 // fastest spread over 16 CTAs (FP32 n = 5000: 4.8 ms at 16 CTAs, 8.7 ms at 8 when
 // the line was drawn), while 48 problems in one launch run fastest packed at 640
-// rows per CTA (17 ms against 27 ms spread then; 8.65 ms packed now).  A caller that knows its launch shares the
+// rows per CTA (17 ms against 27 ms spread then; 8.5 ms packed now).  A caller that knows its launch shares the
 // GPU (a solve service) passes its own rows per CTA in the problem; otherwise
 // the class's measured choice is used (usbs_lanczos_autotune times the
 // candidates on a caller's batch and records the fastest for its precision,
