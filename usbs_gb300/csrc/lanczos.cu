@@ -2750,10 +2750,22 @@ static thread_local int t_launches = 0;   // kernels the last lanczos_run launch
 // the stream path
 static bool x_fits_smem(int n, size_t vt) { return (size_t)n * vt <= (size_t)LZ_XS_BYTES; }
 
-// team path: 3 work vectors, [pass][column][cta] partials, the Ritz vectors
-// and the barrier counters.  Stream path (nctas = its grid): 2 work vectors
-// and the control block in the third vector's place, the same partials and
-// Ritz vectors.
+// Workspace: 3 work vectors, [pass][column][cta] partials, the Ritz vectors and the
+// barrier counters; the stream path adds its operator layout.  The stream and wave
+// paths' control block lies behind the third pass's partials, which are one column
+// (the sums of squares) of the MP1 that the pass has room for: from six CTAs
+// on it needs no room of its own.
+static size_t ctl_offset(int nctas) {      // in bytes from the partials' start
+  return ((size_t)(2 * MP1 + 1) * nctas * sizeof(double) + 15) & ~(size_t)15;
+}
+static size_t part_bytes(int nctas, bool with_ctl) {
+  const size_t p = (size_t)3 * nctas * MP1 * sizeof(double);
+  const size_t c = ctl_offset(nctas) + sizeof(StreamCtl);
+  return align256(with_ctl && c > p ? c : p);
+}
+static bool ctl_fits(int nctas) {          // without more room than the partials'
+  return ctl_offset(nctas) + sizeof(StreamCtl) <= (size_t)3 * nctas * MP1 * sizeof(double);
+}
 // entries per row a stream-path slice holds (longer rows finish from the CSR)
 static int sell_wcap(int n, long long nnz) {
   const long long avg = n > 0 ? (nnz + n - 1) / n : 1;
@@ -2771,14 +2783,14 @@ size_t lanczos_workspace_bytes(int n, long long nnz, int ld, int m, int prec, in
                                bool stream) {
   (void)m;
   const size_t vt = (prec == 64) ? 8 : 4;
+  const bool strm = stream || !x_fits_smem(n, vt);
   size_t b = align256(3 * (size_t)ld * vt);
-  b += align256((size_t)3 * nctas * MP1 * sizeof(double));
+  b += part_bytes(nctas, strm);
   b += align256((size_t)MAXM * MAXM * sizeof(double));
   b += 256;  // barrier counters
-  if (stream || !x_fits_smem(n, vt)) b += sell_bytes(n, nnz, vt);
+  if (strm) b += sell_bytes(n, nnz, vt);
   return b;
 }
-static_assert(sizeof(StreamCtl) <= 32 * 4 * 32, "the control block takes one 32-row vector slot");
 
 int lanczos_lanes(int n, long long nnz) {
   const double avg = n > 0 ? (double)nnz / n : 1.0;
@@ -2930,13 +2942,15 @@ int lanczos_stream_occupancy(int prec) {
 }
 
 // Whether a problem runs on the wave path: a team-size problem whose ranks hold at
-// most four tiles, outside a stream capture (the loop state is read back once per
+// most four tiles and whose workspace has room for the control block (six ranks; below
+// that only what a batch with a larger problem, or a cluster that cannot be had,
+// sends here), outside a stream capture (the loop state is read back once per
 // restart).
 template <typename VT>
 static bool wave_fits(const LanczosProblem& p, int nctas, cudaStream_t stream) {
   if (p.m > MAXM || p.m < 1 || p.n < 1 || p.ld < p.n) return false;
   const int tiles = (p.n + LZ_BLOCK - 1) / LZ_BLOCK;
-  if (nctas < 1 || (tiles + nctas - 1) / nctas > WV_C) return false;
+  if (nctas < 1 || (tiles + nctas - 1) / nctas > WV_C || !ctl_fits(nctas)) return false;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(stream, &cs) != cudaSuccess) { cudaGetLastError(); return false; }
   return cs == cudaStreamCaptureStatusNone;
@@ -3012,9 +3026,10 @@ static int run_stream(const DeviceInfo& di, const LanczosProblem& p, cudaStream_
   t.Q = (VT*)p.Q; t.Qw = t.Q; t.qts = LZ_BLOCK; t.qcs = p.ld;
   char* w = (char*)p.work;
   t.vbuf = (VT*)w;
-  StreamCtl* ctl = (StreamCtl*)(t.vbuf + 2 * (size_t)p.ld);
   w += align256(3 * (size_t)p.ld * sizeof(VT));
-  t.part = (double*)w; w += align256((size_t)3 * G * MP1 * sizeof(double));
+  t.part = (double*)w;
+  StreamCtl* ctl = (StreamCtl*)(w + ctl_offset(G));
+  w += part_bytes(G, !wave);
   t.Ybuf = (double*)w; w += align256((size_t)MAXM * MAXM * sizeof(double));
   t.bar = nullptr;
   w += 256;
