@@ -134,7 +134,8 @@ size_t usbs_eigsh_workspace_bytes(int n, long long nnz, int inner_iterations, in
  * inner_iterations (<= 32) vectors, at most max_restarts cycles and absolute
  * residual tolerance `tolerance`.
  *   q0:   unit start vector, n entries of the `precision` type;
- *   Q:    ldq x (inner_iterations + 1) column-major (`precision` type, ldq >= n);
+ *   Q:    ldq x (inner_iterations + 1) column-major (`precision` type, ldq >= n;
+ *         on the stream path columns start on 16-byte boundaries, or -2);
  *         on return Q[:, :num_desired] are the eigenvectors;
  *   eigenvalues: num_desired doubles (ascending);
  *   info: 16 ints: [0] saved vectors of the last restart, [1] converged count,

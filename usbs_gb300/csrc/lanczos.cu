@@ -38,6 +38,7 @@ constexpr int LZ_XS_BYTES = 160 * 1024;   // dynamic shared memory for a staged 
 template <typename VT>
 struct TeamDesc {
   int n, ld, m, num_desired, max_restarts, lanes, first_cta, nctas, xsmem;
+  int ldv;               // stride of vbuf's vectors: n rounded up to 32, whatever ld is
   long long nnz;
   double tol;
   const int* rowptr;
@@ -224,8 +225,8 @@ __device__ void phase_spmv(const TeamDesc<VT>& P, LzShared<VT>& sh, int t0, int 
   VT* xs = (VT*)lz_dyn;
   const bool use_xs = P.xsmem != 0;
   if (use_xs) {
-    // 16-byte loads, several in flight per thread (xsrc is a 256-byte aligned
-    // vector buffer or a column of Q with ld a multiple of 32)
+    // 16-byte loads, several in flight per thread (xsrc is one of vbuf's vectors,
+    // 128-byte aligned)
     constexpr int VE = 16 / (int)sizeof(VT);
     const int n16 = P.n / VE;
     const uint4* src = (const uint4*)xsrc;
@@ -679,7 +680,7 @@ lanczos_team_kernel(const __grid_constant__ TeamBatch<VT> batch) {
   if (rank == 0 && tid < MAXM) { sh.alpha[tid] = 0.0; sh.beta[tid] = 0.0; }
   if (tid == 0) sh.eig_cycles = 0;
   // the start vector Q[:, 0]: flat copy for the first cycle's gathers
-  VT* xk = P.vbuf + 2 * ld;
+  VT* xk = P.vbuf + 2 * (size_t)P.ldv;
   for (int tile = t0; tile < t1; ++tile) {
     const int row = tile * LZ_BLOCK + tid;
     if (row < n) xk[row] = P.Q[row];
@@ -705,7 +706,7 @@ lanczos_team_kernel(const __grid_constant__ TeamBatch<VT> batch) {
           // Krylov space exhausted: random vector orthogonalised twice
           // against Q[:, :i] (solver/lanczos.py:107-117)
           ++breakdowns;
-          VT* buf = P.vbuf + (size_t)prev * ld;
+          VT* buf = P.vbuf + (size_t)prev * P.ldv;
           phase_random(P, sh, t0, t1, i, (uint64_t)i, buf, part0 + rank);
           if (!team_sync()) return;
           reduce_part(part0, R, i, sh);
@@ -719,10 +720,10 @@ lanczos_team_kernel(const __grid_constant__ TeamBatch<VT> batch) {
         } else {
           invb = (VT)(1.0 / b);
         }
-        xsrc = P.vbuf + (size_t)prev * ld;
+        xsrc = P.vbuf + (size_t)prev * P.ldv;
         wq = true;
       }
-      VT* vout = P.vbuf + (size_t)cur * ld;
+      VT* vout = P.vbuf + (size_t)cur * P.ldv;
       LZ_MARK(1);
       phase_spmv(P, sh, t0, t1, i, xsrc, invb, wq, vout, part0 + rank);
       LZ_MARK(2);
@@ -755,7 +756,7 @@ lanczos_team_kernel(const __grid_constant__ TeamBatch<VT> batch) {
       if (rank == 0 && tid == 0) sh.beta[m - 1] = b;
       if (b < 1e-15) {
         ++breakdowns;
-        VT* buf = P.vbuf + (size_t)prev * ld;
+        VT* buf = P.vbuf + (size_t)prev * P.ldv;
         phase_random(P, sh, t0, t1, m, (uint64_t)m, buf, part0 + rank);
         if (!team_sync()) return;
         reduce_part(part0, R, m, sh);
@@ -785,7 +786,7 @@ lanczos_team_kernel(const __grid_constant__ TeamBatch<VT> batch) {
       sh.u.Ys[e] = (c < kn) ? (VT)__ldcg(P.Ybuf + j * m + c) : (VT)0;
     }
     __syncthreads();
-    const VT* lastv = P.vbuf + (size_t)prev * ld;
+    const VT* lastv = P.vbuf + (size_t)prev * P.ldv;
     for (int tile = t0; tile < t1; ++tile) {
       const int row = tile * LZ_BLOCK + tid;
       if (row < n) {
@@ -1167,13 +1168,13 @@ __global__ void __launch_bounds__(LZ_BLOCK, 8) st_sell_spmv_kernel(
   const size_t ld = (size_t)P.ld;
   const int w0 = blockIdx.x * LZ_BLOCK, row = w0 + threadIdx.x;
   if (mode == SM_BREAKDOWN) {
-    if (row < P.n) P.vbuf[(size_t)buf * ld + row] = (VT)hash_normal((uint64_t)i, (uint64_t)row);
+    if (row < P.n) P.vbuf[(size_t)buf * P.ldv + row] = (VT)hash_normal((uint64_t)i, (uint64_t)row);
     return;
   }
   const int k = ca.y;
   const bool wq = i > k;
   const VT xscale = wq ? (VT)invb_d : (VT)1;
-  const VT* __restrict__ x = wq ? P.vbuf + (size_t)(buf ^ 1) * ld : P.Q + (size_t)k * ld;
+  const VT* __restrict__ x = wq ? P.vbuf + (size_t)(buf ^ 1) * P.ldv : P.Q + (size_t)k * ld;
   const VT xrow = (wq && row < P.n) ? __ldg(x + row) : (VT)0;
   if (has) {
     const int* cp = P.sl_col + sb + lane;
@@ -1203,7 +1204,7 @@ __global__ void __launch_bounds__(LZ_BLOCK, 8) st_sell_spmv_kernel(
   }
   __syncthreads();
   if (row < P.n) {
-    P.vbuf[(size_t)buf * ld + row] = ys[threadIdx.x] * xscale;
+    P.vbuf[(size_t)buf * P.ldv + row] = ys[threadIdx.x] * xscale;
     if (wq) P.Q[(size_t)i * ld + row] = xrow * xscale;
   }
 }
@@ -1229,7 +1230,7 @@ __global__ void __launch_bounds__(LZ_BLOCK) st_dot_kernel(const __grid_constant_
   const size_t ld = (size_t)P.ld;
   const int nch = (P.n + ST_ROWS - 1) / ST_ROWS;
   const int c0 = (int)((long long)nch * rb / R), c1 = (int)((long long)nch * (rb + 1) / R);
-  const VT* v = P.vbuf + (size_t)buf * ld;
+  const VT* v = P.vbuf + (size_t)buf * P.ldv;
   AT acc[DOT_U];
 #pragma unroll
   for (int u = 0; u < DOT_U; ++u) acc[u] = (AT)0;
@@ -1325,7 +1326,7 @@ __global__ void __launch_bounds__(LZ_BLOCK, 2) st_update_dot1_kernel(
   const int nch = (n + CROWS - 1) / CROWS;
   const int c0 = (int)((long long)nch * blockIdx.x / R);
   const int c1 = (int)((long long)nch * (blockIdx.x + 1) / R);
-  VT* v = P.vbuf + (size_t)buf * ld;
+  VT* v = P.vbuf + (size_t)buf * P.ldv;
   for (int ch = c0; ch < c1; ++ch) {
     const int r0 = ch * CROWS + RW * threadIdx.x;
     if (r0 >= n) continue;
@@ -1400,7 +1401,7 @@ __global__ void __launch_bounds__(LZ_BLOCK) st_update_norm_kernel(
   __syncthreads();
   int c0, c1;
   st_chunks(P.n, &c0, &c1);
-  VT* v = P.vbuf + (size_t)buf * ld;
+  VT* v = P.vbuf + (size_t)buf * P.ldv;
   AT nrm[MP1];
   nrm[0] = (AT)0;
   for (int ch = c0; ch < c1; ++ch) {
@@ -1491,7 +1492,7 @@ __global__ void __launch_bounds__(LZ_BLOCK) st_rotate_kernel(const __grid_consta
   const bool stepped = __ldg(&ctl->stepped) != 0;
   const VT invb = (VT)__ldg(&ctl->invb);
   const size_t ld = (size_t)P.ld;
-  const VT* lastv = P.vbuf + (size_t)(__ldg(&ctl->cur) ^ 1) * ld;
+  const VT* lastv = P.vbuf + (size_t)(__ldg(&ctl->cur) ^ 1) * P.ldv;
   for (int e = threadIdx.x; e < m * MAXM; e += LZ_BLOCK) {
     const int j = e / MAXM, c = e - j * MAXM;
     sh.u.Ys[e] = (c < kn) ? (VT)__ldcg(P.Ybuf + j * m + c) : (VT)0;
@@ -1749,14 +1750,14 @@ __global__ void __launch_bounds__(LZ_BLOCK) wv_spmv_kernel(const __grid_constant
   const size_t ld = (size_t)P.ld;
   const int row = blockIdx.x * WV_ROWS + threadIdx.x;
   const bool own = threadIdx.x < WV_ROWS && row < P.n;
-  VT* v = P.vbuf + (size_t)buf * ld;
+  VT* v = P.vbuf + (size_t)buf * P.ldv;
   if (mode == SM_BREAKDOWN) {
     if (own) v[row] = (VT)hash_normal((uint64_t)i, (uint64_t)row);
     return;
   }
   const int k = __ldg(&ctl->k);
   const bool wq = i > k;
-  const VT* x = wq ? P.vbuf + (size_t)(buf ^ 1) * ld : P.Q + (size_t)k * ld;
+  const VT* x = wq ? P.vbuf + (size_t)(buf ^ 1) * P.ldv : P.Q + (size_t)k * ld;
   const VT xscale = wq ? (VT)__ldg(&ctl->invb) : (VT)1;
   if (wq && own) P.Q[(size_t)i * ld + row] = __ldg(x + row) * xscale;
   switch (P.lanes) {
@@ -1778,7 +1779,7 @@ __global__ void __launch_bounds__(LZ_BLOCK) wv_dot_kernel(const __grid_constant_
   int i, nv, buf;
   if (st_mode(ctl, P.m, &i, &nv, &buf) == SM_SKIP) return;
   const WvPlace w = wv_place(P);
-  const VT* v = P.vbuf + (size_t)buf * P.ld;
+  const VT* v = P.vbuf + (size_t)buf * P.ldv;
   VT q[WV_C][WV_U], y[WV_C];
   wv_load(P, w, nv, q);
 #pragma unroll
@@ -1800,7 +1801,7 @@ __global__ void __launch_bounds__(LZ_BLOCK) wv_update_dot_kernel(
   const WvPlace w = wv_place(P);
   const int tid = threadIdx.x, row = w.tile * LZ_BLOCK + tid;
   const bool in = w.j < w.nt && row < P.n;
-  VT* v = P.vbuf + (size_t)buf * P.ld;
+  VT* v = P.vbuf + (size_t)buf * P.ldv;
   WvRow<VT> r;
   r.load(P, row, in, nv, v);
   wv_reduce(P.part, P.nctas, nv, sh);
@@ -1836,7 +1837,7 @@ __global__ void __launch_bounds__(LZ_BLOCK) wv_update_norm_kernel(
   const WvPlace w = wv_place(P);
   const int tid = threadIdx.x, lane = tid & 31, row = w.tile * LZ_BLOCK + tid, R = P.nctas;
   const bool in = w.j < w.nt && row < P.n;
-  VT* v = P.vbuf + (size_t)buf * P.ld;
+  VT* v = P.vbuf + (size_t)buf * P.ldv;
   WvRow<VT> r;
   r.load(P, row, in, nv, v);
   wv_reduce(P.part + (size_t)MP1 * R, R, nv, sh);
@@ -2755,6 +2756,7 @@ static bool x_fits_smem(int n, size_t vt) { return (size_t)n * vt <= (size_t)LZ_
 // paths' control block lies behind the third pass's partials, which are one column
 // (the sums of squares) of the MP1 that the pass has room for: from six CTAs
 // on it needs no room of its own.
+static int vec_stride(int n) { return (n + 31) & ~31; }
 static size_t ctl_offset(int nctas) {      // in bytes from the partials' start
   return ((size_t)(2 * MP1 + 1) * nctas * sizeof(double) + 15) & ~(size_t)15;
 }
@@ -2884,7 +2886,8 @@ static int run_typed(const DeviceInfo& di, const LanczosProblem* probs, int coun
       t.nnz = p.nnz;
       t.Q = (VT*)p.Q;
       char* w = (char*)p.work;
-      t.vbuf = (VT*)w; w += align256(3 * (size_t)p.ld * sizeof(VT));
+      t.ldv = vec_stride(p.n);
+      t.vbuf = (VT*)w; w += align256(3 * (size_t)t.ldv * sizeof(VT));
       t.part = (double*)w; w += align256((size_t)3 * want[i] * MP1 * sizeof(double));
       t.Ybuf = (double*)w; w += align256((size_t)MAXM * MAXM * sizeof(double));
       t.bar = (unsigned int*)w; w += 256;
@@ -2998,6 +3001,11 @@ static int run_stream(const DeviceInfo& di, const LanczosProblem& p, cudaStream_
               "cannot run inside a stream capture", p.n);
     return -2;
   }
+  // the stream path's kernels take four rows of a column as 16-byte words
+  if (!wave && (((uintptr_t)p.Q | (size_t)p.ld * sizeof(VT)) & 15) != 0) {
+    set_error("lanczos: n=%d rows need Q and its columns (ld=%d) on 16-byte boundaries", p.n, p.ld);
+    return -2;
+  }
   const int ntiles = (p.n + LZ_BLOCK - 1) / LZ_BLOCK;
   // partials per pass
   const int G = wave ? wave : lanczos_team_size(di, p.n, sizeof(VT) == 8 ? 64 : 32, true);
@@ -3025,8 +3033,8 @@ static int run_stream(const DeviceInfo& di, const LanczosProblem& p, cudaStream_
   t.rowptr = p.rowptr; t.col = p.col; t.val = (const VT*)p.val;
   t.Q = (VT*)p.Q; t.Qw = t.Q; t.qts = LZ_BLOCK; t.qcs = p.ld;
   char* w = (char*)p.work;
-  t.vbuf = (VT*)w;
-  w += align256(3 * (size_t)p.ld * sizeof(VT));
+  t.ldv = vec_stride(p.n);
+  t.vbuf = (VT*)w; w += align256(3 * (size_t)t.ldv * sizeof(VT));
   t.part = (double*)w;
   StreamCtl* ctl = (StreamCtl*)(w + ctl_offset(G));
   w += part_bytes(G, !wave);
