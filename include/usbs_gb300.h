@@ -116,8 +116,11 @@ int usbs_apply_A_adjoint(int n, int k, const int* row_ptr, const int* r_con, con
 
 /* Which Lanczos path usbs_eigsh_smallest takes for n rows (host call):
  *   1 = one thread-block cluster with the basis in shared memory;
- *   0 = one cooperative launch (a team of CTAs, x staged in shared memory,
- *       n * sizeof(value) <= 160 KB); it needs the whole GPU co-resident;
+ *   0 = a team of CTAs (x staged in shared memory, n * sizeof(value) <= 160 KB)
+ *       in one cooperative launch; it needs the whole GPU co-resident.  One or
+ *       two such problems of a call outside a stream capture run their first
+ *       cycles as ordinary launches (at most 980) before it, with the same
+ *       results;
  *   2 = the stream path (larger n): every Lanczos phase is an ordinary
  *       full-GPU launch, and the loop state is read back once per restart,
  *       so such a call synchronises `stream` at each restart and cannot be
@@ -147,9 +150,11 @@ size_t usbs_eigsh_workspace_bytes(int n, long long nnz, int inner_iterations, in
  *         the three step phases, [13] sum over steps of the active basis
  *         columns, [14] sum over restarts of the saved vectors (for byte counts),
  *         [15] kilo-cycles of CTA 0 in the projected eigensolver.
- * Runs as one kernel launch when the problem's rows fit in a thread-block
- * cluster's shared memory or its x in one CTA's (usbs_lanczos_kernel 1 or 0);
- * the call is then asynchronous.  Larger problems take the stream path
+ * Asynchronous when the problem's rows fit in a thread-block cluster's shared
+ * memory or its x in one CTA's (usbs_lanczos_kernel 1: one launch; 0: one launch,
+ * after the ordinary launches of its first cycles).  The ordinary launches
+ * have no barrier waits ([8]); their counters are those of their first CTAs, [7]
+ * the sum over them.  Larger problems take the stream path
  * (usbs_lanczos_kernel 2): a sequence of launches, with `stream`
  * synchronised once per restart.  Kilo-cycle counters [7..12] stay 0 there. */
 int usbs_eigsh_smallest(int n, long long nnz, const int* rowptr, const int* col,

@@ -35,6 +35,8 @@ constexpr int MP1 = MAXM + 1;
 
 constexpr int LZ_XS_BYTES = 160 * 1024;   // dynamic shared memory for a staged x
 
+struct StreamCtl;
+
 template <typename VT>
 struct TeamDesc {
   int n, ld, m, num_desired, max_restarts, lanes, first_cta, nctas, xsmem;
@@ -65,7 +67,24 @@ struct TeamDesc {
   int* ctl;
   unsigned int* bar;
   int* status;
+  StreamCtl* resume;     // wave path: the loop state the team kernel continues from (else null)
 };
+
+// Loop state of the stream and wave paths (see there).
+struct __align__(16) StreamCtl {
+  int i, k, bd, cur;           // step, saved vectors, breakdown pending, work vector in use
+  int stop, rot, stepped;      // ST_RUN, ...; rotation pending; the finished cycle had steps
+  int restarts, breakdowns, steps, sum_nv, sum_kn, nconv;
+  unsigned ticket[3];          // last-CTA tickets of B, C and the rotation
+  unsigned dticket[4];         // of A2's column groups
+  int breakdowns0, steps0, sum_nv0;   // the counters at the cycle's start
+  double invb;                 // 1 / beta of the latest unnormalised vector
+  double h1[MP1], h2[MP1];
+  double alpha[MAXM], beta[MAXM];
+  unsigned long long cyc[4];   // wave path: cycles of CTA 0 in the reductions and phases A, B, C
+};
+// stop: the loop runs; has ended; (wave path) goes on in the team kernel
+enum { ST_RUN = 0, ST_ENDED = 1, ST_HANDED = 2 };
 
 template <typename VT>
 __device__ __forceinline__ size_t qix(const TeamDesc<VT>& P, int c, int row) {
@@ -679,11 +698,33 @@ lanczos_team_kernel(const __grid_constant__ TeamBatch<VT> batch) {
   } while (0)
   if (rank == 0 && tid < MAXM) { sh.alpha[tid] = 0.0; sh.beta[tid] = 0.0; }
   if (tid == 0) sh.eig_cycles = 0;
-  // the start vector Q[:, 0]: flat copy for the first cycle's gathers
+  if (const StreamCtl* rs = P.resume) {
+    // after the wave path's cycles: its state at the start of a cycle, or its end
+    k = rs->k; nconv = rs->nconv; restart = rs->restarts;
+    breakdowns = rs->breakdowns0; steps = rs->steps0; sum_nv = rs->sum_nv0; sum_kn = rs->sum_kn;
+    if (rank == 0 && tid < MAXM) { sh.alpha[tid] = rs->alpha[tid]; sh.beta[tid] = rs->beta[tid]; }
+    if (timing) {
+      clk_restart = (long long)P.ctl[6] << 10;
+      sh.eig_cycles = (long long)P.ctl[15] << 10;
+      clk_start -= clk_restart;
+      for (int j = 0; j < 4; ++j) {
+        tp[1 + j] = (long long)rs->cyc[j];
+        clk_start -= tp[1 + j];
+      }
+    }
+    if (rs->stop == ST_ENDED) {
+      if (timing) {
+        P.ctl[7] = (int)((clock64() - clk_start) >> 10);
+        for (int j = 0; j < 5; ++j) P.ctl[8 + j] = (int)(tp[j] >> 10);
+      }
+      return;
+    }
+  }
+  // the start vector Q[:, k]: flat copy for the first cycle's gathers
   VT* xk = P.vbuf + 2 * (size_t)P.ldv;
   for (int tile = t0; tile < t1; ++tile) {
     const int row = tile * LZ_BLOCK + tid;
-    if (row < n) xk[row] = P.Q[row];
+    if (row < n) xk[row] = P.Q[(size_t)k * ld + row];
   }
   __syncthreads();
   if (!team_sync()) return;
@@ -848,17 +889,6 @@ lanczos_team_kernel(const __grid_constant__ TeamBatch<VT> batch) {
 // start and derives the same mode (step, breakdown replacement, or nothing
 // to do), so the host enqueues a cycle's launches without reading anything
 // back, and reads the block once per restart.
-struct __align__(16) StreamCtl {
-  int i, k, bd, cur;           // step, saved vectors, breakdown pending, work vector in use
-  int stop, rot, stepped;      // loop ended; rotation pending; the finished cycle had steps
-  int restarts, breakdowns, steps, sum_nv, sum_kn, nconv;
-  unsigned ticket[3];          // last-CTA tickets of B, C and the rotation
-  unsigned dticket[4];         // of A2's column groups
-  double invb;                 // 1 / beta of the latest unnormalised vector
-  double h1[MP1], h2[MP1];
-  double alpha[MAXM], beta[MAXM];
-};
-
 template <typename VT>
 struct StShared {
   union {
@@ -1452,7 +1482,12 @@ __global__ void __launch_bounds__(LZ_BLOCK, 1) st_restart_kernel(
   st_pdl_prologue();
   __shared__ LzShared<VT> sh;
   const int m = P.m, tid = threadIdx.x;
-  if (ctl->stop || ctl->rot || ctl->bd || ctl->i < m) return;
+  if (ctl->stop || ctl->rot) return;
+  if (ctl->bd || ctl->i < m) {
+    // a cycle of the wave path that breakdowns made longer than planned
+    if (P.resume && tid == 0) ctl->stop = ST_HANDED;
+    return;
+  }
   if (tid == 0) sh.eig_cycles = 0;
   if (tid < m) { sh.alpha[tid] = ctl->alpha[tid]; sh.beta[tid] = ctl->beta[tid]; }
   __syncthreads();
@@ -1469,7 +1504,8 @@ __global__ void __launch_bounds__(LZ_BLOCK, 1) st_restart_kernel(
     ctl->sum_kn += kn;
     ctl->rot = 1;
     const bool bad = (*(volatile int*)P.status & ST_NONFINITE) != 0;
-    if (bad || sh.nconv >= P.num_desired || ctl->restarts >= P.max_restarts) ctl->stop = 1;
+    if (bad || sh.nconv >= P.num_desired || ctl->restarts >= P.max_restarts)
+      ctl->stop = ST_ENDED;
     P.ctl[2] = ctl->restarts;
     P.ctl[3] = ctl->breakdowns;
     P.ctl[4] = ctl->steps;
@@ -1539,14 +1575,17 @@ __global__ void __launch_bounds__(LZ_BLOCK) st_rotate_kernel(const __grid_consta
   if (threadIdx.x == 0) {
     ctl->i = kn;     // the next cycle starts from Q[:, kn]
     ctl->rot = 0;
+    ctl->breakdowns0 = __ldcg(&ctl->breakdowns);
+    ctl->steps0 = __ldcg(&ctl->steps);
+    ctl->sum_nv0 = __ldcg(&ctl->sum_nv);
     ctl->ticket[2] = 0u;
   }
 }
 
 // ---------------------------------------------------------------- wave path
 // A team-size problem (too large for one cluster, x of at most 160 KB) that has
-// the GPU's launches to itself runs the team kernel's arithmetic as four
-// ordinary launches per Lanczos step, like the stream path:
+// the GPU's launches to itself runs its first cycles as four ordinary launches
+// per Lanczos step, like the stream path, with the team kernel's arithmetic:
 //   A1  y = Op x, Q[:, i] = x
 //   A2  partial h1 = Q^T y
 //   B   q1 = y - Q h1, partial h2 = Q^T q1
@@ -1559,10 +1598,23 @@ __global__ void __launch_bounds__(LZ_BLOCK) st_rotate_kernel(const __grid_consta
 // vector, in B, from the other CTAs' shared memory).  So four times as many
 // SMs work, a step has four kernel boundaries where the team kernel has three
 // grid barriers of about 20k cycles, and the results are the same bits.
+// The host reads nothing back: a cycle's steps are bounded by the rule of the
+// restart, so all launches are enqueued at once, those past the loop's end
+// return, and a launch of the team kernel follows that continues from the
+// control block: after breakdowns (which take slots of their own; it runs their
+// cycle again from its start), or when there are more restarts than launches
+// planned (see WV_LAUNCHES).
 // ER n = 30,011 of degree 12, FP32, 10 restarts: 4.8 ms per call (14.4 as one
 // cooperative launch of 30 CTAs, 5.3 with A1 and A2 as one kernel).
 constexpr int WV_C = 4;                  // CTAs (tiles) per rank
 constexpr int WV_U = 8;                  // columns per CTA: c = j + 4 u
+
+// adds cycles to one of the control block's counters (CTA 0).  At a kernel's end, where
+// no fence or cluster barrier has to wait for the atomic.
+__device__ __forceinline__ void wv_count(StreamCtl* ctl, int what, long long cycles) {
+  if (blockIdx.x == 0 && threadIdx.x == 0)
+    atomicAdd(&ctl->cyc[what], (unsigned long long)cycles);
+}
 
 struct WvPlace { int rank, j, tile, t0, nt; };
 template <typename VT>
@@ -1744,6 +1796,7 @@ template <typename VT>
 __global__ void __launch_bounds__(LZ_BLOCK) wv_spmv_kernel(const __grid_constant__ TeamDesc<VT> P,
                                                            StreamCtl* ctl) {
   st_pdl_prologue();
+  const long long clk = clock64();
   int i, nv, buf;
   const int mode = st_mode(ctl, P.m, &i, &nv, &buf);
   if (mode == SM_SKIP) return;
@@ -1768,6 +1821,7 @@ __global__ void __launch_bounds__(LZ_BLOCK) wv_spmv_kernel(const __grid_constant
     case 16: wv_spmv_rows<VT, 16>(P, x, xscale, v); break;
     default: wv_spmv_rows<VT, 32>(P, x, xscale, v); break;
   }
+  wv_count(ctl, 1, clock64() - clk);
 }
 
 // A2
@@ -1776,6 +1830,7 @@ __global__ void __launch_bounds__(LZ_BLOCK) wv_dot_kernel(const __grid_constant_
                                                           StreamCtl* ctl) {
   st_pdl_prologue();
   __shared__ WvShared<VT> sh;
+  const long long clk = clock64();
   int i, nv, buf;
   if (st_mode(ctl, P.m, &i, &nv, &buf) == SM_SKIP) return;
   const WvPlace w = wv_place(P);
@@ -1788,6 +1843,7 @@ __global__ void __launch_bounds__(LZ_BLOCK) wv_dot_kernel(const __grid_constant_
     y[t] = (t < w.nt && row < P.n) ? __ldg(v + row) : (VT)0;
   }
   wv_dots(P, w, sh, nv, q, y, P.part);
+  wv_count(ctl, 1, clock64() - clk);
 }
 
 // B
@@ -1804,7 +1860,9 @@ __global__ void __launch_bounds__(LZ_BLOCK) wv_update_dot_kernel(
   VT* v = P.vbuf + (size_t)buf * P.ldv;
   WvRow<VT> r;
   r.load(P, row, in, nv, v);
+  const long long clk = clock64();
   wv_reduce(P.part, P.nctas, nv, sh);
+  const long long clk_red = clock64();
   if (blockIdx.x == 0 && tid < nv) ctl->h1[tid] = sh.h[tid];
   if (in) {
     const VT x = r.update(sh, nv);
@@ -1821,6 +1879,8 @@ __global__ void __launch_bounds__(LZ_BLOCK) wv_update_dot_kernel(
   }
   wv_dots(P, w, sh, nv, q, y, P.part + (size_t)MP1 * P.nctas);
   cl_sync();       // no CTA leaves while another reads its vector
+  wv_count(ctl, 0, clk_red - clk);
+  wv_count(ctl, 2, clock64() - clk_red);
 }
 
 // C; the last rank to finish advances the state (solver/lanczos.py:95-105, and the
@@ -1840,7 +1900,9 @@ __global__ void __launch_bounds__(LZ_BLOCK) wv_update_norm_kernel(
   VT* v = P.vbuf + (size_t)buf * P.ldv;
   WvRow<VT> r;
   r.load(P, row, in, nv, v);
+  const long long clk = clock64();
   wv_reduce(P.part + (size_t)MP1 * R, R, nv, sh);
+  const long long clk_red = clock64();
   if (in) {
     const VT x = r.update(sh, nv);
     v[row] = x;
@@ -1869,6 +1931,8 @@ __global__ void __launch_bounds__(LZ_BLOCK) wv_update_norm_kernel(
     part[w.rank] = s;
     __threadfence();
     sh.last = (atomicAdd(&ctl->ticket[1], 1u) == (unsigned)R - 1u) ? 1 : 0;
+    wv_count(ctl, 0, clk_red - clk);
+    wv_count(ctl, 3, clock64() - clk_red);
     if (sh.last) __threadfence();
   }
   __syncthreads();
@@ -2835,9 +2899,30 @@ constexpr size_t tm_dyn_max() {
 }
 static_assert(tm_dyn_max<double>() >= (size_t)LZ_XS_BYTES, "staged x must fit");
 
+// a problem's descriptor for R CTAs (or ranks), with its part of the workspace;
+// returns the workspace behind it
+template <typename VT>
+static char* fill_desc(TeamDesc<VT>& t, const LanczosProblem& p, int R, bool with_ctl) {
+  memset(&t, 0, sizeof(t));
+  t.n = p.n; t.ld = p.ld; t.ldv = vec_stride(p.n); t.m = p.m; t.num_desired = p.num_desired;
+  t.max_restarts = p.max_restarts; t.tol = p.tol;
+  t.lanes = lanczos_lanes(p.n, p.nnz);
+  t.nctas = R;
+  t.rowptr = p.rowptr; t.col = p.col; t.val = (const VT*)p.val;
+  t.nnz = p.nnz;
+  t.Q = (VT*)p.Q; t.Qw = t.Q; t.qts = LZ_BLOCK; t.qcs = p.ld;
+  t.alpha = p.alpha; t.beta = p.beta; t.ctl = p.ctl; t.status = p.status;
+  char* w = (char*)p.work;
+  t.vbuf = (VT*)w; w += align256(3 * (size_t)t.ldv * sizeof(VT));
+  t.part = (double*)w; w += part_bytes(R, with_ctl);
+  t.Ybuf = (double*)w; w += align256((size_t)MAXM * MAXM * sizeof(double));
+  t.bar = (unsigned int*)w; w += 256;
+  return w;
+}
+
 template <typename VT>
 static int run_typed(const DeviceInfo& di, const LanczosProblem* probs, int count,
-                     cudaStream_t stream) {
+                     cudaStream_t stream, StreamCtl* const* resume = nullptr) {
   const int occ = (sizeof(VT) == 8) ? di.lanczos_occ64 : di.lanczos_occ32;
   const int maxc = (di.sm_count > 4 ? di.sm_count - 2 : di.sm_count) * (occ > 0 ? occ : 1);
   for (int base = 0; base < count; base += MAX_TEAMS) {
@@ -2875,29 +2960,15 @@ static int run_typed(const DeviceInfo& di, const LanczosProblem* probs, int coun
         return -2;
       }
       TeamDesc<VT>& t = batch.t[i];
-      t.n = p.n; t.ld = p.ld; t.m = p.m; t.num_desired = p.num_desired;
-      t.max_restarts = p.max_restarts; t.tol = p.tol;
-      t.lanes = lanczos_lanes(p.n, p.nnz);
+      fill_desc(t, p, want[i], false);
       t.xsmem = ((size_t)p.n * sizeof(VT) <= (size_t)LZ_XS_BYTES) ? 1 : 0;
       if (t.xsmem && (size_t)p.n * sizeof(VT) > dyn) dyn = (size_t)p.n * sizeof(VT);
       t.first_cta = first;
-      t.nctas = want[i];
-      t.rowptr = p.rowptr; t.col = p.col; t.val = (const VT*)p.val;
-      t.nnz = p.nnz;
-      t.Q = (VT*)p.Q;
-      char* w = (char*)p.work;
-      t.ldv = vec_stride(p.n);
-      t.vbuf = (VT*)w; w += align256(3 * (size_t)t.ldv * sizeof(VT));
-      t.part = (double*)w; w += align256((size_t)3 * want[i] * MP1 * sizeof(double));
-      t.Ybuf = (double*)w; w += align256((size_t)MAXM * MAXM * sizeof(double));
-      t.bar = (unsigned int*)w; w += 256;
-      t.Qw = t.Q;
-      t.qts = LZ_BLOCK;
-      t.qcs = p.ld;
-      t.alpha = p.alpha; t.beta = p.beta; t.ctl = p.ctl; t.status = p.status;
+      t.resume = resume ? resume[base + i] : nullptr;
       first += want[i];
       if (cudaMemsetAsync(t.bar, 0, 2 * sizeof(unsigned int), stream) != cudaSuccess ||
-          cudaMemsetAsync(p.ctl, 0, 16 * sizeof(int), stream) != cudaSuccess) {
+          (!t.resume &&
+           cudaMemsetAsync(p.ctl, 0, 16 * sizeof(int), stream) != cudaSuccess)) {
         set_error("lanczos: memset failed");
         return -4;
       }
@@ -2947,8 +3018,7 @@ int lanczos_stream_occupancy(int prec) {
 // Whether a problem runs on the wave path: a team-size problem whose ranks hold at
 // most four tiles and whose workspace has room for the control block (six ranks; below
 // that only what a batch with a larger problem, or a cluster that cannot be had,
-// sends here), outside a stream capture (the loop state is read back once per
-// restart).
+// sends here), outside a stream capture (where a call stays one node).
 template <typename VT>
 static bool wave_fits(const LanczosProblem& p, int nctas, cudaStream_t stream) {
   if (p.m > MAXM || p.m < 1 || p.n < 1 || p.ld < p.n) return false;
@@ -2959,17 +3029,11 @@ static bool wave_fits(const LanczosProblem& p, int nctas, cudaStream_t stream) {
   return cs == cudaStreamCaptureStatusNone;
 }
 
-// Stream path of one problem (wave = 0), or its wave path over `wave` ranks.  The
-// host enqueues a cycle's steps (m - i of
-// them, one more after a breakdown), the restart and the rotation, then reads
-// the control block back once (a synchronisation of `stream`) to learn where
-// the next cycle starts and whether the loop has ended.  The loop state is
-// on the device, so a step that is not needed only returns.
 // a stream kernel launched with programmatic stream serialisation (see
 // st_pdl_prologue)
 template <typename... KArgs, typename... Args>
-static cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int cluster, size_t smem,
-                              cudaStream_t stream, Args... args) {
+static cudaError_t launch_pdl(void (*kernel)(KArgs...), bool early, int grid, int cluster,
+                              size_t smem, cudaStream_t stream, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3(LZ_BLOCK);
@@ -2977,7 +3041,7 @@ static cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int cluster, s
   cfg.stream = stream;
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[0].val.programmaticStreamSerializationAllowed = early ? 1 : 0;
   at[1].id = cudaLaunchAttributeClusterDimension;
   at[1].val.clusterDim.x = (unsigned)cluster;
   at[1].val.clusterDim.y = 1;
@@ -2987,9 +3051,13 @@ static cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int cluster, s
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+// Stream path of one problem.  The host enqueues a cycle's steps (m - i of
+// them, one more after a breakdown), the restart and the rotation, then reads
+// the control block back once (a synchronisation of `stream`) to learn where
+// the next cycle starts and whether the loop has ended.  The loop state is
+// on the device, so a step that is not needed only returns.
 template <typename VT>
-static int run_stream(const DeviceInfo& di, const LanczosProblem& p, cudaStream_t stream,
-                      int wave = 0) {
+static int run_stream(const DeviceInfo& di, const LanczosProblem& p, cudaStream_t stream) {
   if (p.m > MAXM || p.m < 1 || p.n < 1 || p.ld < p.n) {
     set_error("lanczos: unsupported sizes n=%d ld=%d m=%d (m must be in [1, %d])", p.n, p.ld,
               p.m, MAXM);
@@ -3002,13 +3070,13 @@ static int run_stream(const DeviceInfo& di, const LanczosProblem& p, cudaStream_
     return -2;
   }
   // the stream path's kernels take four rows of a column as 16-byte words
-  if (!wave && (((uintptr_t)p.Q | (size_t)p.ld * sizeof(VT)) & 15) != 0) {
+  if ((((uintptr_t)p.Q | (size_t)p.ld * sizeof(VT)) & 15) != 0) {
     set_error("lanczos: n=%d rows need Q and its columns (ld=%d) on 16-byte boundaries", p.n, p.ld);
     return -2;
   }
   const int ntiles = (p.n + LZ_BLOCK - 1) / LZ_BLOCK;
   // partials per pass
-  const int G = wave ? wave : lanczos_team_size(di, p.n, sizeof(VT) == 8 ? 64 : 32, true);
+  const int G = lanczos_team_size(di, p.n, sizeof(VT) == 8 ? 64 : 32, true);
   const int* occ = stream_occ<VT>();
   // each kernel: at most one wave, and every CTA the same number of row
   // chunks (A2 and C use 4 rows per thread, B 8 bytes per thread), so no
@@ -3018,46 +3086,29 @@ static int run_stream(const DeviceInfo& di, const LanczosProblem& p, cudaStream_
     const int rows = (j == 1) ? (8 / (int)sizeof(VT)) * LZ_BLOCK : (j == 3 ? LZ_BLOCK : ST_ROWS);
     const int nch = (p.n + rows - 1) / rows;
     int gmax = di.sm_count * occ[j];
-    if (gmax > G && !wave) gmax = G;
+    if (gmax > G) gmax = G;
     if (gmax < 1) gmax = 1;
     const int per = (nch + gmax - 1) / gmax;
     g[j] = (nch + per - 1) / per;
     if (g[j] < 1) g[j] = 1;
   }
   TeamDesc<VT> t;
-  memset(&t, 0, sizeof(t));
-  t.n = p.n; t.ld = p.ld; t.m = p.m; t.num_desired = p.num_desired;
-  t.max_restarts = p.max_restarts; t.tol = p.tol;
-  t.lanes = lanczos_lanes(p.n, p.nnz);
-  t.first_cta = 0; t.nctas = G; t.xsmem = 0; t.nnz = p.nnz;
-  t.rowptr = p.rowptr; t.col = p.col; t.val = (const VT*)p.val;
-  t.Q = (VT*)p.Q; t.Qw = t.Q; t.qts = LZ_BLOCK; t.qcs = p.ld;
-  char* w = (char*)p.work;
-  t.ldv = vec_stride(p.n);
-  t.vbuf = (VT*)w; w += align256(3 * (size_t)t.ldv * sizeof(VT));
-  t.part = (double*)w;
-  StreamCtl* ctl = (StreamCtl*)(w + ctl_offset(G));
-  w += part_bytes(G, !wave);
-  t.Ybuf = (double*)w; w += align256((size_t)MAXM * MAXM * sizeof(double));
-  t.bar = nullptr;
-  w += 256;
-  t.alpha = p.alpha; t.beta = p.beta; t.ctl = p.ctl; t.status = p.status;
-  if (!wave) {
-    const int ns = (p.n + 31) / 32;
-    t.wcap = sell_wcap(p.n, p.nnz);
-    if ((long long)ns * 32 * t.wcap > 0x7fffffffLL) {
-      set_error("lanczos: n=%d is too large for the stream path's operator layout", p.n);
-      return -2;
-    }
-    t.sl_ptr = (int*)w; w += align256((size_t)(ns + 1) * sizeof(int));
-    t.sl_row = (unsigned char*)w; w += align256((size_t)ns * 32);
-    t.sl_col = (int*)w; w += align256((size_t)ns * 32 * t.wcap * sizeof(int));
-    t.sl_val = (VT*)w;
-    st_sell_order_kernel<VT><<<ntiles, LZ_BLOCK, 0, stream>>>(t);
-    st_sell_scan_kernel<<<1, 1024, 0, stream>>>(ns, t.sl_ptr);
-    st_sell_fill_kernel<VT><<<ntiles, LZ_BLOCK, 0, stream>>>(t);
-    t_launches += 3;
+  char* w = fill_desc(t, p, G, true);
+  StreamCtl* ctl = (StreamCtl*)((char*)t.part + ctl_offset(G));
+  const int ns = (p.n + 31) / 32;
+  t.wcap = sell_wcap(p.n, p.nnz);
+  if ((long long)ns * 32 * t.wcap > 0x7fffffffLL) {
+    set_error("lanczos: n=%d is too large for the stream path's operator layout", p.n);
+    return -2;
   }
+  t.sl_ptr = (int*)w; w += align256((size_t)(ns + 1) * sizeof(int));
+  t.sl_row = (unsigned char*)w; w += align256((size_t)ns * 32);
+  t.sl_col = (int*)w; w += align256((size_t)ns * 32 * t.wcap * sizeof(int));
+  t.sl_val = (VT*)w;
+  st_sell_order_kernel<VT><<<ntiles, LZ_BLOCK, 0, stream>>>(t);
+  st_sell_scan_kernel<<<1, 1024, 0, stream>>>(ns, t.sl_ptr);
+  st_sell_fill_kernel<VT><<<ntiles, LZ_BLOCK, 0, stream>>>(t);
+  t_launches += 3;
   if (cudaMemsetAsync(ctl, 0, sizeof(StreamCtl), stream) != cudaSuccess ||
       cudaMemsetAsync(p.ctl, 0, 16 * sizeof(int), stream) != cudaSuccess) {
     set_error("lanczos: memset failed");
@@ -3074,26 +3125,16 @@ static int run_stream(const DeviceInfo& di, const LanczosProblem& p, cudaStream_
     const int slots = (p.m - i_host) + (bd_host ? 1 : 0);
     cudaError_t e = cudaSuccess;
     for (int j = 0; j < slots && e == cudaSuccess; ++j) {
-      if (wave) {
-        e = launch_pdl(wv_spmv_kernel<VT>, (p.n + WV_ROWS - 1) / WV_ROWS, 1, 0, stream, t, ctl);
-        if (e == cudaSuccess)
-          e = launch_pdl(wv_dot_kernel<VT>, WV_C * wave, 1, 0, stream, t, ctl);
-        if (e == cudaSuccess)
-          e = launch_pdl(wv_update_dot_kernel<VT>, WV_C * wave, WV_C, 0, stream, t, ctl);
-        if (e == cudaSuccess)
-          e = launch_pdl(wv_update_norm_kernel<VT>, WV_C * wave, WV_C, 0, stream, t, ctl);
-        continue;
-      }
-      e = launch_pdl(st_sell_spmv_kernel<VT>, ntiles, 1, 0, stream, t, ctl);
+      e = launch_pdl(st_sell_spmv_kernel<VT>, true, ntiles, 1, 0, stream, t, ctl);
       if (e == cudaSuccess)
-        e = launch_pdl(st_dot_kernel<VT>, DOT_G * g[0], 1, 0, stream, t, ctl);
+        e = launch_pdl(st_dot_kernel<VT>, true, DOT_G * g[0], 1, 0, stream, t, ctl);
       if (e == cudaSuccess)
-        e = launch_pdl(st_update_dot1_kernel<VT>, g[1], 1, st_sacc_bytes<VT>(), stream, t, ctl);
+        e = launch_pdl(st_update_dot1_kernel<VT>, true, g[1], 1, st_sacc_bytes<VT>(), stream, t, ctl);
       if (e == cudaSuccess)
-        e = launch_pdl(st_update_norm_kernel<VT>, g[2], 1, 0, stream, t, ctl);
+        e = launch_pdl(st_update_norm_kernel<VT>, true, g[2], 1, 0, stream, t, ctl);
     }
-    if (e == cudaSuccess) e = launch_pdl(st_restart_kernel<VT>, 1, 1, 0, stream, t, ctl);
-    if (e == cudaSuccess) e = launch_pdl(st_rotate_kernel<VT>, g[3], 1, 0, stream, t, ctl);
+    if (e == cudaSuccess) e = launch_pdl(st_restart_kernel<VT>, true, 1, 1, 0, stream, t, ctl);
+    if (e == cudaSuccess) e = launch_pdl(st_rotate_kernel<VT>, true, g[3], 1, 0, stream, t, ctl);
     t_launches += 4 * slots + 2;
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) {
@@ -3110,6 +3151,63 @@ static int run_stream(const DeviceInfo& di, const LanczosProblem& p, cudaStream_
     i_host = h.i;
     bd_host = h.bd;
   }
+  return 0;
+}
+
+// Most launches a call enqueues for the wave path.  A stream's queue holds 1,024
+// launches (1,020 behind a waiting stream return in 8 ms, 1,100 when it goes on), and a
+// call that stays below returns at once however busy its stream is.  It is room for 18
+// cycles of 32 vectors, or for 8 of each of two problems.
+constexpr int WV_LAUNCHES = 980;
+
+// Wave path of one problem over R ranks: enqueues the launches of its first cycles, at
+// most `budget` of them.  *resume receives the control block from which the team
+// kernel continues (untouched if no cycle is enqueued).  After a restart at most
+// delta = min(m - num_desired, 2 m / 5) vectors are dropped (restart_select), so a
+// cycle takes at most that many steps, the first one m.
+// The rotation and the next cycle's first launch wait for the kernel before them to
+// end: started early they and, each started by the one before it, the next step's
+// kernels would hold the SMs through the one-CTA restart.  Eight streams at once: 13.3
+// ms with n = 30,011 in FP32 (16.0 with both early, 13.8 with the rotation early), 17.9
+// with n = 15,000 in FP64 (27, 19.2); one alone 5.0 either way, 7.5 (8.0, 7.8).
+template <typename VT>
+static int enqueue_wave(const LanczosProblem& p, int R, int budget, cudaStream_t stream,
+                        StreamCtl** resume) {
+  const int more = p.m - p.num_desired < 2 * p.m / 5 ? p.m - p.num_desired : 2 * p.m / 5;
+  if (p.max_restarts < 1 || p.num_desired < 1 || more < 0 || 4 * p.m + 2 > budget) return 0;
+  TeamDesc<VT> t;
+  fill_desc(t, p, R, false);
+  StreamCtl* ctl = (StreamCtl*)((char*)t.part + ctl_offset(R));
+  t.resume = ctl;
+  if (cudaMemsetAsync(ctl, 0, sizeof(StreamCtl), stream) != cudaSuccess ||
+      cudaMemsetAsync(p.ctl, 0, 16 * sizeof(int), stream) != cudaSuccess) {
+    set_error("lanczos: memset failed");
+    return -4;
+  }
+  const int ntiles = (p.n + LZ_BLOCK - 1) / LZ_BLOCK;
+  int used = 0;
+  for (int c = 0; c < p.max_restarts; ++c) {
+    const int slots = c ? more : p.m;
+    if (used + 4 * slots + 2 > budget) break;
+    cudaError_t e = cudaSuccess;
+    for (int j = 0; j < slots && e == cudaSuccess; ++j) {
+      e = launch_pdl(wv_spmv_kernel<VT>, j > 0, (p.n + WV_ROWS - 1) / WV_ROWS, 1, 0, stream, t, ctl);
+      if (e == cudaSuccess) e = launch_pdl(wv_dot_kernel<VT>, true, WV_C * R, 1, 0, stream, t, ctl);
+      if (e == cudaSuccess)
+        e = launch_pdl(wv_update_dot_kernel<VT>, true, WV_C * R, WV_C, 0, stream, t, ctl);
+      if (e == cudaSuccess)
+        e = launch_pdl(wv_update_norm_kernel<VT>, true, WV_C * R, WV_C, 0, stream, t, ctl);
+    }
+    if (e == cudaSuccess) e = launch_pdl(st_restart_kernel<VT>, true, 1, 1, 0, stream, t, ctl);
+    if (e == cudaSuccess) e = launch_pdl(st_rotate_kernel<VT>, false, ntiles, 1, 0, stream, t, ctl);
+    used += 4 * slots + 2;
+    if (e != cudaSuccess) {
+      set_error("lanczos: wave-path launch failed: %s", cudaGetErrorString(e));
+      return -5;
+    }
+  }
+  t_launches += used;
+  *resume = ctl;
   return 0;
 }
 
@@ -3132,29 +3230,25 @@ static int run_noncluster(const DeviceInfo& di, const LanczosProblem* probs, int
       }
     }
     if (nt) {
-      // one or two team-size problems: one after another on the wave path, with the
-      // team sizes, and so the results, of the shared launch.  ms for one, two,
-      // three and four on it / in a shared launch, whose time hardly depends on
-      // their number: FP32 n = 30,011 4.9, 9.7, 14.6, 19.0 / 14.5 - 15.1; FP64
-      // n = 20,000 8.7, 17.4, 25.8, 34.5 / 22.3 - 22.7, n = 12,100 8.2, 16.2, 24.0,
-      // 31.8 / 20.0 - 20.2.  More, or teams shrunk to fit one launch, share it
+      // one or two team-size problems: their cycles one after another on the wave
+      // path, with the team sizes, and so the results, of the shared launch that
+      // follows.  ms for one, two, three and four on it alone / in a shared launch,
+      // whose time hardly depends on their number: FP32 n = 30,011 5.0, 10.8, 14.6, 19.0 /
+      // 14.8; FP64 n = 20,000 8.4, 17.8, 25.8, 34.5 / 21.5.  More, or teams shrunk to fit one launch, share it
       const int occ = (sizeof(VT) == 8) ? di.lanczos_occ64 : di.lanczos_occ32;
       const int maxc = (di.sm_count > 4 ? di.sm_count - 2 : di.sm_count) * (occ > 0 ? occ : 1);
       int want[MAX_TEAMS], total = 0;
-      bool wave = nt <= 2;
+      StreamCtl* resume[MAX_TEAMS] = {};
       for (int i = 0; i < nt; ++i) {
         want[i] = lanczos_team_size(di, team[i].n, sizeof(VT) == 8 ? 64 : 32);
         total += want[i];
-        wave = wave && wave_fits<VT>(team[i], want[i], stream);
       }
-      if (wave && total <= maxc) {
-        for (int i = 0; i < nt; ++i) {
-          const int rc = run_stream<VT>(di, team[i], stream, want[i]);
+      for (int i = 0; i < nt && nt <= 2 && total <= maxc; ++i)
+        if (wave_fits<VT>(team[i], want[i], stream)) {
+          const int rc = enqueue_wave<VT>(team[i], want[i], WV_LAUNCHES / nt, stream, &resume[i]);
           if (rc) return rc;
         }
-        continue;
-      }
-      const int rc = run_typed<VT>(di, team, nt, stream);
+      const int rc = run_typed<VT>(di, team, nt, stream, resume);
       if (rc) return rc;
     }
   }
