@@ -916,13 +916,54 @@ __device__ __forceinline__ int st_mode_of(int4 a, int4 b, int m, int* i, int* nv
   if (ii < m) { *nv = ii + 1; *buf = cur; return SM_STEP; }
   return SM_SKIP;
 }
-// Reads of the control block go through the read-only (L1) path: within a
-// kernel only its last CTA writes the block, after every other CTA has
-// finished, and the L1 caches start empty at each launch.  (Through L2 alone,
-// every warp of every CTA would queue on the same L2 line.)
+// What the solve's own kernels write (the control block, the basis, the work vectors)
+// is read by ordinary loads (ld_seen) after st_pdl_prologue, which makes the writes of the
+// kernels before visible: an early-started kernel's life overlaps theirs, and the
+// read-only path (__ldg) holds only for data that no one writes during it.  The
+// ordinary loads may use the L1 as well.  (Through L2 alone, every warp of every
+// CTA would queue on the control block's line.)  They are volatile asm without a
+// memory clobber: nothing moves them before the prologue or a barrier, and the
+// compiler may issue them ahead of stores to other vectors, as it does with __ldg.
+__device__ __forceinline__ float ld_seen(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double ld_seen(const double* p) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ int ld_seen(const int* p) {
+  int v;
+  asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float2 ld_seen(const float2* p) {
+  float2 v;
+  asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float4 ld_seen(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double2 ld_seen(const double2* p) {
+  double2 v;
+  asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ int4 ld_seen(const int4* p) {
+  int4 v;
+  asm volatile("ld.global.v4.s32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
 __device__ __forceinline__ int st_mode(const StreamCtl* c, int m, int* i, int* nv, int* buf) {
   const int4* p = (const int4*)c;
-  return st_mode_of(__ldg(p), __ldg(p + 1), m, i, nv, buf);
+  return st_mode_of(ld_seen(p), ld_seen(p + 1), m, i, nv, buf);
 }
 
 // Programmatic dependent launch: each stream kernel lets the next one in the
@@ -995,26 +1036,25 @@ __device__ __forceinline__ void st_reduce(const double* part, int R, int nv, SH&
 // ---- vector helpers of the Q-streaming kernels ----
 // 4 consecutive rows of a column (16-byte aligned: ld is a multiple of 32 and
 // the first row a multiple of 4); rows at or past n read as 0.  The basis is
-// read through the read-only path (no stream kernel writes a column it
-// reads); the work vectors, which B and C update, through L2.
+// read through the L1, the work vectors, which B and C update, through L2.
 template <typename VT> struct Row4 { VT v[4]; };
-template <typename VT, bool RO = true>
+template <typename VT, bool L1 = true>
 __device__ __forceinline__ Row4<VT> ld4(const VT* p, int r4, int n) {
   Row4<VT> o;
   if (r4 + 4 <= n) {
     if constexpr (sizeof(VT) == 4) {
-      const float4 a = RO ? __ldg((const float4*)(p + r4)) : __ldcg((const float4*)(p + r4));
+      const float4 a = L1 ? ld_seen((const float4*)(p + r4)) : __ldcg((const float4*)(p + r4));
       o.v[0] = a.x; o.v[1] = a.y; o.v[2] = a.z; o.v[3] = a.w;
     } else {
-      const double2 a = RO ? __ldg((const double2*)(p + r4)) : __ldcg((const double2*)(p + r4));
+      const double2 a = L1 ? ld_seen((const double2*)(p + r4)) : __ldcg((const double2*)(p + r4));
       const double2 b =
-          RO ? __ldg((const double2*)(p + r4 + 2)) : __ldcg((const double2*)(p + r4 + 2));
+          L1 ? ld_seen((const double2*)(p + r4 + 2)) : __ldcg((const double2*)(p + r4 + 2));
       o.v[0] = a.x; o.v[1] = a.y; o.v[2] = b.x; o.v[3] = b.y;
     }
   } else {
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-      o.v[j] = (r4 + j < n) ? (RO ? __ldg(p + r4 + j) : __ldcg(p + r4 + j)) : (VT)0;
+      o.v[j] = (r4 + j < n) ? (L1 ? ld_seen(p + r4 + j) : __ldcg(p + r4 + j)) : (VT)0;
   }
   return o;
 }
@@ -1174,8 +1214,7 @@ __global__ void __launch_bounds__(LZ_BLOCK) st_sell_fill_kernel(
 // gathers, all in flight at once.  Step: vbuf[cur] = Op x with x = (i == k ?
 // Q[:, k] : vbuf[cur ^ 1] / beta), and Q[:, i] = x when i > k.  Breakdown:
 // vbuf[cur ^ 1] = a Gaussian vector keyed by i (the replacement of
-// solver/lanczos.py:107-117).  x is not written here, so it is gathered
-// through the read-only (L1) path.
+// solver/lanczos.py:107-117).  x is gathered through the L1.
 template <typename VT>
 __global__ void __launch_bounds__(LZ_BLOCK, 8) st_sell_spmv_kernel(
     const __grid_constant__ TeamDesc<VT> P, StreamCtl* ctl) {
@@ -1187,8 +1226,8 @@ __global__ void __launch_bounds__(LZ_BLOCK, 8) st_sell_spmv_kernel(
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int s = blockIdx.x * (LZ_BLOCK / 32) + warp;
   const bool has = s < (P.n + 31) / 32;
-  const int4 ca = __ldg((const int4*)ctl), cb = __ldg((const int4*)ctl + 1);
-  const double invb_d = __ldg(&ctl->invb);
+  const int4 ca = ld_seen((const int4*)ctl), cb = ld_seen((const int4*)ctl + 1);
+  const double invb_d = ld_seen(&ctl->invb);
   const int sb = has ? __ldg(P.sl_ptr + s) : 0;
   const int width = has ? (__ldg(P.sl_ptr + s + 1) - sb) >> 5 : 0;
   const int lr = has ? (int)__ldg(P.sl_row + 32 * s + lane) : 0;
@@ -1204,8 +1243,8 @@ __global__ void __launch_bounds__(LZ_BLOCK, 8) st_sell_spmv_kernel(
   const int k = ca.y;
   const bool wq = i > k;
   const VT xscale = wq ? (VT)invb_d : (VT)1;
-  const VT* __restrict__ x = wq ? P.vbuf + (size_t)(buf ^ 1) * P.ldv : P.Q + (size_t)k * ld;
-  const VT xrow = (wq && row < P.n) ? __ldg(x + row) : (VT)0;
+  const VT* x = wq ? P.vbuf + (size_t)(buf ^ 1) * P.ldv : P.Q + (size_t)k * ld;
+  const VT xrow = (wq && row < P.n) ? ld_seen(x + row) : (VT)0;
   if (has) {
     const int* cp = P.sl_col + sb + lane;
     const VT* vp = P.sl_val + sb + lane;
@@ -1218,17 +1257,17 @@ __global__ void __launch_bounds__(LZ_BLOCK, 8) st_sell_spmv_kernel(
       v[u] = (u < width) ? __ldg(vp + 32 * u) : (VT)0;
     }
 #pragma unroll
-    for (int u = 0; u < PF; ++u) xv[u] = (u < width) ? __ldg(x + c[u]) : (VT)0;
+    for (int u = 0; u < PF; ++u) xv[u] = (u < width) ? ld_seen(x + c[u]) : (VT)0;
     AT acc = (AT)0;
 #pragma unroll
     for (int u = 0; u < PF; ++u) acc += (AT)v[u] * (AT)xv[u];
-    for (int u = PF; u < width; ++u) acc += (AT)__ldg(vp + 32 * u) * (AT)__ldg(x + __ldg(cp + 32 * u));
+    for (int u = PF; u < width; ++u) acc += (AT)__ldg(vp + 32 * u) * (AT)ld_seen(x + __ldg(cp + 32 * u));
     const int r = w0 + lr;
     if (r < P.n && width == P.wcap) {
       // the rest of a row longer than the slice capacity
       const int e = P.rowptr[r + 1];
       for (int q = P.rowptr[r] + P.wcap; q < e; ++q)
-        acc += (AT)__ldg(P.val + q) * (AT)__ldg(x + __ldg(P.col + q));
+        acc += (AT)__ldg(P.val + q) * (AT)ld_seen(x + __ldg(P.col + q));
     }
     ys[lr] = (VT)acc;
   }
@@ -1348,7 +1387,7 @@ __global__ void __launch_bounds__(LZ_BLOCK, 2) st_update_dot1_kernel(
   if (mode == SM_SKIP) return;
   const int R = gridDim.x, n = P.n;
   const size_t ld = (size_t)P.ld;
-  for (int c = threadIdx.x; c < nv; c += LZ_BLOCK) sh.hv[c] = (VT)__ldg(&ctl->h1[c]);
+  for (int c = threadIdx.x; c < nv; c += LZ_BLOCK) sh.hv[c] = (VT)ld_seen(&ctl->h1[c]);
   extern __shared__ __align__(16) unsigned char st_dyn[];
   AT* sacc = (AT*)st_dyn;
   for (int c = 0; c < nv; ++c) sacc[c * LZ_BLOCK + threadIdx.x] = (AT)0;
@@ -1368,13 +1407,13 @@ __global__ void __launch_bounds__(LZ_BLOCK, 2) st_update_dot1_kernel(
         const VT* src = P.Q + (size_t)c * ld + r0;
         if constexpr (RW == 2) {
           if (full) {
-            const float2 a = __ldg((const float2*)src);
+            const float2 a = ld_seen((const float2*)src);
             q[c][0] = a.x; q[c][1] = a.y;
           } else {
-            q[c][0] = __ldg(src); q[c][1] = (VT)0;
+            q[c][0] = ld_seen(src); q[c][1] = (VT)0;
           }
         } else {
-          q[c][0] = __ldg(src);
+          q[c][0] = ld_seen(src);
         }
       }
     VT x[RW], s[RW];
@@ -1427,7 +1466,7 @@ __global__ void __launch_bounds__(LZ_BLOCK) st_update_norm_kernel(
   if (mode == SM_SKIP) return;
   const int R = gridDim.x;
   const size_t ld = (size_t)P.ld;
-  for (int c = threadIdx.x; c < nv; c += LZ_BLOCK) sh.hv[c] = (VT)__ldg(&ctl->h2[c]);
+  for (int c = threadIdx.x; c < nv; c += LZ_BLOCK) sh.hv[c] = (VT)ld_seen(&ctl->h2[c]);
   __syncthreads();
   int c0, c1;
   st_chunks(P.n, &c0, &c1);
@@ -1523,12 +1562,12 @@ __global__ void __launch_bounds__(LZ_BLOCK) st_rotate_kernel(const __grid_consta
                                                               StreamCtl* ctl) {
   st_pdl_prologue();
   __shared__ StShared<VT> sh;
-  if (!__ldg(&ctl->rot)) return;
-  const int m = P.m, kn = __ldg(&ctl->k);
-  const bool stepped = __ldg(&ctl->stepped) != 0;
-  const VT invb = (VT)__ldg(&ctl->invb);
+  if (!ld_seen(&ctl->rot)) return;
+  const int m = P.m, kn = ld_seen(&ctl->k);
+  const bool stepped = ld_seen(&ctl->stepped) != 0;
+  const VT invb = (VT)ld_seen(&ctl->invb);
   const size_t ld = (size_t)P.ld;
-  const VT* lastv = P.vbuf + (size_t)(__ldg(&ctl->cur) ^ 1) * P.ldv;
+  const VT* lastv = P.vbuf + (size_t)(ld_seen(&ctl->cur) ^ 1) * P.ldv;
   for (int e = threadIdx.x; e < m * MAXM; e += LZ_BLOCK) {
     const int j = e / MAXM, c = e - j * MAXM;
     sh.u.Ys[e] = (c < kn) ? (VT)__ldcg(P.Ybuf + j * m + c) : (VT)0;
@@ -1686,7 +1725,7 @@ __device__ __forceinline__ void wv_load(const TeamDesc<VT>& P, const WvPlace& w,
 #pragma unroll
     for (int u = 0; u < WV_U; ++u) {
       const int c = w.j + WV_C * u;
-      q[t][u] = (in && c < nv) ? __ldg(P.Q + (size_t)c * P.ld + row) : (VT)0;
+      q[t][u] = (in && c < nv) ? ld_seen(P.Q + (size_t)c * P.ld + row) : (VT)0;
     }
   }
 }
@@ -1742,7 +1781,7 @@ struct WvRow {
     x = in ? __ldcg(v + row) : (VT)0;
 #pragma unroll
     for (int c = 0; c < MAXM; ++c)
-      q[c] = (in && c < nv) ? __ldg(P.Q + (size_t)c * P.ld + row) : (VT)0;
+      q[c] = (in && c < nv) ? ld_seen(P.Q + (size_t)c * P.ld + row) : (VT)0;
   }
   __device__ __forceinline__ VT update(const WvShared<VT>& sh, int nv) const {
     VT s = (VT)0;
@@ -1780,12 +1819,12 @@ __device__ __forceinline__ void wv_spmv_rows(const TeamDesc<VT>& P, const VT* x,
     if (pb[q] < pe[q]) { c0[q] = __ldg(P.col + pb[q]); v0[q] = __ldg(P.val + pb[q]); }
   }
 #pragma unroll
-  for (int q = 0; q < NP; ++q) x0[q] = __ldg(x + c0[q]);
+  for (int q = 0; q < NP; ++q) x0[q] = ld_seen(x + c0[q]);
 #pragma unroll
   for (int q = 0; q < NP; ++q) {
     AT s = (AT)v0[q] * (AT)x0[q];
     for (int p = pb[q] + L; p < pe[q]; p += L)
-      s += (AT)__ldg(P.val + p) * (AT)__ldg(x + __ldg(P.col + p));
+      s += (AT)__ldg(P.val + p) * (AT)ld_seen(x + __ldg(P.col + p));
 #pragma unroll
     for (int o = L >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     const int lr = q * GPP + g;
@@ -1808,11 +1847,11 @@ __global__ void __launch_bounds__(LZ_BLOCK) wv_spmv_kernel(const __grid_constant
     if (own) v[row] = (VT)hash_normal((uint64_t)i, (uint64_t)row);
     return;
   }
-  const int k = __ldg(&ctl->k);
+  const int k = ld_seen(&ctl->k);
   const bool wq = i > k;
   const VT* x = wq ? P.vbuf + (size_t)(buf ^ 1) * P.ldv : P.Q + (size_t)k * ld;
-  const VT xscale = wq ? (VT)__ldg(&ctl->invb) : (VT)1;
-  if (wq && own) P.Q[(size_t)i * ld + row] = __ldg(x + row) * xscale;
+  const VT xscale = wq ? (VT)ld_seen(&ctl->invb) : (VT)1;
+  if (wq && own) P.Q[(size_t)i * ld + row] = ld_seen(x + row) * xscale;
   switch (P.lanes) {
     case 1: wv_spmv_rows<VT, 1>(P, x, xscale, v); break;
     case 2: wv_spmv_rows<VT, 2>(P, x, xscale, v); break;
@@ -1840,7 +1879,7 @@ __global__ void __launch_bounds__(LZ_BLOCK) wv_dot_kernel(const __grid_constant_
 #pragma unroll
   for (int t = 0; t < WV_C; ++t) {
     const int row = (w.t0 + t) * LZ_BLOCK + threadIdx.x;
-    y[t] = (t < w.nt && row < P.n) ? __ldg(v + row) : (VT)0;
+    y[t] = (t < w.nt && row < P.n) ? ld_seen(v + row) : (VT)0;
   }
   wv_dots(P, w, sh, nv, q, y, P.part);
   wv_count(ctl, 1, clock64() - clk);
