@@ -18,11 +18,14 @@ namespace usbs {
 // warp.  On return w[0..n-1] holds the eigenvalues in ascending order and
 // Z (row-major, ldz) the eigenvectors as columns.  A is destroyed.  Returns
 // false if the QR iteration did not converge in 30 n sweeps.  n <= 32.
+// VECTORS = false: the eigenvalues alone, by the same arithmetic (Z is not used).
+template <bool VECTORS = true>
 __device__ inline bool warp_syev(double* A, int lda, int n, double* w, double* Z, int ldz) {
   const int lane = threadIdx.x & 31;
   // Z = I
-  for (int j = 0; j < n; ++j)
-    if (lane < n) Z[lane * ldz + j] = (lane == j) ? 1.0 : 0.0;
+  if (VECTORS)
+    for (int j = 0; j < n; ++j)
+      if (lane < n) Z[lane * ldz + j] = (lane == j) ? 1.0 : 0.0;
   __syncwarp();
   // ---- Householder tridiagonalisation: A <- H A H, Z <- Z H ----
   for (int j = 0; j + 2 < n; ++j) {
@@ -58,7 +61,7 @@ __device__ inline bool warp_syev(double* A, int lda, int n, double* w, double* Z
     // Z <- Z (I - beta v v^T): row i of Z: z_i -= beta (z_i . v) v^T, the rows'
     // dots 16 at a time by a butterfly whose payload halves (lanes 2 i and
     // 2 i + 1 end with row i's, summed as by a warp sum)
-    for (int i0 = 0; i0 < n; i0 += 16) {
+    for (int i0 = 0; VECTORS && i0 < n; i0 += 16) {
       double zr[16], x[16];
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
@@ -149,7 +152,7 @@ __device__ inline bool warp_syev(double* A, int lda, int n, double* w, double* Z
         if (k + 1 < hi) A[(k + 2) * lda + k + 1] = c * f;
       }
       // rotate eigenvector columns k, k+1: (Z P^T)
-      if (lane < n) {
+      if (VECTORS && lane < n) {
         double zk = Z[lane * ldz + k], zk1 = Z[lane * ldz + k + 1];
         Z[lane * ldz + k] = c * zk + s * zk1;
         Z[lane * ldz + k + 1] = -s * zk + c * zk1;
@@ -168,7 +171,7 @@ __device__ inline bool warp_syev(double* A, int lda, int n, double* w, double* Z
     if (kmin != i) {
       __syncwarp();
       double di = d[i];
-      if (lane < n) {
+      if (VECTORS && lane < n) {
         double t = Z[lane * ldz + i];
         Z[lane * ldz + i] = Z[lane * ldz + kmin];
         Z[lane * ldz + kmin] = t;

@@ -145,61 +145,30 @@ __global__ void __launch_bounds__(RD_RED) rd_reduce_kernel(int E, int nblocks,
   if (e < E && ch == 0) gsum[e] = a;
 }
 
-// one CTA: rho from the largest eigenvalue of P^T P, then warp 0 forms L, M^T M
-// and its eigen-decomposition, T and Lambda (see the file comment).  The largest
-// eigenvalue alone comes from the FP32 Jacobi refined to FP64 by two
-// Ogita-Aishima steps (on the matrix scaled by a power of two); the
-// decomposition of M^T M keeps the QR iteration, whose vectors' signs are the
-// result's.  Bound by the QR iteration's chain of FP64 instructions on one warp: 297 us
-// at s = 10 (593 with both decompositions by QR and the partials summed here).
+// one CTA: warp 0 forms rho from the largest eigenvalue of P^T P, L, M^T M and its
+// eigen-decomposition, T and Lambda (see the file comment).  Bound by the two QR
+// iterations' chains of FP64 instructions on one warp, of which the first needs the
+// eigenvalues alone.
 __global__ void __launch_bounds__(RD_BLOCK) rd_small_kernel(int n, int s, double eps,
                                                             const double* __restrict__ gsum,
                                                             double* __restrict__ small) {
   __shared__ double G[3 * RD_MAXS * RD_MAXS];
   __shared__ double A[RD_MAXS * RD_LD], Lm[RD_MAXS * RD_LD], K[RD_MAXS * RD_LD];
-  __shared__ double Z[RD_MAXS * RD_LD], X[RD_MAXS * RD_LD], w[RD_MAXS];
-  __shared__ float wf[RD_MAXS], redf[2];
-  __shared__ unsigned emax;
+  __shared__ double Z[RD_MAXS * RD_LD], w[RD_MAXS];
   const int tid = threadIdx.x, lane = tid & 31, s2 = s * s, E = 3 * s2;
-  if (tid == 0) emax = 0u;
+  for (int e = tid; e < E; e += RD_BLOCK) G[e] = gsum[e];
   __syncthreads();
-  for (int e = tid; e < E; e += RD_BLOCK) {
-    const double g = gsum[e];
-    G[e] = g;
-    if (e < s2) atomicMax(&emax, (unsigned)((__double_as_longlong(g) >> 52) & 0x7ff));
-  }
-  __syncthreads();
-  bool conv = true;
-  double lmax;
-  {
-    // P^T P scaled to entries below 2 (exact, but for entries that underflow)
-    const int sh = (emax == 0u || emax == 0x7ffu) ? 0 : 1023 - (int)emax;
-    const double f = scalbn(1.0, sh);
-    float* Af = (float*)Lm;                          // each of 33^2 doubles' room
-    float* Bf = (float*)K;
-    float* Zf = (float*)Z;
-    for (int e = tid; e < s2; e += RD_BLOCK) {
-      const int i = e / s, j = e - i * s;
-      const double g = G[e] * f;
-      A[i * RD_LD + j] = g;
-      Af[i * RD_LD + j] = (float)g;
-    }
-    __syncthreads();
-    if (s <= 16) conv = cta_jacobi_f32<16>(Af, Bf, RD_LD, s, wf, Zf, RD_LD, redf);
-    else conv = cta_jacobi_f32<32>(Af, Bf, RD_LD, s, wf, Zf, RD_LD, redf);
-    for (int e = tid; e < s2; e += RD_BLOCK) {
-      const int i = e / s, j = e - i * s;
-      X[i * RD_LD + j] = (double)Zf[i * RD_LD + j];
-    }
-    __syncthreads();
-    for (int it = 0; it < 2; ++it) cta_refine_eig(A, X, Lm, K, Z, w, s, RD_LD);
-    lmax = warp_max(w[lane < s ? lane : 0]) * scalbn(1.0, -sh);
-    __syncthreads();
-  }
   if (tid >= 32) return;
   const double* PtP = G;
   const double* OtP = G + s2;
   const double* OtO = G + 2 * s2;
+  // ||P||_2 from the largest eigenvalue of P^T P
+  for (int i = 0; i < s; ++i)
+    if (lane < s) A[i * RD_LD + lane] = PtP[i * s + lane];
+  __syncwarp();
+  bool conv = warp_syev<false>(A, RD_LD, s, w, Z, RD_LD);
+  __syncwarp();
+  const double lmax = w[s - 1];
   const double rho = sqrt((double)n) * eps * sqrt(lmax > 0.0 ? lmax : 0.0);
   // B = sym(Omega^T P + rho Omega^T Omega) into Lm, then its Cholesky factor
   for (int i = 0; i < s; ++i)
