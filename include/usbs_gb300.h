@@ -461,6 +461,11 @@ int usbs_selftest_wait_limits(int which, int nctas, long long limit_ns, unsigned
  * device pointers), for comparison with the IEEE division. */
 int usbs_selftest_recip(long long n, const double* x, double* y, void* stream);
 
+/* The interior-point kernel's inverse of an n x n matrix (row-major, n <= 12, device
+ * pointers): *ok is 0 where a pivot was zero or infinite, which a solve reports as
+ * status bit 8. */
+int usbs_selftest_inverse(int n, const double* A, double* Ainv, int* ok, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -57,6 +57,7 @@ SIGNATURES = {
                                P]),
     "usbs_selftest_wait_limits": (c_int, [c_int, c_int, c_ll, P, P, P]),
     "usbs_selftest_recip": (c_int, [c_ll, P, P, P]),
+    "usbs_selftest_inverse": (c_int, [c_int, P, P, P, P]),
 }
 
 

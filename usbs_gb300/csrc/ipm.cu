@@ -172,7 +172,7 @@ __device__ __forceinline__ unsigned long long abs_key(double x) {
 // integer keys, ties to the smaller row) and forms its reciprocal on the integer
 // pipes.  Per element the arithmetic is that of the row-by-row algorithm (rows
 // j and piv exchanged, pivot row scaled by 1/a_jj, a_ic - a_ij * row_c).  Returns
-// false if a pivot is zero.  (With the exchange, the column copy, the scaling
+// false if a pivot is zero or infinite.  (With the exchange, the column copy, the scaling
 // and the update as four steps between barriers it took 28k cycles at n = 11.)
 __device__ bool cta_inverse(const double* A, int n, double* Ainv, double* ws) {
   const int tid = threadIdx.x, lane = tid & 31, ld = 2 * n;
@@ -196,7 +196,7 @@ __device__ bool cta_inverse(const double* A, int n, double* Ainv, double* ws) {
     const double pv = __shfl_sync(0xffffffffu, a, piv);
     const bool zero = abs_key(pv) == 0ull;
     const double inv = zero ? 0.0 : recip_exact(pv);
-    if (zero) ok = false;
+    if (abs_key(inv) == 0ull) ok = false;        // a zero or an infinite pivot
     for (int e = tid; e < n * ld; e += IPM_BLOCK) {
       const int i = e / ld, c = e - i * ld;
       const int src = (i == j) ? piv : (i == piv) ? j : i;
@@ -1015,6 +1015,24 @@ int launch_ipm(const IpmArgs& a, cudaStream_t st) {
   ipm_kernel<<<1, IPM_BLOCK, dyn, st>>>(a);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { set_error("ipm launch: %s", cudaGetErrorString(e)); return -5; }
+  return 0;
+}
+
+// cta_inverse of one matrix: the inverse and whether every pivot was usable
+__global__ void __launch_bounds__(IPM_BLOCK) selftest_inverse_kernel(
+    int n, const double* __restrict__ A, double* __restrict__ Ainv, int* ok) {
+  __shared__ double M[IPM_MAXK * IPM_MAXK], R[IPM_MAXK * IPM_MAXK], ws[4 * IPM_MAXK * IPM_MAXK];
+  for (int e = threadIdx.x; e < n * n; e += IPM_BLOCK) M[e] = A[e];
+  __syncthreads();
+  const bool good = cta_inverse(M, n, R, ws);
+  for (int e = threadIdx.x; e < n * n; e += IPM_BLOCK) Ainv[e] = R[e];
+  if (threadIdx.x == 0) *ok = good ? 1 : 0;
+}
+
+int launch_selftest_inverse(int n, const double* A, double* Ainv, int* ok, cudaStream_t st) {
+  selftest_inverse_kernel<<<1, IPM_BLOCK, 0, st>>>(n, A, Ainv, ok);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) { set_error("selftest_inverse: %s", cudaGetErrorString(e)); return -5; }
   return 0;
 }
 

@@ -13,6 +13,7 @@
 #include "common.cuh"
 #include "internal.h"
 #include "recip.cuh"
+#include "solver.h"
 
 namespace usbs {
 
@@ -56,6 +57,15 @@ extern "C" int usbs_selftest_recip(long long n, const double* x, double* y, void
     return -5;
   }
   return 0;
+}
+
+extern "C" int usbs_selftest_inverse(int n, const double* A, double* Ainv, int* ok,
+                                     void* stream) {
+  if (n < 1 || n > IPM_MAXK || !A || !Ainv || !ok) {
+    set_error("selftest_inverse: n=%d (1 to %d)", n, IPM_MAXK);
+    return -2;
+  }
+  return launch_selftest_inverse(n, A, Ainv, ok, (cudaStream_t)stream);
 }
 
 extern "C" int usbs_selftest_wait_limits(int which, int nctas, long long limit_ns,

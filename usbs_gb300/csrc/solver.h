@@ -82,6 +82,7 @@ struct CholQRArgs {
 };
 
 int launch_ipm(const IpmArgs& a, cudaStream_t st);
+int launch_selftest_inverse(int n, const double* A, double* Ainv, int* ok, cudaStream_t st);
 int launch_eigS(const EigSArgs& a, cudaStream_t st);
 int launch_cholqr(const CholQRArgs& a, cudaStream_t st);
 
