@@ -2665,7 +2665,9 @@ lanczos_cluster_kernel(const __grid_constant__ ClusterBatch<VT> batch) {
       cg[p - p0] = (uint32_t)gc;
       D[X.vs + p - p0] = P.val[p];
     }
-    for (int lr = tid; lr <= X.rows; lr += LZ_BLOCK) rp[lr] = P.rowptr[X.r0 + lr] - p0;
+    // (a CTA past the problem's last row has no rows, and r0 may be past n)
+    for (int lr = tid; lr <= X.rows; lr += LZ_BLOCK)
+      rp[lr] = (X.rows > 0) ? P.rowptr[X.r0 + lr] - p0 : 0;
     remote = (int)block_sum((double)remote, sh.red);
     // A copy of all of x where there is room for it and the rows' entries in
     // other CTAs number at least a quarter of it: the copy reads consecutive
