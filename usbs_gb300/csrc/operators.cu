@@ -40,6 +40,8 @@ static unsigned long long sign_of_scale(double alpha) {
   return (alpha == 1.0) ? 0ull : (alpha == -1.0) ? 1ull << 63 : 1ull;
 }
 
+// The kernels below count entries, rows and triples in unsigned: the entry points take
+// up to 2^31 - 1 of them, and a position plus a grid's stride stays below 2^32.
 constexpr int AS_BLOCK = 256;
 
 // out = alpha_c C + A*(w) on the pattern.  Entries that no triple lands on (seven of
@@ -49,29 +51,29 @@ constexpr int AS_BLOCK = 256;
 // 50 us (87 with every entry scaled, added to and converted in place).
 template <typename OT, int AS_PER>      // AS_PER pattern entries per thread and round
 __global__ void __launch_bounds__(AS_BLOCK) assemble_kernel(
-    int nnz, const double* __restrict__ c_val, double alpha_c, unsigned long long sgn,
+    unsigned nnz, const double* __restrict__ c_val, double alpha_c, unsigned long long sgn,
     const int* __restrict__ slot_ptr, const int* __restrict__ slot_tid,
     const int* __restrict__ con, const double* __restrict__ a, const double* __restrict__ w,
     OT* __restrict__ out) {
-  __shared__ int list[AS_BLOCK * AS_PER];
+  __shared__ unsigned list[AS_BLOCK * AS_PER];
   __shared__ int count;
   const bool has_c = alpha_c != 0.0 && c_val;
-  constexpr int CH = AS_BLOCK * AS_PER;
-  for (int base = blockIdx.x * CH; base < nnz; base += gridDim.x * CH) {
+  constexpr unsigned CH = AS_BLOCK * AS_PER;
+  for (unsigned base = blockIdx.x * CH; base < nnz; base += gridDim.x * CH) {
     if (threadIdx.x == 0) count = 0;
     __syncthreads();
     double v[AS_PER];
     int n0[AS_PER], n1[AS_PER];
 #pragma unroll
     for (int u = 0; u < AS_PER; ++u) {
-      const int p = base + u * AS_BLOCK + threadIdx.x;
+      const unsigned p = base + u * AS_BLOCK + threadIdx.x;
       v[u] = (has_c && p < nnz) ? c_val[p] : 0.0;
       n0[u] = n1[u] = 0;
       if (w && p < nnz) { n0[u] = slot_ptr[p]; n1[u] = slot_ptr[p + 1]; }
     }
 #pragma unroll
     for (int u = 0; u < AS_PER; ++u) {
-      const int p = base + u * AS_BLOCK + threadIdx.x;
+      const unsigned p = base + u * AS_BLOCK + threadIdx.x;
       const bool more = n1[u] > n0[u];
       const unsigned mb = __ballot_sync(0xffffffffu, more);
       int at = 0;
@@ -83,7 +85,7 @@ __global__ void __launch_bounds__(AS_BLOCK) assemble_kernel(
     __syncthreads();
     const int cnt = count;
     for (int i = threadIdx.x; i < cnt; i += AS_BLOCK) {
-      const int p = list[i];
+      const unsigned p = list[i];
       double x = has_c ? scaled(alpha_c, sgn, c_val[p]) : 0.0;
       const int e = slot_ptr[p + 1];
       for (int q = slot_ptr[p]; q < e; ++q) {
@@ -103,8 +105,8 @@ static void assemble_launch(int nnz, const double* c_val, double alpha_c, const 
   const unsigned long long sgn = sign_of_scale(alpha_c);
   // four entries per thread once that still fills the GPU twice over
   const int per = (nnz >= 152 * 2048) ? 4 : 1;
-  int blocks = (nnz + AS_BLOCK * per - 1) / (AS_BLOCK * per);
-  if (blocks > 152 * 16) blocks = 152 * 16;
+  const unsigned ch = AS_BLOCK * per, need = ((unsigned)nnz + ch - 1) / ch;
+  const int blocks = (int)(need < 152 * 16 ? need : 152 * 16);
   if (per == 4)
     assemble_kernel<OT, 4><<<blocks, AS_BLOCK, 0, stream>>>(nnz, c_val, alpha_c, sgn, slot_ptr,
                                                             slot_tid, con, a, w, out);
@@ -136,10 +138,10 @@ __global__ void csr_spmv_kernel(int n, const int* __restrict__ rowptr, const int
   const int lig = gid % L;
   const int lane = threadIdx.x & 31;
   const unsigned gmask = (L == 32) ? 0xffffffffu : (((1u << L) - 1u) << (lane & ~(L - 1)));
-  for (int row = gid / L; row < n; row += lanes_total / L) {
+  for (unsigned row = gid / L; row < (unsigned)n; row += lanes_total / L) {
     VT s = (VT)0;
-    const int e = rowptr[row + 1];
-    for (int p = rowptr[row] + lig; p < e; p += L) s += val[p] * x[col[p]];
+    const unsigned e = rowptr[row + 1];
+    for (unsigned p = rowptr[row] + lig; p < e; p += L) s += val[p] * x[col[p]];
 #pragma unroll
     for (int o = L >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(gmask, s, o, L);
     if (lig == 0) y[row] = s;
@@ -199,16 +201,16 @@ __global__ void __launch_bounds__(256) fused_apply_kernel(
   const int lane = threadIdx.x & 31;
   const unsigned gmask = (L == 32) ? 0xffffffffu : (((1u << L) - 1u) << (lane & ~(L - 1)));
   constexpr int U = 2;                             // entries in flight per lane
-  for (int row = gid / L; row < n; row += lanes_total / L) {
+  for (unsigned row = gid / L; row < (unsigned)n; row += lanes_total / L) {
     VT s = (VT)0;
-    const int e = rowptr[row + 1];
-    for (int p0 = rowptr[row] + lig; p0 < e; p0 += U * L) {
+    const unsigned e = rowptr[row + 1];
+    for (unsigned p0 = rowptr[row] + lig; p0 < e; p0 += U * L) {
       double v[U];
       VT xv[U];
       int b[U], f[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const int p = min(p0 + u * L, e - 1);
+        const unsigned p = min(p0 + u * L, e - 1);
         v[u] = has_c ? scaled(alpha_c, sgn, c_val[p]) : 0.0;
         xv[u] = x[col[p]];
         b[u] = f[u] = 0;
@@ -412,7 +414,7 @@ int gather_values(long long total, const int* map, const void* src, void* dst, i
 }
 
 // a_t U[i_t, :] . U[j_t, :]
-__device__ __forceinline__ double triple_value(int t, const int* __restrict__ t_row,
+__device__ __forceinline__ double triple_value(unsigned t, const int* __restrict__ t_row,
                                                const int* __restrict__ t_col,
                                                const double* __restrict__ a,
                                                const double* __restrict__ U, int ldu, int k) {
@@ -446,9 +448,9 @@ __global__ void __launch_bounds__(256) A_operator_kernel(
     while (todo) {
       const int src = __ffs(todo) - 1;
       todo &= todo - 1;
-      const int tb = __shfl_sync(0xffffffffu, b, src), te = __shfl_sync(0xffffffffu, e, src);
+      const unsigned tb = __shfl_sync(0xffffffffu, b, src), te = __shfl_sync(0xffffffffu, e, src);
       double s = 0.0;
-      for (int t = tb + lane; t < te; t += 32) {
+      for (unsigned t = tb + lane; t < te; t += 32) {
         const int i = t_row[t], j = t_col[t];
         double d = 0.0;
         for (int q = 0; q < k; ++q) d += U[(size_t)q * ldu + i] * U[(size_t)q * ldu + j];
@@ -458,7 +460,7 @@ __global__ void __launch_bounds__(256) A_operator_kernel(
       if (lane == 0) out[c0 + (long long)src * warps] = s;
     }
   }
-  for (int c = gid; c < m; c += total) {
+  for (unsigned c = gid; c < (unsigned)m; c += total) {
     const int b = con_ptr[c], cnt = con_ptr[c + 1] - b;
     if (cnt > AO_SHORT) continue;
     double v[AO_SHORT];
@@ -511,14 +513,14 @@ __global__ void __launch_bounds__(256) A_adjoint_kernel(
       todo &= todo - 1;
       const long long ws = w0 + (long long)src * warps;
       const int i = (int)(ws / k), q = (int)(ws - (long long)i * k);
-      const int tb = __shfl_sync(0xffffffffu, b, src), te = __shfl_sync(0xffffffffu, e, src);
+      const unsigned tb = __shfl_sync(0xffffffffu, b, src), te = __shfl_sync(0xffffffffu, e, src);
       const double* Uq = U + (size_t)q * ldu;
       double s = 0.0;
-      for (int t = tb + lane; t < te; t += 256) {
+      for (unsigned t = tb + lane; t < te; t += 256) {
         double av[8], zv[8], uv[8];
 #pragma unroll
         for (int h = 0; h < 8; ++h) {
-          const int th = min(t + 32 * h, te - 1);
+          const unsigned th = min(t + 32 * h, te - 1);
           av[h] = r_a[th];
           zv[h] = z[r_con[th]];
           uv[h] = Uq[r_col[th]];
@@ -531,7 +533,7 @@ __global__ void __launch_bounds__(256) A_adjoint_kernel(
       if (lane == 0) out[(size_t)q * ldo + i] = s;
     }
   }
-  for (int i = gid; i < n; i += total) {
+  for (unsigned i = gid; i < (unsigned)n; i += total) {
     const int b = row_ptr[i], cnt = row_ptr[i + 1] - b;
     if (cnt > AO_SHORT) continue;
     double az[AO_SHORT];

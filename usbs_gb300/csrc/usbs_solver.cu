@@ -384,14 +384,16 @@ __global__ void __launch_bounds__(256) svec_project_small_kernel(
   while (q > b) { q -= b + 1; ++b; }
   const double* Vb = V + (size_t)b * ldv;
   const double* Vq = V + (size_t)q * ldv;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < m; c += gridDim.x * blockDim.x) {
+  // (unsigned: a position plus the strides stays in range up to 2^31 - 1)
+  for (unsigned c = blockIdx.x * blockDim.x + threadIdx.x; c < (unsigned)m;
+       c += gridDim.x * blockDim.x) {
     double acc = 0.0;
-    const int e = con_ptr[c + 1];
-    for (int t0 = con_ptr[c]; t0 < e; t0 += 4) {
+    const unsigned e = con_ptr[c + 1];
+    for (unsigned t0 = con_ptr[c]; t0 < e; t0 += 4) {
       double av[4], bi[4], bj[4], qi[4], qj[4];
 #pragma unroll
       for (int h = 0; h < 4; ++h) {
-        const int t = min(t0 + h, e - 1);
+        const unsigned t = min(t0 + h, e - 1);
         const int i = t_row[t], j = t_col[t];
         av[h] = t_a[t];
         bi[h] = Vb[i]; bj[h] = Vb[j]; qi[h] = Vq[i]; qj[h] = Vq[j];
@@ -469,15 +471,16 @@ __global__ void __launch_bounds__(QF_BLOCK) quadform_kernel(
   const int tid = threadIdx.x;
   for (int e = tid; e < k * k; e += QF_BLOCK) { sp[e] = Sp[e]; scp[e] = Scp[e]; }
   __syncthreads();
-  for (int c0 = blockIdx.x * QF_CON; c0 < m; c0 += gridDim.x * QF_CON) {
-    const int c1 = min(c0 + QF_CON, m), c = c0 + (tid & 31);
+  // (unsigned: a position plus the strides stays in range up to 2^31 - 1)
+  for (unsigned c0 = blockIdx.x * QF_CON; c0 < (unsigned)m; c0 += gridDim.x * QF_CON) {
+    const unsigned c1 = min(c0 + QF_CON, (unsigned)m), c = c0 + (tid & 31);
     const int T0 = con_ptr[c0], T1 = con_ptr[c1];
     int b = 0, e = 0;
     if (tid < 64 && c < c1) { b = con_ptr[c]; e = con_ptr[c + 1]; }
     const double* vs = (tid < 32) ? v1 : v2;
     double acc = 0.0;
-    for (int t0 = T0; t0 < T1; t0 += QF_TILE) {
-      const int tn = min(QF_TILE, T1 - t0);
+    for (int t0 = T0, tn; t0 < T1; t0 += tn) {
+      tn = min(QF_TILE, T1 - t0);
       for (int x = tid; x < tn; x += QF_BLOCK) {
         const int i = t_row[t0 + x], j = t_col[t0 + x];
         va[x] = t_a[t0 + x];
@@ -519,7 +522,7 @@ static int launch_quadform(int m, const int* con_ptr, const int* t_row, const in
                            const double* t_a, const double* V, int ldv, int k, const double* Sp,
                            const double* Scp, double* AF, double* AFc, int sm_count,
                            cudaStream_t st) {
-  int blocks = (m + QF_CON - 1) / QF_CON;
+  int blocks = m / QF_CON + (m % QF_CON ? 1 : 0);
   if (blocks > sm_count * 8) blocks = sm_count * 8;
   if (blocks < 1) blocks = 1;
   auto go = [&](auto kern) {
@@ -1321,7 +1324,7 @@ static int body(Solver& X, int t) {
   {
     ++X.launches;
     if (L.s <= 15) {
-      const int blocks = (L.m + 255) / 256;
+      const int blocks = L.m / 256 + (L.m % 256 ? 1 : 0);
       svec_project_small_kernel<<<dim3((unsigned)blocks, (unsigned)L.s), 256, 0, st>>>(
           L.m, P->con_ptr, P->t_row, P->t_col, P->t_a, V, L.ld, L.s, L.Pm, L.m, nullptr);
     } else {
