@@ -1289,7 +1289,7 @@ __global__ void __launch_bounds__(LZ_BLOCK) st_dot_kernel(const __grid_constant_
                                                            StreamCtl* ctl) {
   st_pdl_prologue();
   typedef typename Acc<VT>::type AT;
-  __shared__ StShared<VT> sh;
+  __shared__ int last;
   __shared__ AT sacc[DOT_U * LZ_BLOCK];
   int i, nv, buf;
   if (st_mode(ctl, P.m, &i, &nv, &buf) == SM_SKIP) return;
@@ -1342,9 +1342,9 @@ __global__ void __launch_bounds__(LZ_BLOCK) st_dot_kernel(const __grid_constant_
   // the group's last CTA
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) sh.last = (atomicAdd(&ctl->dticket[g], 1u) == (unsigned)R - 1u) ? 1 : 0;
+  if (threadIdx.x == 0) last = (atomicAdd(&ctl->dticket[g], 1u) == (unsigned)R - 1u) ? 1 : 0;
   __syncthreads();
-  if (!sh.last) return;
+  if (!last) return;
   __threadfence();
   // st_reduce's sums of columns g + DOT_G w: lane l adds partials l, l + 64, ... and
   // l + 32, l + 96, ..., then a butterfly
@@ -2147,7 +2147,7 @@ __device__ __forceinline__ VT cl_row_sum(const ClCtx<VT>& X, int lr, int lig, in
   if (lr < X.rows) {
     constexpr int B = NL < 8 ? NL : 8;           // entries in flight per round trip ...
     constexpr int U = NL < 8 ? 8 / NL : 1;       // ... over U trips round the accumulators
-    if ((NL > 1 && sizeof(VT) == 4) || X.staged) {
+    if (NL > 1 || X.staged) {         // (in global memory lp = lanes: NL = 1)
       const VT* D = cl_dyn_words<VT>();
       const int* rp = cl_dyn_words<int>() + X.rp;
       const uint32_t* cg = cl_dyn_words<uint32_t>() + X.cg;
@@ -2180,7 +2180,7 @@ __device__ __forceinline__ VT cl_row_sum(const ClCtx<VT>& X, int lr, int lig, in
           }
         }
       }
-    } else if constexpr (NL == 1 || sizeof(VT) == 8) {
+    } else if constexpr (NL == 1) {
       const int e = X.g_rowptr[X.r0 + lr + 1];
       for (int p0 = X.g_rowptr[X.r0 + lr] + lig; p0 < e; p0 += U * L) {
 #pragma unroll

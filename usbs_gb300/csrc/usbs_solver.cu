@@ -569,7 +569,7 @@ struct MvecArgs {
 // block's threads read all partials at once; the NR sums are then chains of
 // dependent FP64 adds over shared memory (60 cycles a block, 9 us for 304
 // blocks; 36 us with a global load in front of each add).
-constexpr int MV_MAXB = 512;         // most blocks (mgrid is at most two per SM)
+constexpr int MV_MAXB = 512;         // most blocks (see grid_red: two per SM)
 template <int NR>
 __device__ __forceinline__ bool mvec_finish(const MvecArgs& a, double (&v)[NR], const bool* is_max,
                                             double* red) {
@@ -587,17 +587,14 @@ __device__ __forceinline__ bool mvec_finish(const MvecArgs& a, double (&v)[NR], 
   __syncthreads();
   if (!last) return false;
   __threadfence();
-  const bool fits = nb <= MV_MAXB;
-  if (fits)
-    for (int e = tid; e < nb * NR; e += RED_BLOCK) all[e] = __ldcg(a.partial + e);
+  for (int e = tid; e < nb * NR; e += RED_BLOCK) all[e] = __ldcg(a.partial + e);
   __syncthreads();
   double mx[NR];
 #pragma unroll
   for (int r = 0; r < NR; ++r) {
     mx[r] = 0.0;
     if (is_max[r]) {                 // a maximum does not depend on the order
-      for (int bk = tid; bk < nb; bk += RED_BLOCK)
-        mx[r] = fmax(mx[r], fits ? all[bk * NR + r] : __ldcg(a.partial + (size_t)bk * NR + r));
+      for (int bk = tid; bk < nb; bk += RED_BLOCK) mx[r] = fmax(mx[r], all[bk * NR + r]);
       mx[r] = block_max(mx[r], red);
       __syncthreads();
     }
@@ -610,8 +607,7 @@ __device__ __forceinline__ bool mvec_finish(const MvecArgs& a, double (&v)[NR], 
       if (tid == r && is_max[r]) { s = mx[r]; mine_max = true; }
     if (!mine_max) {
 #pragma unroll 8
-      for (int bk = 0; bk < nb; ++bk)
-        s += fits ? all[bk * NR + tid] : __ldcg(a.partial + (size_t)bk * NR + tid);
+      for (int bk = 0; bk < nb; ++bk) s += all[bk * NR + tid];
     }
     red[tid] = s;
   }
@@ -1025,7 +1021,7 @@ static int plan(const usbs_problem* P, const usbs_params* Pa, const DeviceInfo& 
   L.ld = (L.n + 31) & ~31;
   L.mL = Pa->lanczos_inner_iterations;
   L.vt = (Pa->precision == 64) ? 8 : 4;
-  L.grid_red = di.sm_count * 2;
+  L.grid_red = di.sm_count * 2 < MV_MAXB ? di.sm_count * 2 : MV_MAXB;
   L.grid_gram = di.sm_count * 2;
   int o = 0;
   auto take = [&](int cnt) { int r = o; o += (cnt + 3) & ~3; return r; };
@@ -1701,7 +1697,7 @@ static void cgal_plan(const usbs_problem* P, const usbs_cgal_params* Pa, const D
   L.n = P->n; L.m = P->m; L.ld = (L.n + 31) & ~31; L.mL = Pa->lanczos_inner_iterations;
   L.vt = (Pa->precision == 64) ? 8 : 4;
   L.ssk = (Pa->sketch_mode == 0) ? Pa->sketch_dim : 0;
-  L.grid_red = di.sm_count * 2;
+  L.grid_red = di.sm_count * 2 < MV_MAXB ? di.sm_count * 2 : MV_MAXB;
   L.grid_gram = di.sm_count * 2;
   L.sc = ar.take<double>(CG_NUM + 64);
   L.adj = ar.take<double>(L.m); L.zn = ar.take<double>(L.m); L.Av = ar.take<double>(L.m);
