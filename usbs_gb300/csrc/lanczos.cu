@@ -1643,7 +1643,7 @@ __global__ void __launch_bounds__(LZ_BLOCK) st_rotate_kernel(const __grid_consta
 // control block: after breakdowns (which take slots of their own; it runs their
 // cycle again from its start), or when there are more restarts than launches
 // planned (see WV_LAUNCHES).
-// ER n = 30,011 of degree 12, FP32, 10 restarts: 4.8 ms per call (14.4 as one
+// ER n = 30,011 of degree 12, FP32, 10 restarts: 4.7 ms per call (14.4 as one
 // cooperative launch of 30 CTAs, 5.3 with A1 and A2 as one kernel).
 constexpr int WV_C = 4;                  // CTAs (tiles) per rank
 constexpr int WV_U = 8;                  // columns per CTA: c = j + 4 u
@@ -2022,7 +2022,7 @@ __global__ void __launch_bounds__(LZ_BLOCK) wv_update_norm_kernel(
 // 5.9k, second projection 4.2k, norm pass 2.6k, reductions 4.5k, barriers 1.7k)
 // and 153k per restart, 2.13 ms per call of 131 steps (3.53 ms with one
 // gather, one column and one shuffle level at a time); FP64 ER n = 800 of
-// degree 48 3.06 ms (8.25 ms).
+// degree 48 3.02 ms (8.25 ms).
 constexpr int CL_MAX_CTAS = 16;
 
 template <typename VT>

@@ -184,7 +184,7 @@ int csr_spmv(int n, long long nnz, const int* rowptr, const int* col, const void
 // formed as assemble_kernel forms it (rounded to VT), and the row is summed as
 // csr_spmv_kernel sums it, so the result is that of the two kernels.  One apply
 // then reads the pattern once and writes y, one launch: n = 10^6, 8.1e6 entries,
-// FP32: 81 us (87 as two kernels); n = 800, degree 48, FP64: 16 us a call (37 as two
+// FP32: 84 us (89 as two kernels); n = 800, degree 48, FP64: 16 us a call (37 as two
 // launches and an allocation for the values).  (The Lanczos path applies one operator a hundred
 // times and keeps the assembled values.)
 template <typename VT, int L>

@@ -148,7 +148,8 @@ __global__ void __launch_bounds__(RD_RED) rd_reduce_kernel(int E, int nblocks,
 // one CTA: warp 0 forms rho from the largest eigenvalue of P^T P, L, M^T M and its
 // eigen-decomposition, T and Lambda (see the file comment).  Bound by the two QR
 // iterations' chains of FP64 instructions on one warp, of which the first needs the
-// eigenvalues alone.
+// eigenvalues alone: 408 us at s = 10 (593 with its vectors, and the partials summed
+// here).
 __global__ void __launch_bounds__(RD_BLOCK) rd_small_kernel(int n, int s, double eps,
                                                             const double* __restrict__ gsum,
                                                             double* __restrict__ small) {
